@@ -35,6 +35,10 @@ __host__ __device__ __forceinline__ uint32_t unit30(uint32_t k)
     return uint32_t((0x1D1713110D0B0701ull >> (8 * k)) & 0xFF);
 }
 
+// bit r set for the units r mod 30
+constexpr uint32_t kUnits30 = (1u << 1) | (1u << 7) | (1u << 11) | (1u << 13) | (1u << 17) | (1u << 19) |
+                              (1u << 23) | (1u << 29);
+
 // class array index of a residue mod 30, or 8 when it is not coprime to 30
 __host__ __device__ __forceinline__ uint32_t class_of(uint32_t u)
 {

@@ -614,157 +614,239 @@ __global__ void __launch_bounds__(256) k_large(BatchDesc d)
     }
 }
 
-// floor(x / p) and x mod p for any 64-bit x and 2^7 <= p < 2^32, without a
-// division: two base-2^32 digits, each remainder by mod_below, each digit
-// of the quotient exactly as (digit - remainder) * p^-1 mod 2^32 (the
-// quotient digit is below 2^32, so the multiple of p divides exactly).
-__device__ __forceinline__ uint64_t divmod_u64(uint64_t x, uint32_t p, float rp, uint32_t pinv, uint32_t &rem)
+// floor(2^64 / p), or up to four less, for 3 <= p < 2^32: the hit lists' reciprocal. From 2^20 on
+// without a division: a float estimate of 2^52 / p (error below 2^13 of it),
+// scaled by 2^12 and corrected by the float estimate of what it leaves; the
+// corrected value is within two of 2^64 / p, so two less never exceeds it.
+__device__ __forceinline__ uint64_t recip64(uint32_t p, float rp)
 {
-    const uint32_t hi = uint32_t(x >> 32), lo = uint32_t(x);
-    const uint32_t rh = hi < p ? hi : mod_below(hi, p, rp);
-    const uint32_t qh = (hi - rh) * pinv;
-    const uint64_t x2 = (uint64_t(rh) << 32) | lo;
-    rem = mod_below(x2, p, rp);
-    const uint32_t ql = uint32_t(x2 - rem) * pinv;
-    return (uint64_t(qh) << 32) | ql;
+    if (p < (1u << 20)) return 0xFFFFFFFFFFFFFFFFull / p;
+    const uint32_t q1 = __float2uint_rz(rp * 4503599627370496.0f);  // 2^52 / p, saturated below 2^32
+    const int64_t d = int64_t((1ull << 52) - uint64_t(q1) * p);     // |d| < 2^33
+    const int32_t c = __float2int_rn(__int2float_rn(int32_t(d >> 2)) * (rp * 16384.0f));
+    return (uint64_t(q1) << 12) + uint64_t(int64_t(c)) - 2;
 }
 
-// p^-1 mod 2^32 for odd p (Newton: the correct low bits double each step)
-__device__ __forceinline__ uint32_t inv_mod_2_32(uint32_t p)
+// floor(x / p) and x mod p for x < 2^60 and inv = recip64(p): the high half
+// of x inv is the quotient or one less (x (2^64 / p - inv) / 2^64 < 1 / 4).
+// The remainder before the correction is below 2 p: 32 bits hold it for
+// p < 2^31.
+__device__ __forceinline__ uint64_t divmod_recip(uint64_t x, uint32_t p, uint64_t inv, uint32_t &rem)
 {
-    uint32_t x = p;  // p * p = 1 (mod 8)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) x *= 2u - p * x;
-    return x;
+    const uint64_t q = __umul64hi(x, inv);
+    uint32_t r = uint32_t(x) - uint32_t(q) * p;
+    bool more;
+    if (p >> 31) more = x - q * p >= p;
+    else more = r >= p;
+    if (more) r -= p;
+    rem = r;
+    return q + (more ? 1u : 0u);
 }
 
 // Hit lists through the prime-multiplier table (the reference's mt_build /
 // hl_harvest_mt / hl_apply, kernels/goldbach.cl:3181-3471): for a prime
 // p >= cbrt(q), a composite multiplier m of q = p m has a prime factor below
 // p, which marks q already, so only prime m matter. One thread per prime
-// p and run: the primes m in [ceil(Q0 / p), floor(Q1 / p)] are one
-// contiguous run of bytes of the table; each gives q = p m, whose class bit
-// is cleared with an atomic AND. Every such q is a semiprime whose factors
-// are both above the sieving bound of the other stages, so the bit is set
-// and no read is needed.
+// p and run; each prime m of the run's multiplier range gives q = p m, whose
+// class bit is cleared with an atomic AND. Every such q is a semiprime whose
+// factors are both above the sieving bound of the other stages, so the bit
+// is set and no read is needed.
+//
+// In class bits: with B = base / 30 (base a multiple of 30) and m = 30 b +
+// u_k (byte b of the table, bit k), q = p m is bit p b + floor(p u_k / 30) -
+// B of the class of p u_k mod 30. So one division per (prime, run), B = p b0
+// + rho, places every mark: byte b holds the bits p (b - b0) + v_k - rho,
+// v_k = floor(p u_k / 30) = (p / 30) u_k + floor((p mod 30) u_k / 30), in
+// 32-bit arithmetic, and a mark belongs to the run iff its bit is below
+// nblk (no masks over the end bytes). A run narrower than p / 32 bits holds
+// at most one multiple of p: its multiplier is 30 b0 + j, j the least with
+// floor(p j / 30) >= rho, and most pairs of such a run end there, with j not
+// a unit or the bit past the run, before any table read.
 __device__ __forceinline__ void ovf_push(const BatchParams &bp, uint32_t k, uint32_t t)
 {
     const uint32_t slot = atomicAdd(bp.ovf_cnt, 1u);
     if (slot < bp.ovf_cap) bp.ovf_buf[slot] = make_uint2(k, t);
 }
 
+// Bound by issue (68% on one 467.5M segment, 176 instructions per prime, of
+// them about 70 for a pair that ends in the narrow test) and, where p is
+// below the run's width, by the table's random sectors. Measured against a
+// pair that divided base and base + span apart, took byte bounds and masks
+// with 64-bit divisions by 30 and placed each mark with 64-bit arithmetic
+// (one GB300, harvest and sort): one segment 1.27 -> 0.75 ms, 128 segments
+// 8.13 -> 7.04 ms, 16 runs of 1e6 integers at 4e18..5e18 0.23 ms a run, 292
+// segments of uneven windows 75.1 -> 46.6 ms. Few, large CTAs: every CTA
+// writes one stream per region bin, and the streams share the L2: 2 x 768
+// threads 7.04 ms per 128 segments, 3 x 512 7.37, 4 x 384 8.17, 5 x 256
+// 8.38, 1 x 1024 7.76.
+constexpr int kHlThreads = 768, kHlCtas = 2;
+
+// What the harvest reads of a run, two 16-byte shared-memory loads.
+struct __align__(16) HlRun {
+    uint64_t B;          // base / 30
+    uint32_t nblk, n_hl;
+    uint32_t n_all;
+    uint32_t vbase;      // the run's first virtual bit (binned)
+    uint32_t pad[2];
+};
+
 // direct = 0: a binned batch's harvest (launched before the tiles); direct =
 // 1: every other batch's direct marks (launched after the tiles)
-__global__ void __launch_bounds__(256) k_hitlist(BatchDesc d, uint32_t direct)
+__global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, uint32_t direct)
 {
     const uint32_t nrun = d.h->nrun;
     if (!nrun) return;
     const bool binned = hl_binned(d.runs[0]);
     if (binned == (direct != 0)) return;
-    // per (class of p, class of m): the class kq of q = p m, its residue
-    // u_kq and u_m, as kq | u_kq << 8 | u_m << 16; the class of a residue
+    const BatchParams &run0 = d.runs[0];
+    const uint32_t i_lo = d.h->n_hl_min, nhi = d.h->n_all_max;
+    const uint32_t quota = binned ? run0.hl_quota : 0u;
+    const uint32_t rlog = run0.hl_rlog, nreg = run0.hl_nreg, nbin = 8 * nreg;
+    // per (class of p, class of m): u_m | floor((p mod 30) u_m / 30) << 8 |
+    // the class kq of q = p m << 16 (kq * nreg, its first region bin, << 20);
+    // the class of a residue
     __shared__ uint32_t s_cls[8][8];
     __shared__ uint8_t s_res[32];
+    __shared__ uint32_t s_hcnt[kHlMaxBins];
+    __shared__ HlRun s_run[256];
     if (threadIdx.x < 64) {
         const uint32_t a = threadIdx.x >> 3, b = threadIdx.x & 7;
-        const uint32_t uq = unit30(a) * unit30(b) % 30;
-        s_cls[a][b] = class_of(uq) | (uq << 8) | (unit30(b) << 16);
+        const uint32_t x = unit30(a) * unit30(b), kq = class_of(x % 30);
+        s_cls[a][b] = unit30(b) | (x / 30 << 8) | (kq << 16) | ((binned ? kq * nreg : 0u) << 20);
     } else if (threadIdx.x < 96) {
         s_res[threadIdx.x - 64] = uint8_t(class_of(threadIdx.x - 64));
     }
-    __shared__ uint32_t s_hcnt[kHlMaxBins];
     if (threadIdx.x < kHlMaxBins) s_hcnt[threadIdx.x] = 0;
+    for (uint32_t r = threadIdx.x; r < nrun; r += blockDim.x) {
+        const BatchParams &bp = d.runs[r];
+        HlRun x{};
+        x.B = bp.base / 30;
+        x.nblk = bp.nblk;
+        x.n_hl = bp.n_hl;
+        x.n_all = bp.n_all;
+        x.vbase = bp.tb_vt0 * run0.tile_bits;
+        s_run[r] = x;
+    }
     __syncthreads();
     // a binned batch files its marks in region bins (k_binsort takes them on)
-    const BatchParams &run0 = d.runs[0];
-    const uint32_t quota = binned ? run0.hl_quota : 0u;
-    const uint32_t rlog = run0.hl_rlog, nreg = run0.hl_nreg, nbin = 8 * nreg;
     uint32_t *const hl_mine = quota ? run0.hl_buf + size_t(blockIdx.x) * nbin * quota : nullptr;
-    // bit r set for the units r mod 30: the classes below a residue
-    constexpr uint32_t kUnits = (1u << 1) | (1u << 7) | (1u << 11) | (1u << 13) | (1u << 17) | (1u << 19) |
-                                (1u << 23) | (1u << 29);
-    constexpr uint32_t kInv15 = 0xEEEEEEEFu;  // 15^-1 mod 2^32
-    const uint32_t *primes = d.runs[0].primes;
-    const uint32_t nhi = d.h->n_all_max;
-    for (uint32_t i = d.h->n_hl_min + blockIdx.x * blockDim.x + threadIdx.x; i < nhi;
-         i += gridDim.x * blockDim.x) {
-        const uint32_t p = primes[i];
-        const float rp = __frcp_rn(float(p));
-        const uint32_t pinv = inv_mod_2_32(p);
-        const uint32_t kp = s_res[p % 30];
-        for (uint32_t ri = 0; ri < nrun; ++ri) {
+    const uint32_t rmask = (1u << rlog) - 1u;
+    // the table: bytes [tb0, tb0 + tbn) of the multiplier line (the same for every run)
+    const uint32_t *const mtab = run0.mtab;
+    const uint64_t tb0 = run0.m0 / 30, tbn = (run0.m1 - run0.m0 + 1) / 30;
+    // the marks of class cls of q at bit t of run ri (t < nblk)
+    auto mark = [&](uint32_t ri, uint32_t vbase, uint32_t e, uint32_t t) {
+        if (quota) {
+            const uint32_t v = vbase + t;
+            const uint32_t bin = (e >> 20) + (v >> rlog);
+            const uint32_t pos = atomicAdd(&s_hcnt[bin], 1u);
+            if (pos < quota) hl_mine[bin * quota + pos] = v & rmask;
+            else ovf_push(run0, (e >> 16) & 7u, v);
+        } else {
             const BatchParams &bp = d.runs[ri];
-            if (i < bp.n_hl || i >= bp.n_all) continue;
-            const uint64_t base = bp.base;
-            // m in [ceil(base / p), floor(q1 / p)], q1 = base + span: the
-            // second quotient from the first and a division of r0 + span < 2^37
-            uint32_t r0;
-            const uint64_t qb = divmod_u64(base, p, rp, pinv, r0);
-            const uint64_t span = 30ull * bp.nblk - 1;
-            // a run narrower than p (most pairs of a batch of short windows)
-            // holds a multiple of p only if r0 is 0 or above p - span
-            if (span < p && r0 && p - r0 > span) continue;
-            const uint64_t x = uint64_t(r0) + span;
-            const uint32_t r1 = mod_below(x, p, rp);
-            const uint64_t mlo = qb + (r0 ? 1 : 0), mhi = qb + uint32_t(x - r1) * pinv;
-            if (mhi < mlo) continue;
-            const uint64_t m0 = bp.m0;
-            if (mlo < m0 || mhi > bp.m1) {
-                atomicOr(bp.err, kErrTable);
-                continue;
+            atomicAnd(bp.map + size_t((e >> 16) & 7u) * bp.wpc + (t >> 5), ~(1u << (t & 31)));
+        }
+    };
+    // the pair (prime i = p, run ri): every path of a lane ends here, so the
+    // warp meets again before its next pair
+    auto pair = [&](uint32_t ri, uint32_t p, float rp, uint64_t inv, uint32_t pq, uint32_t pr, const HlRun &run) {
+        const uint32_t *const cls = s_cls[s_res[pr]];
+        uint32_t rho;
+        const uint64_t b = divmod_recip(run.B, p, inv, rho) - tb0;  // byte b0 in the table
+        if (run.nblk <= (p >> 5)) {
+            // at most one multiple: m = 30 b0 + j, j = ceil(30 rho / p).
+            // The estimate is lowered by 0.01, far above its error: when
+            // that gives j - 1, the first multiple is at least 0.99 p / 30
+            // > nblk bits up, and j - 1 itself is below the run.
+            const uint32_t j = __float2uint_ru(fmaxf(__uint2float_rn(rho) * (30.0f * rp) - 0.01f, 0.0f));
+            const uint32_t t = pq * j + ((pr * j * 2185u) >> 16) - rho;  // floor(pr j / 30): pr j < 900
+            if (((kUnits30 >> j) & 1u) && t < run.nblk) {
+                const uint32_t k = __popc(kUnits30 & ((1u << j) - 1u));
+                if (b >= tbn) atomicOr(run0.err, kErrTable);
+                else if ((__ldg(mtab + (b >> 2)) >> (8 * (uint32_t(b) & 3u) + k)) & 1u) mark(ri, run.vbase, cls[k], t);
             }
-            uint32_t *map = bp.map;
-            const uint32_t wpc = bp.wpc;
-            const uint32_t *mtab = bp.mtab;
-            const uint32_t vbase = bp.tb_vt0 * run0.tile_bits;  // the run's first virtual bit (binned)
-            // table bytes b0..b1; in the end bytes only the classes inside [mlo, mhi]
-            const uint64_t b0 = (mlo - m0) / 30, b1 = (mhi - m0) / 30;
-            const uint32_t dl = uint32_t(mlo - m0 - 30 * b0), dh = uint32_t(mhi - m0 - 30 * b1);
-            const uint32_t lo_byte = (0xFFu << __popc(kUnits & ((1u << dl) - 1u))) & 0xFFu;
-            const uint32_t hi_byte = (1u << __popc(kUnits & ((2u << dh) - 1u))) - 1u;
-            const uint64_t w0 = b0 >> 2, w1 = b1 >> 2;
-            const uint32_t lo_mask = (0xFFFFFFFFu << (8 * (b0 & 3))) & ~(0xFFu << (8 * (b0 & 3))) |
-                                     (lo_byte << (8 * (b0 & 3)));
-            const uint32_t hi_shift = 8 * uint32_t(b1 & 3);
-            const uint32_t hi_mask = (hi_shift ? (0xFFFFFFFFu >> (32 - hi_shift)) : 0u) | (hi_byte << hi_shift);
-            // q - base - u_q = xw + p (30 jb + u_m) - u_q for byte jb of word
-            // w, xw = p (m0 + 120 w) - base: a multiple of 30 below 2^64, and
-            // the class bit t = that / 30 < 2^31, so its low 32 bits suffice:
-            // bits 1..32 of it times 15^-1 mod 2^32
-            const uint32_t *tw = mtab + w0;
-            const uint32_t nw = uint32_t(w1 - w0);
-            const uint64_t step = 120ull * p;
-            uint64_t xw = uint64_t(p) * m0 - base + step * w0;
-            // the next table word loaded before this word's marks (its
-            // latency hidden behind them)
-            uint32_t vnext = __ldg(tw);
-            for (uint32_t iw = 0; iw <= nw; ++iw, xw += step) {
-                uint32_t v = vnext;
-                if (iw < nw) vnext = __ldg(tw + iw + 1);
-                if (iw == 0) v &= lo_mask;
-                if (iw == nw) v &= hi_mask;
-                while (v) {
-                    const uint32_t j = __ffs(v) - 1u;
-                    v &= v - 1u;
-                    const uint32_t e = s_cls[kp][j & 7];
-                    const uint64_t xq = xw + uint64_t(p) * (30u * (j >> 3) + (e >> 16)) - ((e >> 8) & 0xFFu);
-                    const uint32_t t = uint32_t(xq >> 1) * kInv15;
-                    if (quota) {
-                        const uint32_t v = vbase + t;
-                        const uint32_t bin = (e & 0xFFu) * nreg + (v >> rlog);
-                        const uint32_t pos = atomicAdd(&s_hcnt[bin], 1u);
-                        if (pos < quota) hl_mine[size_t(bin) * quota + pos] = v & ((1u << rlog) - 1u);
-                        else ovf_push(run0, e & 0xFFu, v);
-                        continue;
-                    }
-                    atomicAnd(map + size_t(e & 0xFFu) * wpc + (t >> 5), ~(1u << (t & 31)));
+            return;
+        }
+        if (p >> 31) {
+            // p >= 2^31 > nblk: at most two bytes, their bits in 64-bit arithmetic
+            const uint32_t more = uint64_t(rho) + run.nblk > p ? 1u : 0u;
+            if (b >= tbn || b + more >= tbn) {
+                atomicOr(run0.err, kErrTable);
+                return;
+            }
+            for (uint32_t nb = 0; nb <= more; ++nb) {
+                const uint64_t at = b + nb;
+                uint32_t v = (__ldg(mtab + (at >> 2)) >> (8 * (uint32_t(at) & 3u))) & 0xFFu;
+                for (; v; v &= v - 1u) {
+                    const uint32_t e = cls[__ffs(v) - 1u];
+                    const int64_t t = int64_t(nb ? uint64_t(p) : 0u) + int64_t(pq * (e & 0xFFu) + ((e >> 8) & 0xFFu)) - rho;
+                    if (t >= 0 && t < int64_t(run.nblk)) mark(ri, run.vbase, e, uint32_t(t));
                 }
             }
+            return;
+        }
+        // bytes b .. b + nb, nb = floor((rho + nblk - 1) / p) (a float
+        // estimate within one of it, corrected); bits in (-p, nblk + p):
+        // one below zero is at least 2^31 as u32
+        const uint32_t x = rho + run.nblk - 1;
+        uint32_t nb = __float2uint_rz(__uint2float_rn(x) * rp);
+        if (uint64_t(nb) * p > x) --nb;
+        else if (x - nb * p >= p) ++nb;
+        if (b >= tbn || b + nb >= tbn) {
+            atomicOr(run0.err, kErrTable);
+            return;
+        }
+        const uint32_t sh = uint32_t(b) & 3u, eb = sh + nb;  // the end byte from the first word's first
+        const uint32_t *tw = mtab + (b >> 2);
+        const uint32_t hi_mask = 0xFFFFFFFFu >> (24 - 8 * (eb & 3u));
+        uint32_t left = eb >> 2;                             // words after the current one
+        uint32_t tb = 0u - rho - p * sh;                     // bit of the word's byte 0, less its v_k
+        uint32_t v = __ldg(tw) & (0xFFFFFFFFu << (8 * sh));
+        if (!left) v &= hi_mask;
+        // the next table word loaded before this word's marks (its
+        // latency hidden behind them); one mark per trip, whichever word
+        // a lane is in, so a warp's trips follow its lanes' total marks
+        // and not the fullest lane of every word
+        uint32_t vn = left ? __ldg(tw + 1) : 0u;
+        for (;;) {
+            if (v) {
+                const uint32_t j = __ffs(v) - 1u;
+                v &= v - 1u;
+                const uint32_t e = cls[j & 7u];
+                const uint32_t t = tb + p * (j >> 3) + pq * (e & 0xFFu) + ((e >> 8) & 0xFFu);
+                if (t < run.nblk) mark(ri, run.vbase, e, t);
+            }
+            if (!v) {
+                if (!left) break;
+                --left;
+                ++tw;
+                tb += 4 * p;
+                v = vn;
+                if (left) vn = __ldg(tw + 1);
+                else v &= hi_mask;
+            }
+        }
+    };
+    const uint32_t *primes = run0.primes;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    // warp-uniform loops: the warp's first prime bounds them
+    uint32_t i = i_lo + blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t p_next = i < nhi ? __ldg(primes + i) : 3u;
+    for (; i - (threadIdx.x & 31u) < nhi; i += stride) {
+        const uint32_t p = p_next;
+        if (i + stride < nhi) p_next = __ldg(primes + i + stride);  // its latency behind this prime's work
+        const float rp = __fdividef(1.0f, __uint2float_rn(p));
+        const uint64_t inv = recip64(p, rp);
+        const uint32_t pq = p / 30, pr = p - 30 * pq;
+        for (uint32_t ri = 0; ri < nrun; ++ri) {
+            const HlRun run = s_run[ri];
+            if (i >= run.n_hl && i < run.n_all) pair(ri, p, rp, inv, pq, pr, run);
+            __syncwarp();
         }
     }
     if (quota) {
         __syncthreads();
-        for (uint32_t b = threadIdx.x; b < nbin; b += blockDim.x) run0.hl_cnt[blockIdx.x * nbin + b] = s_hcnt[b];
+        for (uint32_t bi = threadIdx.x; bi < nbin; bi += blockDim.x) run0.hl_cnt[blockIdx.x * nbin + bi] = s_hcnt[bi];
     }
 }
 
@@ -1024,7 +1106,7 @@ void launch_large(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st)
 
 void launch_hitlist(const gbk::BatchDesc &d, bool direct, const Grids &g, cudaStream_t st)
 {
-    gbk::k_hitlist<<<g.sm * g.hitlist, 256, 0, st>>>(d, direct ? 1u : 0u);
+    gbk::k_hitlist<<<g.sm * g.hitlist, gbk::kHlThreads, 0, st>>>(d, direct ? 1u : 0u);
 }
 
 // the harvest's grid is one wave of resident CTAs: its primes are dealt out
@@ -1032,7 +1114,7 @@ void launch_hitlist(const gbk::BatchDesc &d, bool direct, const Grids &g, cudaSt
 void query_sieve_grids(Grids &g)
 {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gbk::k_hitlist, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gbk::k_hitlist, gbk::kHlThreads, 0);
     g.hitlist = n > 0 ? n : 1;
 }
 

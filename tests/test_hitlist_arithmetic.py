@@ -1,0 +1,114 @@
+"""The hit-list harvest's placement of a prime's multiples (k_hitlist in
+goldbach-l0_gb300/csrc/k_sieve.cu), restated in exact float32 and integer
+arithmetic and compared with the general definition: the multiples q = p m of
+a run, m coprime to 30, as class bits, for runs narrower than p / 32 bits (one
+candidate multiplier), primes from 2^31 on (64-bit bits) and the word loop
+(32-bit bits). A CPU test of the algorithm; the GPU tests check the kernel
+through every map bit."""
+import math
+import random
+from fractions import Fraction as F
+
+import pytest
+
+from test_modulo_emulation import f2i_rn, f2u_rz, rn32
+
+U30 = (1, 7, 11, 13, 17, 19, 23, 29)
+M32, M64 = 2**32 - 1, 2**64 - 1
+
+
+def recip64(p):
+    rp = rn32(F(1, int(rn32(F(p)))))
+    if p < 1 << 20:
+        return M64 // p
+    q1 = f2u_rz(rn32(rp * 2**52))
+    d = 2**52 - q1 * p
+    assert abs(d) < 2**33
+    c = f2i_rn(rn32(rn32(F(d >> 2)) * rn32(rp * 2**14)))
+    return (q1 << 12) + c - 2
+
+
+def divmod_recip(x, p):
+    q = x * recip64(p) >> 64
+    r = x - q * p
+    assert 0 <= r < 2 * p
+    return (q + 1, r - p) if r >= p else (q, r)
+
+
+def marks(base, nblk, p):
+    """(class residue, bit) of every multiple p m in the run, m coprime to 30,
+    by the kernel's steps, every table bit taken as set."""
+    rp = rn32(F(1, int(rn32(F(p)))))
+    b0, rho = divmod_recip(base // 30, p)
+    pq, pr = divmod(p, 30)
+    out = set()
+
+    def v(u):
+        return pq * u + pr * u // 30
+
+    if nblk <= p >> 5:
+        a = rn32(rn32(F(rho)) * rn32(30 * rp))
+        j = math.ceil(max(rn32(a - rn32(F(1, 100))), 0))
+        t = (pq * j + ((pr * j * 2185) >> 16) - rho) & M32
+        if j in U30 and t < nblk:
+            out.add((p * j % 30, t))
+        return b0, out
+    if p >> 31:
+        for nb in range(2 if rho + nblk > p else 1):
+            out |= {(p * u % 30, nb * p + v(u) - rho) for u in U30 if 0 <= nb * p + v(u) - rho < nblk}
+        return b0, out
+    x = rho + nblk - 1
+    assert x <= M32
+    nb = f2u_rz(rn32(rn32(F(x)) * rp))
+    if nb * p > x:
+        nb -= 1
+    elif x - nb * p >= p:
+        nb += 1
+    assert nb == x // p
+    for b in range(nb + 1):
+        for u in U30:
+            t = (b * p + v(u) - rho) & M32
+            if t < nblk:
+                out.add((p * u % 30, t))
+    return b0, out
+
+
+def general(base, nblk, p):
+    m, out = -(-base // p), set()
+    while p * m < base + 30 * nblk:
+        if m % 30 in U30:
+            out.add((p * m % 30, (p * m - base) // 30))
+        m += 1
+    return out
+
+
+PRIMES = [131, 1009, 65537, 1048573, 1048583, 1703941, 4194319, 16777259, 99999989, 499999993,
+          1999999973, 2147483647, 2147483659, 2236067969, 4294967291]
+
+
+@pytest.mark.parametrize("p", PRIMES)
+def test_division_by_the_reciprocal(p):
+    rnd = random.Random(p)
+    assert 0 <= 2**64 - recip64(p) * p < 5 * p + p
+    top = (2**64 - 2**40) // 30
+    for x in [0, 1, p - 1, p, top, top // p * p, top // p * p - 1] + [rnd.randrange(top) for _ in range(200)]:
+        assert divmod_recip(x, p) == divmod(x, p)
+
+
+@pytest.mark.parametrize("p", PRIMES)
+def test_marks_equal_the_general_form(p):
+    rnd = random.Random(p + 1)
+    widths = {1, 2, 33, max(p >> 5, 1), (p >> 5) + 1, p // 30 + 1, p // 2 + 1, p - 1, p, p + 1, 40 * p}
+    for nblk in sorted(w for w in widths if 0 < w < 2**31 and w < 4096 * p):
+        if nblk // p > 50:
+            continue
+        for _ in range(12):
+            # bases whose first multiple sits at either end of the run or anywhere
+            m = rnd.randrange(p, max(p + 1, min(2**63 // p, 1 << 42)))
+            off = rnd.choice((0, 30, -30, 30 * nblk, 30 * (nblk - 1), rnd.randrange(30 * p)))
+            base = max(0, p * m - off) // 30 * 30
+            assert marks(base, nblk, p)[1] == general(base, nblk, p), (p, nblk, base)
+
+
+def test_small_product_division_by_30():
+    assert all((x * 2185) >> 16 == x // 30 for x in range(900))
