@@ -44,7 +44,6 @@ KNOBS = {
     "tile_bits": [0, 1572864, 1835008],  # 0: 2^tile_log2 bits
     "max_batch": [32, 48, 64, 96, 128],
     "plan_funnels": [6, 8, 12, 16],
-    "verify_funnels": [2, 3, 4],
 }
 DEFAULTS = {"p_mid": 1 << 22, "mtab_max_gb": 48, "tile_log2": 20, "tile_bits": 0, "max_batch": 16,
             "plan_funnels": 8, "verify_funnels": 3}

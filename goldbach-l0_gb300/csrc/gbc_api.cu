@@ -568,6 +568,7 @@ extern "C" int gbc_create(const gbc_config *cfg_in, gbc_ctx **out)
     if (!gbh::tile_attributes(ctx->tile_bits, cfg.tile_log2, ctx->gi, cfg.device, &ctx->tile_stage))
         return fail(ctx, GBC_E_ARG, "tile_bits: the tile does not fit the device's shared memory");
     gbh::query_check_grids(ctx->grids);
+    gbh::query_verify_grids(ctx->grids);
     gbh::query_count_grids(ctx->grids);
     gbh::query_sieve_grids(ctx->grids);
     CK(dev_alloc(ctx, &ctx->d_primes, (pr.size() + kPrimePad) * 4));
@@ -608,53 +609,36 @@ extern "C" int gbc_create(const gbc_config *cfg_in, gbc_ctx **out)
     ctx->ct.cand = ctx->d_cand;
     ctx->ct.list = ctx->d_list;
     ctx->ct.ridge_min = cfg.ridge_min;
-    CK(dev_alloc(ctx, &ctx->d_fun, std::max<size_t>(fun.size(), 1) * sizeof(uint2)));
-    if (!fun.empty()) CK(cudaMemcpy(ctx->d_fun, fun.data(), fun.size() * sizeof(uint2), cudaMemcpyHostToDevice));
-    // member pairs of each funnel: in shift space (member p0 + 30 d at shift
-    // dm - d below the top member), pairs {a, a + delta} inside the members,
-    // each tested by one shift of the window ORed with itself shifted by
-    // delta; the delta with the fewest shifts (+ 4 for the OR) or none
-    {
-        std::vector<uint2> pairs(std::max<size_t>(fun.size(), 1), make_uint2(0u, 0u));
-        for (size_t f = 0; f < fun.size(); ++f) {
-            const uint32_t y = fun[f].y;
-            const int dm = 31 - __builtin_clz(y);
-            uint32_t S = 0;
-            for (int d = 0; d <= dm; ++d)
-                if (y >> d & 1u) S |= 1u << (dm - d);
-            // costs in half ALU operations: a member 3 (a funnel shift and
-            // half a three-input OR), the OR of the window with its shift 8
-            int best_cost = 3 * __builtin_popcount(S), best_delta = 0;
-            uint32_t best_a = 0;
-            for (int delta = 1; delta < 32; ++delta) {
-                uint32_t used = 0, A = 0;
-                for (int a = 0; a + delta < 32; ++a)
-                    if ((S >> a & 1u) && (S >> (a + delta) & 1u) && !(used >> a & 1u) && !(used >> (a + delta) & 1u)) {
-                        A |= 1u << a;
-                        used |= (1u << a) | (1u << (a + delta));
-                    }
-                const uint32_t R = S & ~used;
-                const int cost = 8 + 3 * (__builtin_popcount(A) + __builtin_popcount(R));
-                const int groups = (__builtin_popcount(A) + 3) / 4 + (__builtin_popcount(R) + 3) / 4;
-                if (A && cost < best_cost && groups <= int(gbk::kVerifyMaxGroups)) {
-                    best_cost = cost;
-                    best_delta = delta;
-                    best_a = A;
-                }
+    // the plan's funnels as k_verify reads them: per class those the word form
+    // does not take first, in plan order
+    ctx->vt.word = 1;
+    std::vector<uint2> ev;
+    for (int cr = 0; cr < GBC_NCLASS; ++cr) {
+        const uint32_t r = 2u * cr, b = ctx->vt.fun_off[cr], n = ctx->vt.fun_cnt[cr];
+        uint32_t words = 0;
+        for (uint32_t last = 0; last < 2; ++last)
+            for (uint32_t f = b; f < b + n; ++f) {
+                const uint32_t p0 = cand[fun[f].x], y = fun[f].y, dm = 31 - __builtin_clz(y);
+                const bool word = gbh::verify_word_funnel(r, p0, y);
+                words += last && word ? 1 : 0;
+                if (word != (last != 0)) continue;
+                // member p0 + 30 d at offset p0 / 30 + d + [r < p0 mod 30]
+                uint32_t m = 0;
+                for (uint32_t d = 0; d <= dm; ++d)
+                    if (y >> d & 1u) m |= 1u << (dm - d);
+                const uint32_t omax = p0 / 30 + dm + (r < p0 % 30 ? 1 : 0);
+                ev.push_back(make_uint2(gbk::class_of((r + 30 - p0 % 30) % 30) | (omax << 8), m));
             }
-            pairs[f] = make_uint2(uint32_t(best_delta), best_a);
-        }
-        CK(dev_alloc(ctx, &ctx->d_fpair, pairs.size() * sizeof(uint2)));
-        CK(cudaMemcpy(ctx->d_fpair, pairs.data(), pairs.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+        if (words != 3) ctx->vt.word = 0;
     }
+    CK(dev_alloc(ctx, &ctx->d_ev, std::max<size_t>(ev.size(), 1) * sizeof(uint2)));
+    if (!ev.empty()) CK(cudaMemcpy(ctx->d_ev, ev.data(), ev.size() * sizeof(uint2), cudaMemcpyHostToDevice));
     CK(dev_alloc(ctx, &ctx->d_rest, std::max<size_t>(rest.size(), 1) * 2));
     if (!rest.empty()) CK(cudaMemcpy(ctx->d_rest, rest.data(), rest.size() * 2, cudaMemcpyHostToDevice));
     ctx->vt.cand = ctx->d_cand;
-    ctx->vt.fun = ctx->d_fun;
-    ctx->vt.fpair = ctx->d_fpair;
+    ctx->vt.ev = ctx->d_ev;
     ctx->vt.rest = ctx->d_rest;
     ctx->vt.ridge_min = cfg.ridge_min;
-    ctx->vt.f1 = cfg.verify_funnels;
     ctx->vt.spin0 = (cfg.test_flags & GBC_TEST_STAGING_WAIT) ? 0u : gbk::kStageSpin;
     ctx->slot.resize(cfg.nslots);
     for (auto &s : ctx->slot)
@@ -669,8 +653,7 @@ extern "C" void gbc_destroy(gbc_ctx *ctx)
     if (ctx->outputs && ctx->outputs_del) ctx->outputs_del(ctx->outputs);
     if (ctx->stats && ctx->stats_del) ctx->stats_del(ctx->stats);
     for (auto &s : ctx->slot) slot_free(s);
-    cudaFree(ctx->d_fun);
-    cudaFree(ctx->d_fpair);
+    cudaFree(ctx->d_ev);
     cudaFree(ctx->d_rest);
     cudaFree(ctx->mtab);
     cudaFree(ctx->d_primes);
@@ -827,10 +810,10 @@ static void finish_desc(const gbc_ctx *ctx, DescImage &img)
         img.ver_pref[i] = h.ver_vb;
         img.cnt_pref[i] = h.cnt_vb;
         const uint64_t evens = (sp.seg_end - sp.seg_start) / 2 + 1;
-        sp.vbx = gbh::check_vbx(evens, ctx->grids.sm);
+        sp.vbx = sp.sampled ? gbh::check_vbx(evens, ctx->grids.sm) : gbh::verify_vbx(evens, ctx->grids.sm);
         if (sp.low) ++h.nlow;
         else if (sp.sampled) h.chk_vb += GBC_NCLASS * sp.vbx;
-        else h.ver_vb += GBC_NCLASS * sp.vbx;
+        else h.ver_vb += sp.vbx;
         h.cnt_vb += gbh::count_ranges(img.runs[sp.run].base, sp, sp.cr);
     }
     img.chk_pref[nseg] = h.chk_vb;
@@ -1157,6 +1140,7 @@ static int issue_plain(gbc_ctx *ctx, Slot &s)
         gbh::launch_hl_overflow(d, g, st);
         gbh::launch_check(d, ctx->ct, g, st);
         gbh::launch_verify(d, ctx->vt, g, st);
+        gbh::launch_tail(d, ctx->vt, g, st);
         gbh::launch_retry(d, ctx->cfg.ridge_min, (ctx->cfg.test_flags & GBC_TEST_RETRY_LIMIT) ? 1u : (1u << 22), g,
                           st);
         gbh::launch_count(d, g, st);
@@ -1192,6 +1176,7 @@ static int issue_pipeline(gbc_ctx *ctx, Slot &s, bool capture)
     CK(cudaEventRecordWithFlags(s.ev[2], st, rec));
     gbh::launch_check(d, ctx->ct, g, st);
     gbh::launch_verify(d, ctx->vt, g, st);
+    gbh::launch_tail(d, ctx->vt, g, st);
     gbh::launch_retry(d, ctx->cfg.ridge_min, (ctx->cfg.test_flags & GBC_TEST_RETRY_LIMIT) ? 1u : (1u << 22), g, st);
     CK(cudaEventRecordWithFlags(s.ev[3], st, rec));
     gbh::launch_count(d, g, st);

@@ -29,7 +29,7 @@ constexpr uint32_t kWheelTabWords = 1001 + 720 + 1001 + 240;
 constexpr uint32_t kPackGroup = 256;  // packed large primes per group (one warp decodes a group)
 
 // u_k, the residue of class array k
-__host__ __device__ __forceinline__ uint32_t unit30(uint32_t k)
+__host__ __device__ __forceinline__ constexpr uint32_t unit30(uint32_t k)
 {
     // bytes, low to high: 1, 7, 11, 13, 17, 19, 23, 29
     return uint32_t((0x1D1713110D0B0701ull >> (8 * k)) & 0xFF);
@@ -40,7 +40,7 @@ constexpr uint32_t kUnits30 = (1u << 1) | (1u << 7) | (1u << 11) | (1u << 13) | 
                               (1u << 23) | (1u << 29);
 
 // class array index of a residue mod 30, or 8 when it is not coprime to 30
-__host__ __device__ __forceinline__ uint32_t class_of(uint32_t u)
+__host__ __device__ __forceinline__ constexpr uint32_t class_of(uint32_t u)
 {
     uint32_t c = 8;
     for (uint32_t k = 0; k < 8; ++k)
@@ -172,7 +172,7 @@ struct SegParams {
     uint2 *pend;                  // phase-A misses: (class r / 2 << 27 | word, unresolved bits)
     uint32_t pend_cap;
     uint32_t run;                 // the segment's run (class map) in the batch
-    uint32_t vbx;                 // checker CTAs per class of the segment
+    uint32_t vbx;                 // checker CTAs of the segment: per class (sampled), in all (verify)
     uint32_t pad;
     CountRanges cr;
 };
@@ -254,13 +254,16 @@ struct CheckTables {
 // of its exact continuation (phase B), per class r / 2.
 struct VerifyTables {
     const uint16_t *cand;
-    const uint2 *fun;       // funnel: candidate index of its smallest member p, members (bit d: p + 30 d, d < 32)
-    const uint2 *fpair;     // per funnel: delta, pair starts a (bit a: shifts a and a + delta), or 0, 0
+    // a plan funnel as the even form reads it: the class array k its members
+    // read | omax << 8, and the member mask: member at offset o (it reads bit
+    // T - o for the even T of the class) <-> bit omax - o. The funnels the word
+    // form takes last.
+    const uint2 *ev;
     const uint16_t *rest;   // candidates no funnel tests, ascending
     uint32_t fun_off[GBC_NCLASS], fun_cnt[GBC_NCLASS];
     uint32_t rest_off[GBC_NCLASS], rest_cnt[GBC_NCLASS];
     uint32_t ridge_min;     // evens with p(n) >= ridge_min are listed with their p(n)
-    uint32_t f1;            // funnels every word takes before the unresolved ones are gathered (>= 1)
+    uint32_t word;          // 1: the plan holds the word form's three funnels of every class
     uint32_t spin0;         // try_wait rounds of the first wait on a chunk's bulk copies (kStageSpin)
 };
 
@@ -279,8 +282,6 @@ constexpr uint32_t kErrHlOverflow = 1u << 10; // more hit-list overflow marks th
 
 // funnels per class the verify kernel holds (the plan has at most this many)
 constexpr uint32_t kVerifyMaxFun = 32;
-// shift groups (four shifts each) per funnel: pair starts, then single members
-constexpr uint32_t kVerifyMaxGroups = 9;
 
 // tiles per hit-list region k_binsort handles
 constexpr uint32_t kSortMaxTiles = 1024;
@@ -441,6 +442,7 @@ void launch_hl_overflow(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st
 void query_sieve_grids(Grids &g);
 void launch_check(const gbk::BatchDesc &d, const gbk::CheckTables &ct, const Grids &g, cudaStream_t st);
 void launch_verify(const gbk::BatchDesc &d, const gbk::VerifyTables &vt, const Grids &g, cudaStream_t st);
+void launch_tail(const gbk::BatchDesc &d, const gbk::VerifyTables &vt, const Grids &g, cudaStream_t st);
 void launch_retry(const gbk::BatchDesc &d, uint32_t ridge_min, uint32_t tries, const Grids &g, cudaStream_t st);
 void launch_count(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st);
 void launch_map_compare(const gbk::BatchDesc &a, const gbk::BatchDesc &b, uint32_t *count, const Grids &g,
@@ -450,8 +452,11 @@ void launch_map_compare(const gbk::BatchDesc &a, const gbk::BatchDesc &b, uint32
 // and returns false when the tile itself does not fit
 bool tile_attributes(uint32_t tile_bits, uint32_t tile_log2, const gbk::GroupInfo &gi, int device, uint32_t *stage);
 void query_check_grids(Grids &g);
+void query_verify_grids(Grids &g);
+bool verify_word_funnel(uint32_t r, uint32_t p0, uint32_t members);
 void query_count_grids(Grids &g);
 uint32_t check_vbx(uint64_t evens, int sm);
+uint32_t verify_vbx(uint64_t evens, int sm);
 // single-run forms (the allocation-free entry point and the table build)
 void launch_xfirst1(const gbk::BatchParams &bp, cudaStream_t st);
 void launch_tile1(const gbk::BatchParams &bp, const gbk::GroupInfo &gi, cudaStream_t st);

@@ -91,7 +91,7 @@ struct gbc_ctx {
     uint16_t *d_wheel = nullptr, *d_cand = nullptr, *d_list = nullptr;
     uint8_t *d_pk_gap = nullptr;   // packed large primes from n_mid: half gaps
     uint32_t *d_pk_base = nullptr; // and the first prime of each group
-    uint2 *d_fun = nullptr, *d_fpair = nullptr;
+    uint2 *d_ev = nullptr;
     uint16_t *d_rest = nullptr;
     gbk::GroupInfo gi{};
     gbk::CheckTables ct{};

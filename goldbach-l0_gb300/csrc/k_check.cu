@@ -410,317 +410,6 @@ __global__ void __launch_bounds__(64) k_retry(BatchDesc d, uint32_t ridge_min, u
     }
 }
 
-constexpr int kVerifyThreads = 128;
-constexpr uint32_t kVerifyWarps = kVerifyThreads / 32;
-constexpr uint32_t kVW = 6;                // words per lane in a chunk
-constexpr uint32_t kVChunk = 32 * kVW;     // words per warp chunk
-constexpr uint32_t kVWin = kVChunk + 12;   // staged words per class array and buffer: chunk + funnel span (<= 5) + 3 + alignment (<= 3), a multiple of 4
-constexpr uint32_t kMaxFun = kVerifyMaxFun;
-constexpr size_t kVerifySmem = size_t(kVerifyWarps) * 2 * 8 * kVWin * 4;  // k_verify's dynamic shared memory
-
-// one chunk's eight class-array windows into a staging buffer: 8 bulk
-// copies of `bytes` each, completing on bar (issued by one lane)
-__device__ __forceinline__ void stage_chunk(uint32_t *dst, uint64_t *bar, const uint32_t *src, uint32_t wpc,
-                                            uint32_t bytes)
-{
-    mbar_arrive_expect_tx(bar, 8 * bytes);
-#pragma unroll
-    for (uint32_t k = 0; k < 8; ++k) bulk_copy_g2s(dst + k * kVWin, src + size_t(k) * wpc, bytes, bar);
-}
-
-// Funnel entry in shared memory: staged word offset (12 bits) | shift << 12
-// | pair groups << 17 | single groups << 21 | delta << 25.
-static_assert(7 * kVWin + 7 < 4096, "staged word offsets must fit the funnel entry's 12 bits");
-__device__ __forceinline__ uint32_t fent_make(uint32_t off, uint32_t sh, uint32_t nga, uint32_t ngr, uint32_t delta)
-{
-    return off | (sh << 12) | (nga << 17) | (ngr << 21) | (delta << 25);
-}
-__device__ __forceinline__ uint32_t fent_off(uint32_t e) { return e & 0xFFFu; }
-__device__ __forceinline__ uint32_t fent_sh(uint32_t e) { return (e >> 12) & 31u; }
-__device__ __forceinline__ uint32_t fent_nga(uint32_t e) { return (e >> 17) & 15u; }
-__device__ __forceinline__ uint32_t fent_ngr(uint32_t e) { return (e >> 21) & 15u; }
-__device__ __forceinline__ uint32_t fent_delta(uint32_t e) { return e >> 25; }
-
-// ORs into wa the four shifted windows of one group (a funnel shift uses the
-// low 5 bits of its operand)
-__device__ __forceinline__ uint32_t group_hits(uint32_t lo, uint32_t hi, uint4 q)
-{
-    return __funnelshift_r(lo, hi, q.x) | __funnelshift_r(lo, hi, q.y) | __funnelshift_r(lo, hi, q.z) |
-           __funnelshift_r(lo, hi, q.w);
-}
-
-// The OR over one funnel's members of the 32 candidates' bits of word
-// window w (three staged words from w): the top member's 64-bit window at
-// bit sh, every other member's the same shifted down by its distance. A
-// pair of members a, a + delta is one shift of the window ORed with itself
-// shifted by delta (the bits a pair reads stay below 63).
-__device__ __forceinline__ uint32_t funnel_hits(const uint32_t *w, uint32_t e, const uint4 *fsh)
-{
-    const uint32_t x0 = w[0], x1 = w[1], x2 = w[2], sh = fent_sh(e), nga = fent_nga(e), ngr = fent_ngr(e);
-    const uint32_t al = __funnelshift_r(x0, x1, sh), ah = __funnelshift_r(x1, x2, sh);
-    uint32_t wa = 0;
-    if (nga) {
-        const uint32_t dl = fent_delta(e);
-        const uint32_t bl = al | __funnelshift_r(al, ah, dl), bh = ah | (ah >> dl);
-        for (uint32_t g = 0; g < nga; ++g) wa |= group_hits(bl, bh, fsh[g]);
-    }
-    for (uint32_t g = 0; g < ngr; ++g) wa |= group_hits(al, ah, fsh[nga + g]);
-    return wa;
-}
-
-// Phase A (the reference's check30_a, kernels/goldbach.cl:2029-2189): any
-// witness. Each funnel is a set of plan members p + 30 d (d < 32) of one
-// residue class, all prime, whose windows are the same staged words shifted
-// by their distance in bits, so one 96-bit read and one funnel shift per
-// member test up to 32 candidates for 32 evens. No statistics here: evens
-// left without a plan witness go to a pending list of (class, word, bits)
-// for k_tail.
-//
-// Staging: each warp double-buffers its 128-word chunks in shared memory;
-// one lane moves the next chunk's eight class-array windows with bulk
-// copies (cp.async.bulk on an mbarrier) while the warp tests the current
-// one. The windows start 16-byte aligned (the class arrays are, and chunks
-// are 128 words apart), o = 0..3 words below the lowest word a funnel reads.
-//
-// Work balance: every lane holds four words (words l, l + 32, l + 64, l + 96
-// of the chunk) through the plan's first f1 funnels, which leave about one
-// word in ten with an even still unresolved; the warp then gathers those
-// words, one per lane (in rounds of 32), for the plan's other funnels, so
-// the last funnels cost one word per lane instead of four and no lane waits
-// for the slowest even of 4096.
-__global__ void __launch_bounds__(kVerifyThreads, 3) k_verify(BatchDesc d, VerifyTables vt)
-{
-    __shared__ uint32_t s_fent[kMaxFun];  // see fent_off .. fent_delta
-    // per funnel: groups of four window offsets above the top member's, the
-    // pair starts first, then the single members, each padded with its first
-    __shared__ uint4 s_fsh[kMaxFun][kVerifyMaxGroups];
-    // per warp: two staging buffers of eight class-array windows (dynamic
-    // shared memory: kVerifySmem bytes)
-    extern __shared__ __align__(16) uint32_t s_dyn[];
-    uint32_t (*s_win)[2][8 * kVWin] = reinterpret_cast<uint32_t (*)[2][8 * kVWin]>(s_dyn);
-    __shared__ __align__(8) uint64_t s_bar[kVerifyWarps][2];
-    __shared__ uint32_t s_dmin, s_dmax;
-    __shared__ unsigned long long s_pend;
-
-    __shared__ uint32_t s_vb;
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    uint64_t *bar = s_bar[warp];
-    if (lane == 0) {
-        mbar_init(bar, 1);
-        mbar_init(bar + 1, 1);
-        mbar_init_fence();
-    }
-    __syncwarp();
-    uint32_t phase = 0;  // bit b: parity of buffer b's next completion
-    const uint32_t total = d.h->ver_vb, nseg = d.h->nseg;
-    for (;;) {
-        const uint32_t vb = next_item(d.work + kWorkVerify, &s_vb);
-        if (vb >= total) break;
-        const uint32_t si = find_prefix(d.ver_pref, nseg, vb);
-        const SegParams &sp = d.segs[si];
-        const BatchParams &bp = d.runs[sp.run];
-        const uint32_t local = vb - __ldg(d.ver_pref + si);
-        const uint32_t cr = local % GBC_NCLASS, bx = local / GBC_NCLASS, gx = sp.vbx, r = 2 * cr;
-        const uint64_t seg_start = sp.seg_start, base = bp.base;
-        const uint32_t wpc = bp.wpc;
-        const uint32_t *map = bp.map;
-        const uint64_t n0 = seg_start + (r + 30 - uint32_t(seg_start % 30)) % 30;
-        if (n0 > sp.seg_end) {
-            __syncthreads();
-            continue;
-        }
-        const uint64_t ecount = (sp.seg_end - n0) / 30 + 1;
-        const uint32_t nwords = uint32_t((ecount + 31) / 32);
-        const uint32_t nfun = vt.fun_cnt[cr] < kMaxFun ? vt.fun_cnt[cr] : kMaxFun;
-        const uint32_t f1 = vt.f1 < nfun ? vt.f1 : nfun;
-        gbc_segment_result *res = sp.res;
-        uint2 *pend_list = sp.pend;
-        const uint32_t pend_cap = sp.pend_cap;
-
-        if (tid == 0) {
-            s_dmin = kNone;
-            s_dmax = 0;
-            s_pend = 0;
-        }
-        __syncthreads();
-        // the lowest window bit of each funnel: its top member p + 30 d
-        for (uint32_t f = tid; f < nfun; f += blockDim.x) {
-            const uint2 e = vt.fun[vt.fun_off[cr] + f];
-            const uint32_t p0 = vt.cand[e.x], dm = 31 - __clz(e.y);
-            const uint32_t u = (r + 30 - p0 % 30) % 30;
-            const uint32_t dlow = uint32_t((n0 - base - p0 - u) / 30) - dm;
-            atomicMin(&s_dmin, dlow);
-            atomicMax(&s_dmax, dlow);
-        }
-        __syncthreads();
-        const uint32_t dlo = s_dmin & ~31u, o = (dlo >> 5) & 3u;
-        // words each class copy moves: the chunk, the funnels' span and the
-        // three words a 96-bit read needs, from the aligned start
-        const uint32_t cwords = nfun ? ((s_dmax - dlo) / 32 + kVChunk + 4 + o + 3) & ~3u : 0u;
-        if (cwords > kVWin) {  // funnel span beyond the staging buffer: nothing tested
-            if (tid == 0) atomicOr(&res->err, kErrStaging);
-            __syncthreads();
-            continue;
-        }
-        for (uint32_t f = tid; f < nfun; f += blockDim.x) {
-            const uint2 e = vt.fun[vt.fun_off[cr] + f];
-            const uint32_t p0 = vt.cand[e.x], dm = 31 - __clz(e.y);
-            const uint32_t u = (r + 30 - p0 % 30) % 30;
-            const uint32_t dd = uint32_t((n0 - base - p0 - u) / 30) - dm - dlo;
-            // member p0 + 30 d's window starts dm - d bits above the top
-            // member's (shift space, bit 0: the top member); the host's
-            // pairs {a, a + delta} take their members out of the singles
-            const uint2 pr = vt.fpair[vt.fun_off[cr] + f];
-            const uint32_t S = __brev(e.y) >> (31 - dm), dl = pr.x, A = pr.y;
-            const uint32_t R = S & ~(A | (dl ? A << dl : 0u));
-            uint32_t ng = 0, nga = 0;
-            for (uint32_t sel = 0; sel < 2; ++sel) {
-                uint32_t sm = sel ? R : A;
-                const uint32_t first = sm ? uint32_t(__ffs(sm) - 1) : 0u;
-                while (sm) {
-                    uint32_t q[4] = {first, first, first, first};
-#pragma unroll
-                    for (uint32_t j = 0; j < 4; ++j)
-                        if (sm) {
-                            q[j] = uint32_t(__ffs(sm) - 1);
-                            sm &= sm - 1u;
-                        }
-                    s_fsh[f][ng++] = make_uint4(q[0], q[1], q[2], q[3]);
-                }
-                if (!sel) nga = ng;
-            }
-            s_fent[f] = fent_make(class_of(u) * kVWin + o + (dd >> 5), dd & 31, nga, ng - nga, dl);
-        }
-        __syncthreads();
-
-        uint32_t pend = 0;
-        const uint32_t step = gx * kVerifyWarps;
-        if (nfun) {
-            const uint32_t bytes = cwords * 4;
-            const uint32_t *src0 = map + ((dlo >> 5) - o);
-            uint32_t ch = bx * kVerifyWarps + warp, buf = 0;
-            if (ch * kVChunk < nwords && lane == 0) {
-                fence_proxy_async();
-                stage_chunk(s_win[warp][0], bar, src0 + size_t(ch) * kVChunk, wpc, bytes);
-            }
-            for (; ch * kVChunk < nwords; ch += step, buf ^= 1u) {
-                const uint32_t nx = ch + step;
-                if (nx * kVChunk < nwords) {
-                    __syncwarp();  // every lane is done with the other buffer (the chunk before)
-                    if (lane == 0) {
-                        fence_proxy_async();
-                        stage_chunk(s_win[warp][buf ^ 1u], bar + (buf ^ 1u), src0 + size_t(nx) * kVChunk, wpc, bytes);
-                    }
-                }
-                if (!mbar_wait(bar + buf, (phase >> buf) & 1u, vt.spin0)) {
-                    atomicOr(&res->err, kErrStaging);
-                    mbar_wait(bar + buf, (phase >> buf) & 1u);
-                }
-                phase ^= 1u << buf;
-                const uint32_t J = ch * kVChunk;
-                const uint32_t *win = s_win[warp][buf];
-                uint32_t u[kVW];
-#pragma unroll
-                for (uint32_t w = 0; w < kVW; ++w) u[w] = word_mask(J + lane + 32 * w, ecount);
-                // the first f1 funnels on all four words of every lane
-                for (uint32_t f = 0; f < f1; ++f) {
-                    uint32_t any = 0;
-#pragma unroll
-                    for (uint32_t w = 0; w < kVW; ++w) any |= u[w];
-                    if (!__any_sync(~0u, any)) break;
-                    const uint32_t e = s_fent[f];
-                    const uint32_t *wl = win + lane + fent_off(e);
-                    const uint32_t sh = fent_sh(e), nga = fent_nga(e), ngr = fent_ngr(e), dl = fent_delta(e);
-                    uint32_t al[kVW], ah[kVW], wa[kVW];
-#pragma unroll
-                    for (uint32_t w = 0; w < kVW; ++w) {
-                        const uint32_t x0 = wl[32 * w], x1 = wl[32 * w + 1], x2 = wl[32 * w + 2];
-                        al[w] = __funnelshift_r(x0, x1, sh);
-                        ah[w] = __funnelshift_r(x1, x2, sh);
-                        wa[w] = 0;
-                    }
-                    if (nga) {
-                        uint32_t bl[kVW], bh[kVW];
-#pragma unroll
-                        for (uint32_t w = 0; w < kVW; ++w) {
-                            bl[w] = al[w] | __funnelshift_r(al[w], ah[w], dl);
-                            bh[w] = ah[w] | (ah[w] >> dl);
-                        }
-                        for (uint32_t g = 0; g < nga; ++g) {
-                            const uint4 q = s_fsh[f][g];
-#pragma unroll
-                            for (uint32_t w = 0; w < kVW; ++w) wa[w] |= group_hits(bl[w], bh[w], q);
-                        }
-                    }
-                    for (uint32_t g = 0; g < ngr; ++g) {
-                        const uint4 q = s_fsh[f][nga + g];
-#pragma unroll
-                        for (uint32_t w = 0; w < kVW; ++w) wa[w] |= group_hits(al[w], ah[w], q);
-                    }
-#pragma unroll
-                    for (uint32_t w = 0; w < kVW; ++w) u[w] &= ~wa[w];
-                }
-                // the words still unresolved, gathered one per lane (word
-                // order: w-major, then lane) for the other funnels
-                uint32_t bal[kVW], cpre[kVW], nun = 0;  // cpre[w]: unresolved words in w' <= w
-#pragma unroll
-                for (uint32_t w = 0; w < kVW; ++w) {
-                    bal[w] = __ballot_sync(~0u, u[w] != 0u);
-                    nun += __popc(bal[w]);
-                    cpre[w] = nun;
-                }
-                for (uint32_t r0 = 0; r0 < nun; r0 += 32) {
-                    const uint32_t t = r0 + lane;
-                    uint32_t wt = 0, before = 0, bm = bal[0];
-#pragma unroll
-                    for (uint32_t w = 0; w + 1 < kVW; ++w)
-                        if (t >= cpre[w]) {
-                            wt = w + 1;
-                            before = cpre[w];
-                            bm = bal[w + 1];
-                        }
-                    const uint32_t srcl = t < nun ? nth_set_bit(bm, t - before) : 0u;
-                    uint32_t uu = 0;
-#pragma unroll
-                    for (uint32_t w = 0; w < kVW; ++w) {
-                        const uint32_t v = __shfl_sync(~0u, u[w], srcl);
-                        if (w == wt) uu = v;
-                    }
-                    if (t >= nun) uu = 0;
-                    const uint32_t jl = srcl + 32 * wt;  // the word within the chunk
-                    for (uint32_t f = f1; f < nfun; ++f) {
-                        if (!__any_sync(~0u, uu)) break;
-                        const uint32_t e = s_fent[f];
-                        uu &= ~funnel_hits(win + jl + fent_off(e), e, s_fsh[f]);
-                    }
-                    if (uu) {  // every funnel tried: pending (rare)
-                        const uint32_t at = atomicAdd(&res->npend, 1u);
-                        if (at < pend_cap) pend_list[at] = make_uint2((cr << 27) | (J + jl), uu);
-                        else atomicOr(&res->err, kErrPendOverflow);
-                        pend += __popc(uu);
-                    }
-                }
-            }
-        } else {
-            // no funnels for the class: every word of the warp's chunks is pending
-            for (uint32_t ch = bx * kVerifyWarps + warp; ch * kVChunk < nwords; ch += step)
-                for (uint32_t jj = ch * kVChunk + lane; jj < ch * kVChunk + kVChunk; jj += 32) {
-                    const uint32_t uw = word_mask(jj, ecount);
-                    if (!uw) continue;
-                    const uint32_t at = atomicAdd(&res->npend, 1u);
-                    if (at < pend_cap) pend_list[at] = make_uint2((cr << 27) | jj, uw);
-                    else atomicOr(&res->err, kErrPendOverflow);
-                    pend += __popc(uw);
-                }
-        }
-        pend = __reduce_add_sync(~0u, pend);
-        if (lane == 0 && pend) atomicAdd(&s_pend, (unsigned long long)pend);
-        __syncthreads();
-        if (tid == 0 && s_pend) atomicAdd((unsigned long long *)&res->pending, s_pend);
-        __syncthreads();
-    }
-}
-
 // Phase B (the reference's check30_b, kernels/goldbach.cl:2210-2306): the
 // exact p(n) of every pending even, by the class's rest candidates in
 // ascending order (every plan member already failed for it), one thread per
@@ -853,9 +542,8 @@ void launch_check(const gbk::BatchDesc &d, const gbk::CheckTables &ct, const Gri
     gbk::k_check<<<g.sm * g.check, gbk::kCheckThreads, gbk::kCheckSmem, st>>>(d, ct);
 }
 
-void launch_verify(const gbk::BatchDesc &d, const gbk::VerifyTables &vt, const Grids &g, cudaStream_t st)
+void launch_tail(const gbk::BatchDesc &d, const gbk::VerifyTables &vt, const Grids &g, cudaStream_t st)
 {
-    gbk::k_verify<<<g.sm * g.verify, gbk::kVerifyThreads, gbk::kVerifySmem, st>>>(d, vt);
     gbk::k_tail<<<g.sm * 2, gbk::kTailThreads, 0, st>>>(d, vt);
 }
 
@@ -870,10 +558,6 @@ void query_check_grids(Grids &g)
     cudaFuncSetAttribute(gbk::k_check, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gbk::kCheckSmem));
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gbk::k_check, gbk::kCheckThreads, gbk::kCheckSmem);
     g.check = n > 0 ? n : 1;
-    n = 0;
-    cudaFuncSetAttribute(gbk::k_verify, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gbk::kVerifySmem));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gbk::k_verify, gbk::kVerifyThreads, gbk::kVerifySmem);
-    g.verify = n > 0 ? n : 1;
 }
 
 }  // namespace gbh

@@ -85,7 +85,8 @@ typedef struct gbc_config {
                                 run_pmax over tail counts alone, include/gstats.hpp:690-701) */
     uint32_t plan_funnels;   /* funnels per class of the verify plan (default 8, at most 32; below 6
                                 the evens a production segment leaves to the exact continuation can
-                                overflow its pending list, and the batch fails closed) */
+                                overflow its pending list, and the batch fails closed; below 5 the
+                                verify kernel takes every funnel even by even, which is slower) */
     uint32_t ridge_min;      /* evens with p(n) >= ridge_min are listed (default 3000,
                                 include/config.hpp:104 RIDGE_MIN_DEFAULT) */
     uint32_t launch_mode;    /* 0 or 1: a batch is one replay of the slot's CUDA graph of the whole
@@ -97,9 +98,9 @@ typedef struct gbc_config {
     uint32_t selfcheck_every;/* every selfcheck_every-th batch that uses hit lists rebuilds its maps
                                 without them and compares every word (src/verifier.cpp:2057-2112);
                                 a mismatch fails the batch closed. 0: never (default) */
-    uint32_t verify_funnels; /* funnels of the plan every word of a chunk takes before the verify
-                                kernel gathers the words still without a witness, one per lane, for
-                                the plan's other funnels (default 3; at most plan_funnels) */
+    uint32_t verify_funnels; /* accepted and reported for callers that set it (default 3; at most
+                                plan_funnels): the verify kernel takes three funnels of every class
+                                word by word, the plan's others even by even */
     uint32_t hl_cap_pct;     /* the hit-list bins' quotas and capacities in percent of their sizing
                                 (default 100; lower values make marks take the overflow list, which
                                 is cleared after the tiles: for tests of that path) */
