@@ -503,15 +503,28 @@ extern "C" int gbc_create(const gbc_config *cfg_in, gbc_ctx **out)
         return fail(ctx, GBC_E_ARG, "candidate count mismatch");
     }
     std::vector<uint16_t> cand(c32.begin(), c32.end()), list;
+    uint32_t list_off[GBC_NCLASS], list_cnt[GBC_NCLASS];
     for (int cr = 0; cr < GBC_NCLASS; ++cr) {
-        ctx->ct.off[cr] = uint32_t(list.size());
+        list_off[cr] = uint32_t(list.size());
         for (int i = 0; i < GBC_NCAND; ++i) {
             const uint32_t u = (2u * cr + 30 - cand[i] % 30) % 30;
             if (gbk::class_of(u) < 8) list.push_back(uint16_t(i));
         }
-        ctx->ct.cnt[cr] = uint32_t(list.size()) - ctx->ct.off[cr];
-        if (cfg.test_flags & GBC_TEST_RETRY_LIMIT) ctx->ct.cnt[cr] = std::min<uint32_t>(ctx->ct.cnt[cr], 1);
+        list_cnt[cr] = uint32_t(list.size()) - list_off[cr];
+        if (cfg.test_flags & GBC_TEST_RETRY_LIMIT) list_cnt[cr] = std::min<uint32_t>(list_cnt[cr], 1);
     }
+    // the exact checker's windows (CheckTables): candidate p of class r is at
+    // distance i blocks and class k with p = 30 i + r - u_k
+    std::vector<uint16_t> ck_ci(size_t(GBC_NCLASS) * gbk::kCkWindows * 64, 0);
+    std::vector<uint2> ck_mask(size_t(GBC_NCLASS) * gbk::kCkWindows, make_uint2(0u, 0u));
+    for (uint32_t cr = 0; cr < GBC_NCLASS; ++cr)
+        for (uint32_t li = list_off[cr]; li < list_off[cr] + list_cnt[cr]; ++li) {
+            const uint32_t p = cand[list[li]], u = (2 * cr + 30 - p % 30) % 30;
+            const uint32_t i = (p + u - 2 * cr) / 30, w = i / 8, b = 8 * (i % 8) + 7 - gbk::class_of(u);
+            ck_ci[(size_t(cr) * gbk::kCkWindows + w) * 64 + b] = list[li];
+            uint2 &m = ck_mask[size_t(cr) * gbk::kCkWindows + w];
+            (b < 32 ? m.y : m.x) |= 1u << (31 - b % 32);
+        }
     // verify plan (the reference's make_plan30, include/check30.hpp:88-174,
     // with our own greedy order): per class, the useful candidates below
     // GBC_TAIL_T in ascending order, each uncovered one p opening a funnel
@@ -529,7 +542,7 @@ extern "C" int gbc_create(const gbc_config *cfg_in, gbc_ctx **out)
         for (int cr = 0; cr < GBC_NCLASS; ++cr) {
             std::vector<char> covered(GBC_NCAND, 0);
             ctx->vt.fun_off[cr] = uint32_t(fun.size());
-            const uint32_t b = ctx->ct.off[cr], e = b + ctx->ct.cnt[cr];
+            const uint32_t b = list_off[cr], e = b + list_cnt[cr];
             for (uint32_t li = b; li < e; ++li) {
                 const int i = list[li];
                 if (fun.size() - ctx->vt.fun_off[cr] >= cfg.plan_funnels || cand[i] >= GBC_TAIL_T) break;
@@ -604,11 +617,19 @@ extern "C" int gbc_create(const gbc_config *cfg_in, gbc_ctx **out)
     }
     CK(dev_alloc(ctx, &ctx->d_cand, cand.size() * 2));
     CK(cudaMemcpy(ctx->d_cand, cand.data(), cand.size() * 2, cudaMemcpyHostToDevice));
-    CK(dev_alloc(ctx, &ctx->d_list, list.size() * 2));
-    CK(cudaMemcpy(ctx->d_list, list.data(), list.size() * 2, cudaMemcpyHostToDevice));
+    CK(dev_alloc(ctx, &ctx->d_ck_ci, ck_ci.size() * 2));
+    CK(cudaMemcpy(ctx->d_ck_ci, ck_ci.data(), ck_ci.size() * 2, cudaMemcpyHostToDevice));
+    CK(dev_alloc(ctx, &ctx->d_ck_mask, ck_mask.size() * sizeof(uint2)));
+    CK(cudaMemcpy(ctx->d_ck_mask, ck_mask.data(), ck_mask.size() * sizeof(uint2), cudaMemcpyHostToDevice));
     ctx->ct.cand = ctx->d_cand;
-    ctx->ct.list = ctx->d_list;
+    ctx->ct.ci = ctx->d_ck_ci;
+    ctx->ct.mask = ctx->d_ck_mask;
+    for (int cr = 0; cr < GBC_NCLASS; ++cr) {
+        ctx->ct.m0[cr] = ck_mask[size_t(cr) * gbk::kCkWindows];
+        ctx->ct.m1[cr] = ck_mask[size_t(cr) * gbk::kCkWindows + 1];
+    }
     ctx->ct.ridge_min = cfg.ridge_min;
+    ctx->ct.ridge_w = cfg.ridge_min < 240 ? 0 : std::min<uint32_t>((cfg.ridge_min - 237) / 240, gbk::kCkWindows);
     // the plan's funnels as k_verify reads them: per class those the word form
     // does not take first, in plan order
     ctx->vt.word = 1;
@@ -663,7 +684,8 @@ extern "C" void gbc_destroy(gbc_ctx *ctx)
     cudaFree(ctx->d_pk_gap);
     cudaFree(ctx->d_pk_base);
     cudaFree(ctx->d_cand);
-    cudaFree(ctx->d_list);
+    cudaFree(ctx->d_ck_ci);
+    cudaFree(ctx->d_ck_mask);
     delete ctx;
 }
 
@@ -804,15 +826,21 @@ static void finish_desc(const gbc_ctx *ctx, DescImage &img)
     img.tile_pref[nrun] = h.tile_items;
     if (!nrun) h.n_mid_min = h.n_hl_min = 0;
     h.chk_vb = h.ver_vb = h.cnt_vb = h.nlow = 0;
+    uint64_t sampled_words = 0;  // class words of the exact checker's segments
+    for (uint32_t i = 0; i < nseg; ++i) {
+        const gbk::SegParams &sp = img.segs[i];
+        if (sp.sampled && !sp.low) sampled_words += (sp.seg_end - sp.seg_start) / 960 + 2;
+    }
     for (uint32_t i = 0; i < nseg; ++i) {
         gbk::SegParams &sp = img.segs[i];
         img.chk_pref[i] = h.chk_vb;
         img.ver_pref[i] = h.ver_vb;
         img.cnt_pref[i] = h.cnt_vb;
         const uint64_t evens = (sp.seg_end - sp.seg_start) / 2 + 1;
-        sp.vbx = sp.sampled ? gbh::check_vbx(evens, ctx->grids.sm) : gbh::verify_vbx(evens, ctx->grids.sm);
+        if (sp.sampled) gbh::check_split(evens, sampled_words, ctx->grids.sm, &sp.cw, &sp.vbx);
+        else sp.vbx = gbh::verify_vbx(evens, ctx->grids.sm);
         if (sp.low) ++h.nlow;
-        else if (sp.sampled) h.chk_vb += GBC_NCLASS * sp.vbx;
+        else if (sp.sampled) h.chk_vb += sp.vbx;
         else h.ver_vb += sp.vbx;
         h.cnt_vb += gbh::count_ranges(img.runs[sp.run].base, sp, sp.cr);
     }

@@ -172,8 +172,8 @@ struct SegParams {
     uint2 *pend;                  // phase-A misses: (class r / 2 << 27 | word, unresolved bits)
     uint32_t pend_cap;
     uint32_t run;                 // the segment's run (class map) in the batch
-    uint32_t vbx;                 // checker CTAs of the segment: per class (sampled), in all (verify)
-    uint32_t pad;
+    uint32_t vbx;                 // checker CTAs of the segment
+    uint32_t cw;                  // words per chunk of the exact checker
     CountRanges cr;
 };
 
@@ -241,13 +241,49 @@ __device__ __forceinline__ uint32_t find_prefix(const uint32_t *pref, uint32_t n
     return lo;
 }
 
-// Candidate tables of the checker (uploaded once per context).
+// transpose of an 8 x 8 bit matrix: bit 8 i + j -> bit 8 j + i (the
+// delta-swap method of Warren, Hacker's Delight, section 7-3)
+__device__ __forceinline__ uint64_t transpose8(uint64_t x)
+{
+    uint64_t t;
+    t = (x ^ (x >> 7)) & 0x00AA00AA00AA00AAull;
+    x = x ^ t ^ (t << 7);
+    t = (x ^ (x >> 14)) & 0x0000CCCC0000CCCCull;
+    x = x ^ t ^ (t << 14);
+    t = (x ^ (x >> 28)) & 0x00000000F0F0F0F0ull;
+    x = x ^ t ^ (t << 28);
+    return x;
+}
+
+// a word of the eight class arrays as one byte per block of 30 (bit k: class
+// k), natural order: T[i] holds blocks 4 i .. 4 i + 3
+__device__ __forceinline__ void transpose_word(const uint32_t (&h)[8], uint32_t *T)
+{
+#pragma unroll
+    for (uint32_t g = 0; g < 4; ++g) {
+        const uint32_t sel = g | ((g + 4) << 4);
+        const uint32_t lo = __byte_perm(__byte_perm(h[0], h[1], sel), __byte_perm(h[2], h[3], sel), 0x5410);
+        const uint32_t hi = __byte_perm(__byte_perm(h[4], h[5], sel), __byte_perm(h[6], h[7], sel), 0x5410);
+        const uint64_t t = transpose8((uint64_t(hi) << 32) | lo);
+        T[2 * g] = uint32_t(t);
+        T[2 * g + 1] = uint32_t(t >> 32);
+    }
+}
+
+// windows of eight blocks the exact checker reads below an even: p <= 9781
+constexpr uint32_t kCkWindows = 41;
+
+// Candidate tables of the exact checker (uploaded once per context). Window
+// w of class c = r / 2 holds the blocks T - 8 w - 7 .. T - 8 w of the even
+// base + 30 T + r, 64 bits with the last block topmost; bit b from its top is
+// the q at distance p = 30 (8 w + b / 8) + r - u_k, k = 7 - b % 8.
 struct CheckTables {
     const uint16_t *cand;   // odd primes 3..9781
-    const uint16_t *list;   // per class r / 2: useful candidate indices ascending
-    uint32_t off[GBC_NCLASS];
-    uint32_t cnt[GBC_NCLASS];
+    const uint16_t *ci;     // [c][64 w + b]: the candidate's index
+    const uint2 *mask;      // [c][w]: the window's candidate bits (x: low, y: high word)
+    uint2 m0[GBC_NCLASS], m1[GBC_NCLASS];  // mask[c][0], mask[c][1]
     uint32_t ridge_min;     // evens with p(n) >= ridge_min are listed with their p(n)
+    uint32_t ridge_w;       // the first window with a candidate >= ridge_min
 };
 
 // Funnel plan of the verify (phase A) checker and the ascending rest lists
@@ -455,7 +491,7 @@ void query_check_grids(Grids &g);
 void query_verify_grids(Grids &g);
 bool verify_word_funnel(uint32_t r, uint32_t p0, uint32_t members);
 void query_count_grids(Grids &g);
-uint32_t check_vbx(uint64_t evens, int sm);
+void check_split(uint64_t evens, uint64_t words, int sm, uint32_t *cw, uint32_t *vbx);
 uint32_t verify_vbx(uint64_t evens, int sm);
 // single-run forms (the allocation-free entry point and the table build)
 void launch_xfirst1(const gbk::BatchParams &bp, cudaStream_t st);

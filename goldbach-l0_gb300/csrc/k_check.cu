@@ -1,24 +1,18 @@
 // k_check.cu -- the exact smallest Goldbach prime p(n) of every even.
 //
-// Evens are grouped by class r = n mod 30 (the reference's check30 layout,
-// include/check30.hpp:1-19): for a candidate p, q = n - p of every even of
-// class r lies in the class array of residue r - p, and consecutive evens of
-// the class are consecutive bits there, so one funnel shift tests 32 evens
-// (goldbach.cl:1950-2001). Unlike the reference's phase A (funnels of
-// several candidates, any witness), this checker tests the candidates of
-// each class in ascending order, so the first candidate that hits an even
-// IS p(n): the exact per-even result that the reference only computes on
-// sampled segments (check30_xs* + check30_xb, goldbach.cl:2339-2418,
-// 2880-3021). Per candidate, a warp reduction adds the hits to the
-// histogram and the first occurrence; evens left without a witness <= 9781
-// go to a list that k_retry settles on the GPU (the reference's CPU
-// fallback cpu_min_goldbach_prime, src/primes.cpp:482-493, moved on device).
+// The reference computes it on sampled segments (check30_xs* + check30_xb,
+// goldbach.cl:2339-2418, 2880-3021), testing candidates over words of 32
+// evens; here an even finds its smallest candidate in one or two 64-bit
+// windows of the map (k_check below). Evens left without a witness <= 9781
+// go to a list that k_retry settles on the GPU (the reference's CPU fallback
+// cpu_min_goldbach_prime, src/primes.cpp:482-493, moved on device).
 //
 // Every kernel here is persistent: a fixed grid takes the "virtual CTAs"
-// of all segments of the batch (per segment: vbx CTAs per class) from a
+// of all segments of the batch (per segment: vbx CTAs) from a
 // work counter, each found through the batch descriptor's prefix arrays.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstddef>
 
 #include "gbc_common.cuh"
@@ -43,287 +37,264 @@ __device__ __forceinline__ void append_ridge(gbc_segment_result *res, uint64_t n
     } else atomicOr(&res->err, kErrRidgeOverflow);
 }
 
-constexpr int kCheckThreads = 256;
-constexpr int kCheckWarps = kCheckThreads / 32;
-constexpr uint32_t kWL = 4;                 // words per lane of a warp's chunk
-constexpr uint32_t kChunk = 32 * kWL;       // words per chunk
-constexpr uint32_t kWin = kChunk + 16;      // staged words per class array per warp: chunk + span of the candidates + 2
-constexpr uint32_t kCheckSmem = kCheckWarps * 8 * kWin * 4;  // dynamic shared memory of k_check (bytes)
+// ---- p(n) of every even of a sampled segment -----------------------------------
+//
+// In class bits of a run the even n = base + 30 T + r and the prime q = base +
+// 30 (T - i) + u_k meet in p = 30 i + r - u_k: the largest q below n whose
+// distance is a candidate is the witness of p(n). So the class arrays are
+// transposed to one byte per block of 30 (bit k: class k), where q ascends, and
+// a 64-bit window of eight blocks ending at T is ANDed with the class's mask
+// of the candidates it reaches: its highest bit is p(n). The window of T serves
+// all fifteen classes (classes with few candidates in it take the next one
+// too); about 96 evens in a hundred are settled. The others go to a queue of the
+// warp, which takes the windows below (kCkWindows in all, the candidates to
+// 9781) one T per lane.
+//
+// A mark in the histogram is a shared-memory atomic at (class, bit of the
+// window), for the first kCkHist windows; at the item's end the bits become
+// candidates. First occurrences need a look only at candidates not seen
+// before the present part: an item's evens ascend from part to part.
+//
+// Bound by the ALU pipe (18 ALU of 32 instructions per 32 evens, issue 76%).
+// One GB300, p(n) of every even: 48 segments of 467.5M at 4e18 11.8 ms
+// against 17.6 for candidates tested over words of 32 evens until the last
+// even of 4096 was settled; 195 segments of uneven windows 36.5 against 53.4;
+// 1e7 evens at 1e12 with the p(n) array 0.08 against 1.45.
+constexpr int kCkThreads = 512;
+constexpr int kCkCtas = 2;                         // CTAs per SM
+constexpr uint32_t kCkWarps = kCkThreads / 32;
+constexpr uint32_t kCkHalo = 11;                   // words below a chunk: 41 windows of 8 blocks reach 335 back
+constexpr uint32_t kCkWords = kCkThreads - kCkHalo;  // words of a full chunk: one word per thread staged
+constexpr uint32_t kCkHist = 8;                    // windows counted in shared memory
+constexpr uint32_t kCkRow = 64 * kCkHist + 2;
+static_assert(32 * kCkHalo >= 8 * kCkWindows + 7, "the last window is staged");
 
-// valid-even mask of word j of a class with ecount evens
-__device__ __forceinline__ uint32_t word_mask(uint32_t j, uint64_t ecount)
+struct CkShared {
+    uint32_t hist[GBC_NCLASS][kCkRow];             // the windows' bits, after windows 0 and 1 one entry for none
+    uint4 mask[GBC_NCLASS][kCkWindows];            // x, y: the window's candidates; z, w: those seen before the part
+    uint32_t first[GBC_NCAND];
+    uint32_t slow;                                 // classes with a window-0 candidate not seen yet
+    uint32_t vb;
+    uint32_t queue[kCkWarps][32];                  // a step's T with open classes: classes << 16 | block in the chunk
+    __align__(16) uint32_t bytes[8 * kCkThreads + 4];  // one byte per block, halo first; a window reads three words
+};
+
+// bytes at - 7 .. at of the staged blocks as two words (byte `at` topmost)
+__device__ __forceinline__ void ck_window(const uint32_t *bytes, uint32_t at, uint32_t &lo, uint32_t &hi)
 {
-    const uint64_t e0 = uint64_t(j) * 32;
-    if (e0 >= ecount) return 0u;
-    return (ecount - e0 >= 32) ? ~0u : ((1u << uint32_t(ecount - e0)) - 1u);
+    const uint32_t a = at - 7, s = 8 * (a & 3u);
+    const uint32_t *w = bytes + (a >> 2);
+    const uint32_t w0 = w[0], w1 = w[1], w2 = w[2];
+    lo = __funnelshift_r(w0, w1, s);
+    hi = __funnelshift_r(w1, w2, s);
 }
 
-__device__ __forceinline__ void write_pn(uint16_t *pn, uint32_t idx0, uint32_t j, uint32_t h, uint16_t pv)
-{
-    while (h) {
-        const uint32_t b = __ffs(h) - 1u;
-        pn[idx0 + 15u * (32u * j + b)] = pv;
-        h &= h - 1u;
-    }
-}
+// Class c = r / 2 takes windows 0 and 1 at once, for every T: r is prime to 3
+// (19 or 26 candidates in a window, 39 or 50 in the others').
+__host__ __device__ __forceinline__ constexpr bool ck_wide(uint32_t c) { return c % 3 != 0; }
 
-// position of the k-th set bit (from 0) of m; m has more than k set bits
-__device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t k)
+__global__ void __launch_bounds__(kCkThreads, kCkCtas) k_check(BatchDesc d, CheckTables ct)
 {
-    uint32_t pos = 0;
-#pragma unroll
-    for (uint32_t s = 16; s > 0; s >>= 1) {
-        const uint32_t lo = __popc(m & ((1u << s) - 1u));
-        if (k >= lo) {
-            k -= lo;
-            m >>= s;
-            pos += s;
-        }
-    }
-    return pos;
-}
-
-// Virtual CTA (chunk column bx of vbx, class r) of a sampled segment; each
-// warp takes kChunk consecutive words (32 kWL words, 1024 kWL evens) of class
-// r at a time, stages the 8 class-array windows they read (the chunk + the
-// candidates' span) in its own shared memory, and tests the class's useful
-// candidates in ascending order: lane l holds words l, l + 32, ..., so every
-// shared-memory read of the warp is 32 consecutive words. Four words per
-// lane share each candidate's warp reduction and bookkeeping among 4096
-// evens: against two words per lane, the windows leg's checker took 200.2
-// instead of 239.7 ms and p(n) of every even on production segments ran at
-// 369 instead of 326 G evens/s (one GB300), although a chunk then waits for
-// the slowest of twice as many evens.
-__global__ void __launch_bounds__(kCheckThreads) k_check(BatchDesc d, CheckTables ct)
-{
-    __shared__ uint32_t s_ent[GBC_NCAND];   // word offset | shift << 16
-    __shared__ uint16_t s_p[GBC_NCAND];
-    __shared__ uint16_t s_ci[GBC_NCAND];
-    __shared__ uint32_t s_hist[GBC_NCAND];
-    __shared__ uint32_t s_first[GBC_NCAND];
-    extern __shared__ __align__(16) uint32_t s_chk_win[];  // kCheckWarps x 8 x kWin words
-    __shared__ uint32_t s_dmin, s_dmax, s_cridge;
-
-    __shared__ uint32_t s_vb;
+    extern __shared__ __align__(16) uint8_t s_ck[];
+    CkShared &sh = *reinterpret_cast<CkShared *>(s_ck);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t total = d.h->chk_vb, nseg = d.h->nseg;
+    uint32_t *const queue = sh.queue[warp];
+    for (uint32_t i = tid; i < GBC_NCLASS * kCkWindows; i += kCkThreads) {
+        const uint2 m = ct.mask[i];
+        sh.mask[0][i] = make_uint4(m.x, m.y, 0u, 0u);
+    }
     for (;;) {
-        const uint32_t vb = next_item(d.work + kWorkCheck, &s_vb);
+        const uint32_t vb = next_item(d.work + kWorkCheck, &sh.vb);  // synchronizes the CTA
         if (vb >= total) break;
         const uint32_t si = find_prefix(d.chk_pref, nseg, vb);
         const SegParams &sp = d.segs[si];
         const BatchParams &bp = d.runs[sp.run];
-        const uint32_t local = vb - __ldg(d.chk_pref + si);
-        const uint32_t cr = local % GBC_NCLASS, bx = local / GBC_NCLASS, gx = sp.vbx, r = 2 * cr;
-        const uint64_t seg_start = sp.seg_start, base = bp.base;
+        const uint32_t bx = vb - __ldg(d.chk_pref + si), cw = sp.cw;
         const uint32_t wpc = bp.wpc;
-        const uint32_t *map = bp.map;
-        gbc_segment_result *res = sp.res;
-        uint16_t *pn = sp.pn;
-        const uint64_t n0 = seg_start + (r + 30 - uint32_t(seg_start % 30)) % 30;  // first even of class r
-        if (n0 > sp.seg_end) {
+        const uint32_t *const map = bp.map;
+        gbc_segment_result *const res = sp.res;
+        uint16_t *const pn = sp.pn;
+        // the segment's evens: T in [A, B] of every class, without A of the
+        // classes below ra and B of those above rb; even (T, c) has index 15 T + c - D
+        const uint64_t da = sp.seg_start - bp.base, db = sp.seg_end - bp.base;
+        const uint32_t A = uint32_t(da / 30), ra = uint32_t(da % 30), B = uint32_t(db / 30), rb = uint32_t(db % 30);
+        const uint32_t D = uint32_t(da / 2);
+        const uint32_t jlo = A >> 5, jhi = B >> 5;
+        const uint32_t nch = (jhi - jlo) / cw + 1;
+        const uint32_t c0 = uint32_t(uint64_t(nch) * bx / sp.vbx), c1 = uint32_t(uint64_t(nch) * (bx + 1) / sp.vbx);
+        for (uint32_t i = tid; i < GBC_NCLASS * kCkRow; i += kCkThreads) sh.hist[0][i] = 0;
+        for (uint32_t i = tid; i < GBC_NCAND; i += kCkThreads) sh.first[i] = kNone;
+        // everything of an even but its histogram mark: first occurrence, p(n), ridge
+        auto note = [&](uint32_t c, uint32_t bit, uint32_t T) {
+            const uint32_t ci = __ldg(ct.ci + c * (64 * kCkWindows) + bit), idx = 15 * T + c - D;
+            if (sh.first[ci] > idx) atomicMin(&sh.first[ci], idx);
+            if (pn || bit >= 64 * ct.ridge_w) {
+                const uint32_t p = __ldg(ct.cand + ci);
+                if (pn) pn[idx] = uint16_t(p);
+                if (p >= ct.ridge_min) append_ridge(res, bp.base + 30ull * T + 2 * c, p);
+            }
+            return ci;
+        };
+        // The candidates of the counted windows seen before word j (every one
+        // when notes are for first occurrences only: p(n) and ridges note all):
+        // theirs cannot come first from j on. Between barriers.
+        auto look = [&](uint32_t j) {
+            if (tid == 0) sh.slow = 0;
             __syncthreads();
-            continue;
-        }
-        const uint64_t ecount = (sp.seg_end - n0) / 30 + 1;
-        const uint32_t nwords = uint32_t((ecount + 31) / 32);
-        const uint32_t ncand = ct.cnt[cr];
-
-        if (tid == 0) {
-            s_dmin = kNone;
-            s_dmax = 0;
-            s_cridge = ncand;  // the first candidate with p >= ridge_min (ascending list)
-        }
-        __syncthreads();
-        // q = n0 + 30 t - p = base + 30 (D + t) + u: D is the bit of the
-        // candidate's window at word 0 of class r
-        for (uint32_t c = tid; c < ncand; c += blockDim.x) {
-            const uint32_t ci = ct.list[ct.off[cr] + c];
-            const uint32_t p = ct.cand[ci];
-            const uint32_t D = uint32_t((n0 - base - p - (r + 30 - p % 30) % 30) / 30);
-            atomicMin(&s_dmin, D);
-            atomicMax(&s_dmax, D);
-        }
-        __syncthreads();
-        const uint32_t dlo = s_dmin & ~31u;                        // staged windows start at word dlo / 32 + J
-        const uint32_t nstage = (s_dmax - dlo) / 32 + kChunk + 2;  // words per class array (<= kWin)
-        for (uint32_t c = tid; c < ncand; c += blockDim.x) {
-            const uint32_t ci = ct.list[ct.off[cr] + c];
-            const uint32_t p = ct.cand[ci];
-            const uint32_t u = (r + 30 - p % 30) % 30;
-            const uint32_t dd = uint32_t((n0 - base - p - u) / 30) - dlo;
-            // word offset of the window in the warp's staging area | shift << 16
-            s_ent[c] = (class_of(u) * kWin + (dd >> 5)) | ((dd & 31) << 16);
-            if (p >= ct.ridge_min) atomicMin(&s_cridge, c);
-            s_p[c] = uint16_t(p);
-            s_ci[c] = uint16_t(ci);
-            s_hist[c] = 0;
-            s_first[c] = kNone;
-        }
-        __syncthreads();
-
-        const uint32_t idx0 = uint32_t((n0 - seg_start) / 2);  // index of n0 among the segment's evens
-        const uint32_t c_ridge = s_cridge;
-        uint32_t *win = s_chk_win + warp * (8 * kWin);
-        for (uint32_t ch = bx * kCheckWarps + warp; ch * kChunk < nwords; ch += gx * kCheckWarps) {
-            const uint32_t J = ch * kChunk;
-            // stage the windows: class array k, words dlo / 32 + J + [0, nstage)
-            const uint32_t *src = map + (dlo >> 5) + J;
-#pragma unroll
-            for (uint32_t k = 0; k < 8; ++k)
-                for (uint32_t i = lane; i < nstage; i += 32) win[k * kWin + i] = __ldg(src + size_t(k) * wpc + i);
-            __syncwarp();
-            uint32_t um[kWL];  // evens of word J + 32 w + lane still without a witness
-#pragma unroll
-            for (uint32_t w = 0; w < kWL; ++w) um[w] = word_mask(J + 32 * w + lane, ecount);
-            const uint32_t chunk_min = idx0 + 15u * 32u * J;  // smallest even index of this chunk
-            const uint32_t *wl = win + lane;
-            // records the hits h of candidate c (um already updated)
-            auto record = [&](uint32_t c, const uint32_t (&h)[kWL], uint32_t cnt) {
-                if (s_first[c] > chunk_min) {  // this chunk can still hold the first occurrence
-                    uint32_t mine = kNone;
-#pragma unroll
-                    for (int w = kWL - 1; w >= 0; --w)
-                        if (h[w]) mine = idx0 + 15u * (32u * (J + 32u * w + lane) + __ffs(h[w]) - 1u);
-                    const uint32_t mn = __reduce_min_sync(~0u, mine);
-                    if (lane == 0) atomicMin(&s_first[c], mn);
+            const uint32_t idx0 = j == jlo ? 0u : 15 * 32 * j - D;  // no even from word j on has a smaller index
+            for (uint32_t i = warp; i < GBC_NCLASS * kCkHist; i += kCkWarps) {
+                const uint32_t c = i / kCkHist, w = i % kCkHist;
+                const uint16_t *ci = ct.ci + c * (64 * kCkWindows) + 64 * w;
+                const uint4 m = sh.mask[c][w];
+                // lane l: bits l and 32 + l from the top
+                const bool hi = (m.y >> (31 - lane) & 1u) && sh.first[__ldg(ci + lane)] < idx0;
+                const bool lo = (m.x >> (31 - lane) & 1u) && sh.first[__ldg(ci + 32 + lane)] < idx0;
+                const uint32_t sy = __brev(__ballot_sync(~0u, hi)), sx = __brev(__ballot_sync(~0u, lo));
+                const bool all = pn || w >= ct.ridge_w;
+                if (lane == 0) {
+                    sh.mask[c][w].z = all ? 0u : sx;
+                    sh.mask[c][w].w = all ? 0u : sy;
+                    if ((w == 0 || (w == 1 && ck_wide(c))) && (all || sx != m.x || sy != m.y))
+                        atomicOr(&sh.slow, 1u << c);
                 }
-                if (lane == 0) atomicAdd(&s_hist[c], cnt);
-                if (pn) {
+            }
+            __syncthreads();
+        };
+        for (uint32_t ch = c0; ch < c1; ++ch) {
+            const uint32_t j0 = jlo + ch * cw, j1 = min(j0 + cw, jhi + 1);  // the chunk's words [j0, j1)
+            __syncthreads();  // the last chunk's bytes read, the item's tables ready
+            if (tid < j1 - j0 + kCkHalo) {
+                // word j of the eight arrays as 32 bytes (no block below the map)
+                const uint32_t j = j0 + tid - kCkHalo;
+                uint32_t h[8];
 #pragma unroll
-                    for (uint32_t w = 0; w < kWL; ++w) write_pn(pn, idx0, J + 32 * w + lane, h[w], s_p[c]);
-                }
-                if (c >= c_ridge) {
-#pragma unroll
-                    for (uint32_t w = 0; w < kWL; ++w)
-                        for (uint32_t x = h[w]; x; x &= x - 1u)
-                            append_ridge(res, n0 + 30ull * (32ull * (J + 32 * w + lane) + __ffs(x) - 1u), s_p[c]);
-                }
-            };
-            auto open = [&]() {
-                uint32_t o = 0;
-#pragma unroll
-                for (uint32_t w = 0; w < kWL; ++w) o |= um[w];
-                return __any_sync(~0u, o);
-            };
-            uint32_t c = 0;
-            bool gather = false;
-            // two candidates per trip: their window reads are independent; the
-            // second one only tests what the first one left. Every fourth trip
-            // counts the words still open: once they fit one per lane, they
-            // are gathered and take the remaining candidates one word per lane
-            // (p(n) of every even on 128 production segments: the checker
-            // 48.3 -> 46.7 ms)
-            for (; c + 1 < ncand; c += 2) {
-                if ((c & 7u) == 0) {
-                    uint32_t nopen = 0;
-#pragma unroll
-                    for (uint32_t w = 0; w < kWL; ++w) nopen += __popc(__ballot_sync(~0u, um[w] != 0));
-                    if (nopen <= 32) {
-                        gather = true;
+                for (uint32_t k = 0; k < 8; ++k) h[k] = j < wpc ? __ldg(map + size_t(k) * wpc + j) : 0u;
+                uint4 o[2];
+                uint32_t *t = reinterpret_cast<uint32_t *>(o);
+                transpose_word(h, t);
+                uint4 *dst = reinterpret_cast<uint4 *>(sh.bytes + 8 * tid);
+                dst[0] = o[0];
+                dst[1] = o[1];
+            }
+            look(j0);
+            // The classes of one T left open by window 0, one T per lane: the
+            // open classes qm, its block in the chunk, and for the highest open
+            // class the next window. A lane that is done takes the queue's last
+            // T. Ends with the queue empty (a T may stay with a lane), or with
+            // all settled.
+            uint32_t qn = 0, qm = 0, qt = 0, qw = 0;  // qw 0: the class's first queue window
+            auto settle = [&](bool finish) {
+                for (;;) {
+                    const uint32_t idle = __ballot_sync(~0u, qm == 0);
+                    if (qn) {
+                        const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
+                        if (qm == 0 && rank < qn) {
+                            const uint32_t e = queue[qn - 1 - rank];
+                            qm = e >> 16;
+                            qt = e & 0xFFFFu;
+                        }
+                        qn -= min(qn, uint32_t(__popc(idle)));
+                    } else if (!finish || idle == ~0u) {
                         break;
                     }
+                    // (an idle lane goes through the motions of class 0 without a mark)
+                    const bool busy = qm != 0;
+                    const uint32_t c = busy ? 31u - __clz(qm) : 0u;
+                    if (!qw) qw = ck_wide(c) ? 2u : 1u;
+                    uint32_t lo, hi;
+                    ck_window(sh.bytes, 32 * kCkHalo + qt - 8 * qw, lo, hi);
+                    const uint4 m = sh.mask[c][qw];
+                    lo &= m.x;
+                    hi &= m.y;
+                    const uint32_t z = hi ? hi : lo, b = __clz(z);
+                    const bool hit = busy && z;
+                    const uint32_t bit = 64 * qw + b + (hi ? 0u : 32u);
+                    if (hit && qw < kCkHist) atomicAdd(&sh.hist[c][bit + min(qw, 2u)], 1u);
+                    const bool seen = (hi ? m.w : m.z) << b >> 31;
+                    bool last = qw + 1 == kCkWindows;
+                    if ((hit && !seen) || (busy && last)) {  // rare
+                        if (hit) {
+                            const uint32_t ci = note(c, bit, 32 * j0 + qt);
+                            if (qw >= kCkHist) atomicAdd(&res->hist[c][ci], 1u);
+                        } else {
+                            append_leftover(res, bp.base + 30ull * (32 * j0 + qt) + 2 * c);
+                        }
+                    }
+                    __syncwarp();
+                    const bool done = hit || last;
+                    qw = done || !busy ? 0u : qw + 1;
+                    if (done) qm &= ~(1u << c);
                 }
-                const uint32_t e0 = s_ent[c], e1 = s_ent[c + 1];
-                const uint32_t *w0 = wl + (e0 & 0xFFFF), *w1 = wl + (e1 & 0xFFFF);
-                const uint32_t s0 = e0 >> 16, s1 = e1 >> 16;
-                uint32_t h0[kWL], h1[kWL], n0c = 0, n1c = 0;
+                __syncwarp();
+            };
+            // the item's first chunk in two parts: a few words, after which the
+            // window-0 candidates have been seen, then the others
+            const uint32_t jm = ch == c0 ? min(j0 + 4 * kCkWarps, j1) : j1;
+            for (uint32_t part = 0, ja = j0, jb = jm; ja < jb; ++part, ja = jm, jb = part == 1 ? j1 : jm) {
+                if (part) {
+                    __syncthreads();
+                    look(ja);
+                }
+                const uint32_t slow = sh.slow;
+                for (uint32_t j = ja + warp; j < jb; j += kCkWarps) {
+                    const uint32_t T = 32 * j + lane, tl = T - 32 * j0;
+                    uint32_t lo, hi, lo1, hi1, open = 0;  // open: classes these windows leave open at T
+                    ck_window(sh.bytes, 32 * kCkHalo + tl, lo, hi);
+                    ck_window(sh.bytes, 32 * kCkHalo + tl - 8, lo1, hi1);
+                    if (j > jlo && j < jhi && !slow) {
 #pragma unroll
-                for (uint32_t w = 0; w < kWL; ++w) {
-                    const uint32_t a0 = __funnelshift_r(w0[32 * w], w0[32 * w + 1], s0);
-                    const uint32_t a1 = __funnelshift_r(w1[32 * w], w1[32 * w + 1], s1);
-                    h0[w] = um[w] & a0;
-                    um[w] ^= h0[w];
-                    h1[w] = um[w] & a1;
-                    um[w] ^= h1[w];
-                    n0c += __popc(h0[w]);
-                    n1c += __popc(h1[w]);
+                        for (uint32_t c = 0; c < GBC_NCLASS; ++c) {
+                            // branchless: an even left open marks the row's entry for none
+                            const uint32_t y = lo & ct.m0[c].x;
+                            uint32_t z = hi & ct.m0[c].y, at = z ? 0u : 32u;
+                            z = z ? z : y;
+                            if (ck_wide(c)) {
+                                const uint32_t u = hi1 & ct.m1[c].y, v = lo1 & ct.m1[c].x;
+                                at = z ? at : 65u;
+                                z = z ? z : u;
+                                at = z ? at : 97u;
+                                z = z ? z : v;
+                            }
+                            atomicAdd(&sh.hist[c][at + __clz(z)], 1u);
+                            open |= z ? 0u : 1u << c;
+                        }
+                    } else {
+                        // a word at the segment's ends, or candidates not all seen yet
+#pragma unroll 1
+                        for (uint32_t c = 0; c < GBC_NCLASS; ++c) {
+                            const bool in = T >= A + (2 * c < ra ? 1u : 0u) && T <= B - (2 * c > rb ? 1u : 0u);
+                            const uint4 m = sh.mask[c][0], m1 = sh.mask[c][1];
+                            const uint32_t x = hi & m.y, y = lo & m.x;
+                            const uint32_t u = ck_wide(c) ? hi1 & m1.y : 0u, v = ck_wide(c) ? lo1 & m1.x : 0u;
+                            if (in && (x | y | u | v)) {
+                                const uint32_t bit =
+                                    x ? __clz(x) : y ? 32u + __clz(y) : u ? 64u + __clz(u) : 96u + __clz(v);
+                                atomicAdd(&sh.hist[c][bit + (bit >> 6)], 1u);
+                                if (slow >> c & 1u) note(c, bit, T);
+                            } else if (in) {
+                                open |= 1u << c;
+                            }
+                            __syncwarp();
+                        }
+                    }
+                    const uint32_t any = __ballot_sync(~0u, open != 0);
+                    if (open) queue[__popc(any & ((1u << lane) - 1u))] = (open << 16) | tl;
+                    qn = __popc(any);
+                    __syncwarp();
+                    settle(j + kCkWarps >= jb);
                 }
-                // both candidates' hit counts in one reduction (each <= 32 kWL 32 < 2^16)
-                const uint32_t cnt = __reduce_add_sync(~0u, n0c + (n1c << 16));
-                if (cnt & 0xFFFFu) record(c, h0, cnt & 0xFFFFu);
-                if (cnt >> 16) record(c + 1, h1, cnt >> 16);
             }
-            if (!gather) {
-                // the candidates ran out with more than 32 words open
-                if (c < ncand && open()) {
-                    const uint32_t e0 = s_ent[c];
-                    const uint32_t *w0 = wl + (e0 & 0xFFFF);
-                    const uint32_t s0 = e0 >> 16;
-                    uint32_t h0[kWL], n0c = 0;
-#pragma unroll
-                    for (uint32_t w = 0; w < kWL; ++w) {
-                        h0[w] = um[w] & __funnelshift_r(w0[32 * w], w0[32 * w + 1], s0);
-                        um[w] ^= h0[w];
-                        n0c += __popc(h0[w]);
-                    }
-                    const uint32_t cnt0 = __reduce_add_sync(~0u, n0c);
-                    if (cnt0) record(c, h0, cnt0);
-                }
-#pragma unroll
-                for (uint32_t w = 0; w < kWL; ++w)
-                    for (uint32_t x = um[w]; x; x &= x - 1u)
-                        append_leftover(res, n0 + 30ull * (32ull * (J + 32 * w + lane) + __ffs(x) - 1u));
-            } else {
-                // lane L takes the L-th open word, in (w, source lane) order
-                uint32_t ug = 0, jl = 0, rank = lane;
-                bool found = false;
-#pragma unroll
-                for (uint32_t w = 0; w < kWL; ++w) {
-                    const uint32_t b = __ballot_sync(~0u, um[w] != 0);
-                    const uint32_t nb = __popc(b);
-                    const bool mine = !found && rank < nb;
-                    const uint32_t src = mine ? nth_set_bit(b, rank) : lane;
-                    const uint32_t v = __shfl_sync(~0u, um[w], src);
-                    if (mine) {
-                        ug = v;
-                        jl = 32 * w + src;
-                        found = true;
-                    } else if (!found) {
-                        rank -= nb;
-                    }
-                }
-                const uint32_t *wg = win + jl;  // the lane's word in the staged windows
-                const uint32_t jw = J + jl;     // and in class r
-                auto record1 = [&](uint32_t cc, uint32_t h, uint32_t cnt) {
-                    if (s_first[cc] > chunk_min) {
-                        const uint32_t m1 = h ? idx0 + 15u * (32u * jw + __ffs(h) - 1u) : kNone;
-                        const uint32_t mn = __reduce_min_sync(~0u, m1);
-                        if (lane == 0) atomicMin(&s_first[cc], mn);
-                    }
-                    if (lane == 0) atomicAdd(&s_hist[cc], cnt);
-                    if (pn) write_pn(pn, idx0, jw, h, s_p[cc]);
-                    if (cc >= c_ridge)
-                        for (uint32_t x = h; x; x &= x - 1u)
-                            append_ridge(res, n0 + 30ull * (32ull * jw + __ffs(x) - 1u), s_p[cc]);
-                };
-                for (; c < ncand; c += 2) {
-                    if (!__any_sync(~0u, ug)) break;
-                    const uint32_t e0 = s_ent[c];
-                    const uint32_t o0 = e0 & 0xFFFF;
-                    const uint32_t h0 = ug & __funnelshift_r(wg[o0], wg[o0 + 1], e0 >> 16);
-                    ug ^= h0;
-                    uint32_t h1 = 0;
-                    if (c + 1 < ncand) {
-                        const uint32_t e1 = s_ent[c + 1];
-                        const uint32_t o1 = e1 & 0xFFFF;
-                        h1 = ug & __funnelshift_r(wg[o1], wg[o1 + 1], e1 >> 16);
-                        ug ^= h1;
-                    }
-                    const uint32_t cnt = __reduce_add_sync(~0u, __popc(h0) + (__popc(h1) << 16));
-                    if (cnt & 0xFFFFu) record1(c, h0, cnt & 0xFFFFu);
-                    if (cnt >> 16) record1(c + 1, h1, cnt >> 16);
-                }
-                for (uint32_t x = ug; x; x &= x - 1u)
-                    append_leftover(res, n0 + 30ull * (32ull * jw + __ffs(x) - 1u));
-            }
-            __syncwarp();
         }
         __syncthreads();
-        for (uint32_t c = tid; c < ncand; c += blockDim.x) {
-            if (s_hist[c]) atomicAdd(&res->hist[cr][s_ci[c]], s_hist[c]);
-            if (s_first[c] != kNone) atomicMin(&res->first[s_ci[c]], s_first[c]);
+        for (uint32_t i = tid; i < GBC_NCLASS * kCkRow; i += kCkThreads) {
+            const uint32_t v = sh.hist[0][i], c = i / kCkRow, at = i % kCkRow;
+            if (!v || at == 64 || at == 129) continue;
+            const uint32_t bit = at - (at > 129 ? 2u : at > 64 ? 1u : 0u);
+            atomicAdd(&res->hist[c][__ldg(ct.ci + c * (64 * kCkWindows) + bit)], v);
         }
+        for (uint32_t i = tid; i < GBC_NCAND; i += kCkThreads)
+            if (sh.first[i] != kNone) atomicMin(&res->first[i], sh.first[i]);
         __syncthreads();
     }
 }
@@ -520,26 +491,24 @@ void launch_init(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st)
     gbk::k_init<<<g.sm * 2, 256, 0, st>>>(d);
 }
 
-// checker CTAs per class of a segment with the given evens (a virtual grid
-// column count: each warp about twelve chunks of 128 words, to spread the
-// CTA's table setup; at most two per SM). Measured per 128-segment batch
-// with every segment sampled, three / six / twelve chunks per warp: 55.4 /
-// 50.7 / 48.3 ms.
-uint32_t check_vbx(uint64_t evens, int sm)
+// words per chunk and CTAs of a sampled segment: full chunks, up to 16 per CTA
+// while the batch (words: of all its sampled segments) keeps three CTAs per
+// resident one (a CTA clears and flushes 31 KB of counts); below that shorter
+// chunks, down to a word per warp: 5e5 evens take 0.03 ms, against 0.06 on one CTA a class.
+void check_split(uint64_t evens, uint64_t words, int sm, uint32_t *cw, uint32_t *vbx)
 {
-    const uint64_t words = (evens / 15 + 32) / 32 + 1;
-    constexpr uint64_t kPerVb = gbk::kCheckWarps * gbk::kChunk * 12;  // about twelve chunks per warp
-    uint64_t bx = (words + kPerVb - 1) / kPerVb;
-    const uint64_t cap = uint64_t(sm) * 2;
-    if (bx > cap) bx = cap;
-    if (bx < 1) bx = 1;
-    return uint32_t(bx);
+    const uint64_t mine = evens / 15 / 32 + 2, want = uint64_t(sm) * gbk::kCkCtas;
+    const uint64_t w = (words + want - 1) / want;
+    *cw = uint32_t(w < gbk::kCkWarps ? gbk::kCkWarps : w > gbk::kCkWords ? gbk::kCkWords : w);
+    const uint64_t nch = (mine + *cw - 1) / *cw;
+    const uint64_t per = std::min<uint64_t>(16, std::max<uint64_t>(1, words / *cw / (3 * want)));
+    *vbx = uint32_t((nch + per - 1) / per);
 }
 
 void launch_check(const gbk::BatchDesc &d, const gbk::CheckTables &ct, const Grids &g, cudaStream_t st)
 {
     gbk::k_check_low<<<g.sm * 16, 256, 0, st>>>(d, ct.cand, ct.ridge_min);
-    gbk::k_check<<<g.sm * g.check, gbk::kCheckThreads, gbk::kCheckSmem, st>>>(d, ct);
+    gbk::k_check<<<g.sm * g.check, gbk::kCkThreads, sizeof(gbk::CkShared), st>>>(d, ct);
 }
 
 void launch_tail(const gbk::BatchDesc &d, const gbk::VerifyTables &vt, const Grids &g, cudaStream_t st)
@@ -555,8 +524,8 @@ void launch_retry(const gbk::BatchDesc &d, uint32_t ridge_min, uint32_t tries, c
 void query_check_grids(Grids &g)
 {
     int n = 0;
-    cudaFuncSetAttribute(gbk::k_check, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gbk::kCheckSmem));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gbk::k_check, gbk::kCheckThreads, gbk::kCheckSmem);
+    cudaFuncSetAttribute(gbk::k_check, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(gbk::CkShared)));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gbk::k_check, gbk::kCkThreads, sizeof(gbk::CkShared));
     g.check = n > 0 ? n : 1;
 }
 

@@ -42,20 +42,6 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t q)
     return z ^ (z >> 31);
 }
 
-// transpose of an 8 x 8 bit matrix: bit 8 i + j -> bit 8 j + i (the
-// delta-swap method of Warren, Hacker's Delight, section 7-3)
-__device__ __forceinline__ uint64_t transpose8(uint64_t x)
-{
-    uint64_t t;
-    t = (x ^ (x >> 7)) & 0x00AA00AA00AA00AAull;
-    x = x ^ t ^ (t << 7);
-    t = (x ^ (x >> 14)) & 0x0000CCCC0000CCCCull;
-    x = x ^ t ^ (t << 14);
-    t = (x ^ (x >> 28)) & 0x00000000F0F0F0F0ull;
-    x = x ^ t ^ (t << 28);
-    return x;
-}
-
 // x - q0 as int32, clamped to +-2^30
 __device__ __forceinline__ int32_t rel_clamp(uint64_t x, uint64_t q0)
 {
@@ -156,15 +142,7 @@ __global__ void __launch_bounds__(kCountThreads, 6) k_count(BatchDesc d)
 
             // one byte per block, natural order: word i of T holds blocks 4 i .. 4 i + 3
             uint32_t T[8];
-    #pragma unroll
-            for (uint32_t g = 0; g < 4; ++g) {
-                const uint32_t sel = g | ((g + 4) << 4);
-                const uint32_t lo = __byte_perm(__byte_perm(h[0], h[1], sel), __byte_perm(h[2], h[3], sel), 0x5410);
-                const uint32_t hi = __byte_perm(__byte_perm(h[4], h[5], sel), __byte_perm(h[6], h[7], sel), 0x5410);
-                const uint64_t t = transpose8((uint64_t(hi) << 32) | lo);
-                T[2 * g] = uint32_t(t);
-                T[2 * g + 1] = uint32_t(t >> 32);
-            }
+            transpose_word(h, T);
             const int32_t cbase = int32_t(960 * (rd * kCountThreads + tid));  // this thread's first block
             uint32_t nh = 0;
     #pragma unroll

@@ -83,3 +83,39 @@ def test_pending_evens_are_the_plans(funnels):
                     hist[r // 2, CAND.index(p)] += 1
             assert (s.pending, s.npend, s.nleft, s.err) == (pend, words, 0, 0), (a, w)
             assert np.array_equal(np.frombuffer(s.hist, dtype=np.uint32).reshape(15, -1), hist), (a, w)
+
+
+@pytest.mark.parametrize("want_pn", [False, True])
+def test_exact_checker_edges(want_pn):
+    """p(n) of every even on the same segments: the histogram by class, the
+    first occurrences, the ridges from a low floor, and the p(n) array."""
+    floor = 500
+    for a, w in CASES:
+        b = a + w - 2
+        with gbc.Context(limit=BASE + 10**7, segment_even=4_000_000, max_batch=1, want_pn=want_pn,
+                         ridge_min=floor if w < 10_000 else 3000) as c:
+            c.enqueue_batch(0, [(a, b)], b)
+            (s,), _ = c.collect(0, 1)
+            got_pn = np.frombuffer(c.copy_pn(0, 0, w // 2), dtype=np.uint16) if want_pn else None
+        prime = is_prime_window(a - 9790, b)
+        n = np.arange(a, b + 1, 2)
+        pn = np.zeros(len(n), dtype=np.int64)
+        open_ = np.arange(len(n))
+        for p in CAND:
+            hit = prime[n[open_] - p - (a - 9790)]
+            pn[open_[hit]] = p
+            open_ = open_[~hit]
+        assert not len(open_)
+        index = {p: i for i, p in enumerate(CAND)}
+        hist = np.zeros((15, gbc.NCAND), dtype=np.int64)
+        first = np.full(gbc.NCAND, 0xFFFFFFFF, dtype=np.int64)
+        ci = np.array([index[p] for p in pn])
+        np.add.at(hist, (n % 30 // 2, ci), 1)
+        np.minimum.at(first, ci, np.arange(len(n)))
+        assert np.array_equal(np.frombuffer(s.hist, dtype=np.uint32).reshape(15, -1), hist), (a, w)
+        assert np.array_equal(np.frombuffer(s.first, dtype=np.uint32), first), (a, w)
+        ridges = sorted(zip(s.ridge_n[:s.nridge], s.ridge_p[:s.nridge]))
+        at = pn >= (floor if w < 10_000 else 3000)
+        assert ridges == list(zip(n[at].tolist(), pn[at].tolist())), (a, w)
+        if want_pn:
+            assert np.array_equal(got_pn, pn), (a, w)
