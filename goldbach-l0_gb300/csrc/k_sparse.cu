@@ -25,10 +25,12 @@
 //               staged in shared memory by bulk copies (two buffers: the next
 //               item's copies land while this one is checked); a warp takes an
 //               even class, each lane four words of its evens, and ORs in the
-//               plan entries (class, window word, up to six packed offsets) in
-//               plan order until every even of the warp is verified; words left
-//               unverified go to the pending list, which the host resolves by
-//               an ascending Miller-Rabin scan.
+//               entries (class, window word, up to six packed offsets) of the
+//               plan's first three groups; the evens still open, about one in
+//               a hundred, are then taken one per lane, a group as one 32-bit window
+//               of its row ANDed with the group's candidates; evens no group
+//               verifies go to the pending list, which the host resolves by an
+//               ascending Miller-Rabin scan.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -59,6 +61,7 @@ constexpr uint32_t kClassBlocks = (kHalfM + kClassBlock - 1) / kClassBlock;
 constexpr uint32_t kPendCap = 1u << 20;      // pending words per segment
 constexpr uint32_t kErrStaging = 1u << 0;    // a bulk copy missed its wait limit
 constexpr uint32_t kEntryMax = 6;            // candidates per plan entry
+constexpr uint32_t kWordGroups = 3;          // plan groups every word takes before its open evens
 
 // A plan entry: up to six candidates of one class k and one window word o,
 // as x = k | o << 4 | count << 12 and y = their offsets within the word, 5
@@ -217,10 +220,21 @@ __device__ __forceinline__ void sp_stage(const SpSeg &s, uint32_t *buf, uint64_t
         gbk::bulk_copy_g2s(buf + k * s.rw, s.map + size_t(k) * s.stride + size_t(c) * kChunkWords, s.rw * 4, bar);
 }
 
+// The word form costs a word of 32 evens a funnel shift and half a three-input
+// OR per candidate, however many of its evens are open; the even form about 35
+// instructions for the 10 to 17 candidates of a group. An even is verified by
+// a candidate with probability 0.12 at 4e18, so after the 50 or so candidates
+// of the three fullest groups the even form is the cheaper one. With a
+// group_cap every word takes the capped entries, word by word.
+// Bound by the ALU pipe (83%). One GB300, 1.05e12 evens at 4e18: 244.0 ms
+// (two groups word by word: 251.7) against 321.6 for entries word by word
+// until every even of 4096 was verified.
 __global__ void __launch_bounds__(kCheckThreads, 4) k_sp_check(SpSeg s, const uint2 *groups, const uint32_t *goff,
-                                                            uint4 *pend)
+                                                            const uint2 *masks, const uint2 *cls, uint4 *pend)
 {
     extern __shared__ __align__(16) uint32_t win[];  // two buffers of kK * rw words
+    __shared__ uint32_t s_qbits[kCheckWarps][kChunkWords];  // a task's words with open evens: their bits
+    __shared__ uint8_t s_qword[kCheckWarps][kChunkWords];   // and which word
     __shared__ uint64_t s_bar[2];
     __shared__ uint32_t s_j[2];  // alternate: no barrier separates two item fetches
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -232,6 +246,9 @@ __global__ void __launch_bounds__(kCheckThreads, 4) k_sp_check(SpSeg s, const ui
     }
     uint32_t phase = 0, buf = 0;
     unsigned long long ngroups = 0, nevens = 0;
+    const bool capped = s.group_cap != ~0u;
+    uint32_t *const q_bits = s_qbits[warp];
+    uint8_t *const q_word = s_qword[warp];
     uint32_t j = gbk::next_item(&s.ctr->work_check, &s_j[0]);
     if (j < items && tid == 0) sp_stage(s, win, &s_bar[0], j / kClassBlocks);
     while (j < items) {
@@ -260,9 +277,11 @@ __global__ void __launch_bounds__(kCheckThreads, 4) k_sp_check(SpSeg s, const ui
             // the group ranges of the warp's next 32 classes, one per lane
             const uint32_t mine = q0 + lane * kCheckWarps;
             uint32_t lg0 = 0, lg1 = 0;
+            uint2 lcls = make_uint2(0u, 0u);
             if (mine < cr1) {
                 lg0 = __ldg(goff + mine);
-                lg1 = lg0 + min(__ldg(goff + mine + 1) - lg0, s.group_cap);
+                lcls = __ldg(cls + mine);
+                lg1 = capped ? lg0 + min(__ldg(goff + mine + 1) - lg0, s.group_cap) : lg0 + (lcls.y >> 16);
             }
             const uint32_t nt = min(32u, (cr1 - q0 + kCheckWarps - 1) / kCheckWarps);
             for (uint32_t tj = 0; tj < nt; ++tj) {
@@ -295,7 +314,7 @@ __global__ void __launch_bounds__(kCheckThreads, 4) k_sp_check(SpSeg s, const ui
                     if (__all_sync(~0u, all == ~0u)) continue;
                 }
                 // the groups in plan order, 32 entries per coalesced load
-                uint32_t g = g0;
+                uint32_t g = g0, head = ~0u, a[kV] = {}, b[kV] = {};
                 bool done = false;
                 while (!done && g < g1) {
                     const uint32_t ng = min(32u, g1 - g);
@@ -305,12 +324,15 @@ __global__ void __launch_bounds__(kCheckThreads, 4) k_sp_check(SpSeg s, const ui
                     while (u < ng) {
                         const uint32_t ex = __shfl_sync(~0u, le.x, u), ey = __shfl_sync(~0u, le.y, u);
                         ++u;
-                        const uint32_t *row = w0 + entry_k(ex) * s.rw + entry_o(ex) + lane;
-                        uint32_t a[kV], b[kV];
+                        // a group's entries share their window
+                        if ((ex & 0xFFFu) != head) {
+                            head = ex & 0xFFFu;
+                            const uint32_t *row = w0 + entry_k(ex) * s.rw + entry_o(ex) + lane;
 #pragma unroll
-                        for (uint32_t v = 0; v < kV; ++v) {
-                            a[v] = row[32 * v];
-                            b[v] = row[32 * v + 1];
+                            for (uint32_t v = 0; v < kV; ++v) {
+                                a[v] = row[32 * v];
+                                b[v] = row[32 * v + 1];
+                            }
                         }
                         // two candidates per step
                         const uint32_t np = (entry_n(ex) + 1) >> 1;
@@ -324,6 +346,7 @@ __global__ void __launch_bounds__(kCheckThreads, 4) k_sp_check(SpSeg s, const ui
                                     f[v] |= __funnelshift_r(a[v], b[v], y) | __funnelshift_r(a[v], b[v], y2);
                                 y >>= 10;
                             }
+                        if (!capped) continue;
                         uint32_t all = f[0];
 #pragma unroll
                         for (uint32_t v = 1; v < kV; ++v) all &= f[v];
@@ -335,12 +358,63 @@ __global__ void __launch_bounds__(kCheckThreads, 4) k_sp_check(SpSeg s, const ui
                     g += u;
                 }
                 ngroups += g - g0;
+                auto leave = [&](uint32_t word, uint32_t bits) {
+                    const uint32_t slot = atomicAdd(&s.ctr->npend, 1u);
+                    if (slot < kPendCap) pend[slot] = make_uint4(cr, c * kChunkWords + word, bits, 0u);
+                };
+                if (capped) {
 #pragma unroll
-                for (uint32_t v = 0; v < kV; ++v)
+                    for (uint32_t v = 0; v < kV; ++v)
+                        if (f[v] != ~0u) leave(32 * v + lane, ~f[v]);
+                    continue;
+                }
+                // the words with open evens into the queue
+                uint32_t qn = 0;
+#pragma unroll
+                for (uint32_t v = 0; v < kV; ++v) {
+                    const uint32_t bal = __ballot_sync(~0u, f[v] != ~0u);
                     if (f[v] != ~0u) {
-                        const uint32_t slot = atomicAdd(&s.ctr->npend, 1u);
-                        if (slot < kPendCap) pend[slot] = make_uint4(cr, c * kChunkWords + 32 * v + lane, ~f[v], 0u);
+                        const uint32_t at = qn + __popc(bal & ((1u << lane) - 1u));
+                        q_bits[at] = ~f[v];
+                        q_word[at] = uint8_t(32 * v + lane);
                     }
+                    qn += __popc(bal);
+                }
+                __syncwarp();
+                // even by even: a lane takes a word, then the queue's last one;
+                // the class's next 32 groups one per lane
+                const uint32_t m0 = __shfl_sync(~0u, lcls.x, tj), mn = __shfl_sync(~0u, lcls.y, tj) & 0xFFFFu;
+                const uint2 lm = lane < mn ? __ldg(masks + m0 + lane) : make_uint2(0u, 0u);
+                uint32_t m = 0, word = 0, h = 0;
+                for (;;) {
+                    const uint32_t idle = __ballot_sync(~0u, m == 0);
+                    if (qn) {
+                        const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
+                        if (m == 0 && rank < qn) {
+                            m = q_bits[qn - 1 - rank];
+                            word = q_word[qn - 1 - rank];
+                        }
+                        qn -= min(qn, uint32_t(__popc(idle)));
+                    } else if (idle == ~0u) {
+                        break;
+                    }
+                    uint2 e;
+                    e.x = __shfl_sync(~0u, lm.x, h & 31u);
+                    e.y = __shfl_sync(~0u, lm.y, h & 31u);
+                    if (h >= 32) e = h < mn ? __ldg(masks + m0 + h) : make_uint2(0u, 0u);
+                    const uint32_t b = 31u - __clz(m | 1u);
+                    const uint32_t *row = w0 + entry_k(e.x) * s.rw + entry_o(e.x) + word;
+                    const bool hit = (__funnelshift_r(row[0], row[1], b) & e.y) != 0;
+                    ++h;
+                    const bool lost = !hit && h >= mn;  // every group tried (rare)
+                    if (lost && m) leave(word, 1u << b);
+                    if (hit || lost) {
+                        m &= ~(1u << b);
+                        h = 0;
+                    }
+                    if (m == 0) h = 0;
+                }
+                __syncwarp();
             }
         }
         j = jn;
@@ -401,6 +475,8 @@ struct gbc_sparse {
     uint32_t *d_xf = nullptr;
     uint2 *d_groups = nullptr;
     uint32_t *d_goff = nullptr;
+    uint2 *d_masks = nullptr;              // the groups after the first kWordGroups: class | word << 4, offsets as a mask
+    uint2 *d_cls = nullptr;                // per even class: first mask, masks | entries of the first groups << 16
     uint32_t *d_map = nullptr;
     uint32_t *d_out = nullptr;             // witness output
     uint32_t out_cap = 0;
@@ -615,6 +691,30 @@ bool validate_plan(const gbc_sparse *sp, const std::vector<uint8_t> &isp, std::s
     return true;
 }
 
+// The plan as the checker's even form reads it: per even class the entries of
+// its first kWordGroups groups counted, every later group as one mask.
+void group_masks(const gbc_sparse *sp, std::vector<uint2> &masks, std::vector<uint2> &cls)
+{
+    cls.assign(kHalfM, make_uint2(0u, 0u));
+    for (uint32_t x = 0; x < kHalfM; ++x) {
+        uint32_t seen = 0, head = 0, entries = 0;
+        cls[x].x = uint32_t(masks.size());
+        for (uint32_t g = sp->goff[x]; g < sp->goff[x + 1]; ++g) {
+            const uint2 e = sp->groups[g];
+            const uint32_t h = e.x & 0xFFFu;  // class and window word
+            if (!seen || h != head) {
+                ++seen;
+                head = h;
+                if (seen > kWordGroups) masks.push_back(make_uint2(h, 0u));
+            }
+            if (seen <= kWordGroups) ++entries;
+            else
+                for (uint32_t q = 0; q < entry_n(e.x); ++q) masks.back().y |= 1u << ((e.y >> (5 * q)) & 31u);
+        }
+        cls[x].y = (uint32_t(masks.size()) - cls[x].x) | entries << 16;
+    }
+}
+
 SpSeg make_seg(const gbc_sparse *sp, uint64_t N, uint32_t dl, uint64_t start, uint64_t limit)
 {
     SpSeg s{};
@@ -745,6 +845,15 @@ extern "C" int gbc_sparse_create(const gbc_sparse_config *cfg_in, gbc_sparse **o
         SPCK(cudaMemcpy(sp->d_groups, sp->groups.data(), sp->groups.size() * sizeof(uint2), cudaMemcpyHostToDevice));
     SPCK(cudaMalloc(&sp->d_goff, (kHalfM + 1) * 4));
     SPCK(cudaMemcpy(sp->d_goff, sp->goff.data(), (kHalfM + 1) * 4, cudaMemcpyHostToDevice));
+    {
+        std::vector<uint2> masks, cls;
+        group_masks(sp, masks, cls);
+        SPCK(cudaMalloc(&sp->d_masks, std::max<size_t>(masks.size(), 1) * sizeof(uint2)));
+        if (!masks.empty())
+            SPCK(cudaMemcpy(sp->d_masks, masks.data(), masks.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+        SPCK(cudaMalloc(&sp->d_cls, cls.size() * sizeof(uint2)));
+        SPCK(cudaMemcpy(sp->d_cls, cls.data(), cls.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+    }
     SPCK(cudaMalloc(&sp->d_map, size_t(kK) * sp->stride * 4));
     SPCK(cudaMemset(sp->d_map, 0, size_t(kK) * sp->stride * 4));
     SPCK(cudaMalloc(&sp->d_ctr, sizeof(SpCtr)));
@@ -767,6 +876,8 @@ extern "C" void gbc_sparse_destroy(gbc_sparse *sp)
     cudaFree(sp->d_xf);
     cudaFree(sp->d_groups);
     cudaFree(sp->d_goff);
+    cudaFree(sp->d_masks);
+    cudaFree(sp->d_cls);
     cudaFree(sp->d_map);
     cudaFree(sp->d_out);
     cudaFree(sp->d_ctr);
@@ -828,7 +939,7 @@ extern "C" int gbc_sparse_verify(gbc_sparse *sp, uint64_t start, uint64_t limit,
         if (s.tiles > sp->tiles_max) return sp_fail(sp, GBC_E_STATE, "segment larger than the map");
         if (int rc = build_map(sp, s)) return rc;
         k_sp_check<<<sp->check_ctas, kCheckThreads, 2 * kK * sp->rw * 4, sp->st>>>(s, sp->d_groups, sp->d_goff,
-                                                                                 sp->d_pend);
+                                                                                 sp->d_masks, sp->d_cls, sp->d_pend);
         SPCK(cudaGetLastError());
         SPCK(cudaEventRecord(sp->ev[3], sp->st));
         SpCtr ctr{};
