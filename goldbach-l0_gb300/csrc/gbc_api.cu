@@ -578,7 +578,7 @@ extern "C" int gbc_create(const gbc_config *cfg_in, gbc_ctx **out)
     ctx->layout = DescLayout(cfg.max_runs, cfg.max_batch);
 
     *out = ctx;
-    if (!gbh::tile_attributes(ctx->tile_bits, cfg.tile_log2, ctx->gi, cfg.device, &ctx->tile_stage))
+    if (!gbh::tile_attributes(ctx->tile_bits, ctx->gi, cfg.device, &ctx->tile_stage))
         return fail(ctx, GBC_E_ARG, "tile_bits: the tile does not fit the device's shared memory");
     gbh::query_check_grids(ctx->grids);
     gbh::query_verify_grids(ctx->grids);
@@ -782,7 +782,6 @@ static void plan_run(const gbc_ctx *ctx, gbk::BatchParams &bp, uint64_t s0, uint
     bp.tiles_pc = tiles_of(uint64_t(bp.wpc) * 32, ctx->tile_bits);
     bp.tb_vt0 = 0;
     bp.tb_tiles = bp.tiles_pc;
-    bp.tile_log2 = ctx->cfg.tile_log2;
     bp.tile_bits = ctx->tile_bits;
     bp.tile_rcp = uint32_t(((uint64_t(1) << 32) + ctx->tile_bits - 1) / ctx->tile_bits);
     bp.primes = ctx->d_primes;
@@ -1062,7 +1061,6 @@ static int ensure_mtab(gbc_ctx *ctx, uint64_t need0, uint64_t need1)
         bb.wpc = uint32_t(wpc);
         bb.tiles_pc = uint32_t(wpc * 32 / tb);
         bb.tb_tiles = bb.tiles_pc;
-        bb.tile_log2 = ctx->cfg.tile_log2;
         bb.tile_bits = tb;
         bb.tile_rcp = uint32_t(((uint64_t(1) << 32) + tb - 1) / tb);
         bb.map = tmp;

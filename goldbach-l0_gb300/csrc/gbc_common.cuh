@@ -82,8 +82,7 @@ struct BatchParams {
     uint32_t i_warp;          // primes [i0, i_warp): warp-cooperative marking
     uint32_t n_mid;           // primes [i_warp, n_mid): one thread per prime
     uint32_t n_all;           // primes [n_mid, n_all): large-prime kernel
-    uint32_t tile_log2;       // the single-run forms' tiles: 2^tile_log2 bits
-    uint32_t tile_bits;       // the batch kernels' tiles: bits per tile, a multiple of 128
+    uint32_t tile_bits;       // bits per tile, a multiple of 128
     uint32_t tile_rcp;        // ceil(2^32 / tile_bits): t / tile_bits by one multiply and a correction
     uint32_t tiles_pc;        // tiles per class array
     const uint32_t *pat;      // pattern words of the groups, back to back
@@ -486,7 +485,7 @@ void launch_map_compare(const gbk::BatchDesc &a, const gbk::BatchDesc &b, uint32
 // the persistent tile kernel's shared memory for tile_bits-bit tiles; sets
 // *stage to the tile-bin offsets it can stage (0 when the tile leaves no room)
 // and returns false when the tile itself does not fit
-bool tile_attributes(uint32_t tile_bits, uint32_t tile_log2, const gbk::GroupInfo &gi, int device, uint32_t *stage);
+bool tile_attributes(uint32_t tile_bits, const gbk::GroupInfo &gi, int device, uint32_t *stage);
 void query_check_grids(Grids &g);
 void query_verify_grids(Grids &g);
 bool verify_word_funnel(uint32_t r, uint32_t p0, uint32_t members);
@@ -495,7 +494,8 @@ void check_split(uint64_t evens, uint64_t words, int sm, uint32_t *cw, uint32_t 
 uint32_t verify_vbx(uint64_t evens, int sm);
 // single-run forms (the allocation-free entry point and the table build)
 void launch_xfirst1(const gbk::BatchParams &bp, cudaStream_t st);
-void launch_tile1(const gbk::BatchParams &bp, const gbk::GroupInfo &gi, cudaStream_t st);
+// tiles of bp.tile_bits <= max_bits bits
+cudaError_t launch_tile1(const gbk::BatchParams &bp, uint32_t max_bits, const gbk::GroupInfo &gi, cudaStream_t st);
 void launch_wheel_bytes(const gbk::BatchParams &bp, uint32_t *out, cudaStream_t st);
 // host geometry of the count kernel: CountRanges of a segment on its run's map, and its CTAs
 uint32_t count_ranges(uint64_t base, const gbk::SegParams &sp, gbk::CountRanges &cr);

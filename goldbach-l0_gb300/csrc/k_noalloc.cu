@@ -20,9 +20,9 @@
 
 namespace {
 
-constexpr uint32_t kTileLog2 = 16;          // 64 Ki bits of a class array per CTA
+constexpr uint32_t kUnitBits = 1u << 16;    // a class array is a whole number of these
+constexpr uint32_t kMaxTileUnits = 28;      // the largest tile: 224 KB of shared memory
 constexpr uint32_t kFirstTilePrimeIdx = 18; // 71 among the odd primes 3, 5, 7, ...
-constexpr uint32_t kWarpPrimeIdx = 171;     // 1031: the first prime >= 2^16 / 64
 constexpr size_t kScratchWords = size_t(9) * GBC_NOALLOC_MAX_PRIMES;
 
 // floor(2^32 / p) per prime | 8 first class bits per prime
@@ -138,6 +138,27 @@ __global__ void k_noalloc_magic(const uint32_t *primes, uint32_t n, uint32_t *ma
         magic[i] = uint32_t((1ull << 32) / primes[i]);
 }
 
+// Units per tile for class arrays of `units` units on sms multiprocessors, a
+// CTA each: the eight class arrays' tiles in as few, as short waves as can be.
+// A tile costs its visits of every prime, whatever its size (kVisit), and its
+// marks and words (1 per unit): 2^16-bit tiles paid 545 us for 2^29 integers
+// at 1e12, 2184 tiles of one unit each; 114 us in 144 of 16.
+uint32_t tile_units(uint32_t units, uint32_t sms)
+{
+    constexpr uint32_t kVisit = 8;
+    uint32_t best = 1;
+    uint64_t cost = UINT64_MAX;
+    for (uint32_t m = 1; m <= kMaxTileUnits; ++m) {
+        const uint64_t tiles = 8ull * ((units + m - 1) / m);
+        const uint64_t c = (tiles + sms - 1) / sms * (kVisit + m);
+        if (c < cost) {
+            cost = c;
+            best = m;
+        }
+    }
+    return best;
+}
+
 // bits t >= nblk of each class array: cleared, so the map past the range is
 // zero (the tile sieve writes whole tiles)
 __global__ void k_noalloc_tail(uint32_t *map, uint32_t nblk, uint32_t wpc)
@@ -174,16 +195,13 @@ extern "C" int gbc_class_map_noalloc(uint64_t q_lo, uint64_t q_hi, const uint32_
     if (pb * pb < q_hi)
         return set_error(err, err_cap, GBC_E_ARG, "the primes end below sqrt(q_hi): the map would not be exact");
 
-    const uint32_t tb = 1u << kTileLog2, tw = tb / 32;
     gbk::BatchParams bp{};
     bp.base = q_lo / 30 * 30;
     bp.qmax = q_hi;
     const uint64_t nblk = (q_hi - bp.base) / 30 + 1;
-    const uint64_t tiles = (nblk + 64 + tb - 1) / tb;
+    const uint32_t units = uint32_t((nblk + 64 + kUnitBits - 1) / kUnitBits);
     bp.nblk = uint32_t(nblk);
-    bp.tiles_pc = uint32_t(tiles);
-    bp.tb_tiles = bp.tiles_pc;
-    bp.wpc = uint32_t(tiles * tw);
+    bp.wpc = units * (kUnitBits / 32);
     if (base_out) *base_out = bp.base;
     if (nblk_out) *nblk_out = bp.nblk;
     if (wpc_out) *wpc_out = bp.wpc;
@@ -203,17 +221,24 @@ extern "C" int gbc_class_map_noalloc(uint64_t q_lo, uint64_t q_hi, const uint32_
     bp.pat = static_cast<const uint32_t *>(pat_v);
     bp.magic = scratch;
     bp.xfirst = scratch + GBC_NOALLOC_MAX_PRIMES;
-    bp.tile_log2 = kTileLog2;
     bp.i0 = nprimes < kFirstTilePrimeIdx ? nprimes : kFirstTilePrimeIdx;
     bp.n_mid = nprimes;
     bp.n_all = nprimes;
-    bp.i_warp = nprimes < kWarpPrimeIdx ? nprimes : kWarpPrimeIdx;
+    int dev = 0, sms = 0;
+    e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return set_error(err, err_cap, GBC_E_CUDA, cudaGetErrorString(e));
+    bp.tile_bits = tile_units(units, uint32_t(sms > 0 ? sms : 1)) * kUnitBits;
+    // primes with at least 128 marks per tile: a warp per prime; above, a thread per prime
+    const uint32_t warp = odd_primes_upto(bp.tile_bits / 128);
+    bp.i_warp = nprimes < warp ? nprimes : warp;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // every scratch word a kernel reads is written earlier in this call:
     // nothing needs clearing
     k_noalloc_magic<<<64, 256, 0, st>>>(d_primes, nprimes, scratch);
     gbh::launch_xfirst1(bp, st);
-    gbh::launch_tile1(bp, kPatterns.gi, st);  // 2^16-bit tiles: under the default shared-memory limit
+    e = gbh::launch_tile1(bp, kMaxTileUnits * kUnitBits, kPatterns.gi, st);
+    if (e != cudaSuccess) return set_error(err, err_cap, GBC_E_CUDA, cudaGetErrorString(e));
     const uint32_t tail_words = 8 * (bp.wpc - (bp.nblk >> 5));
     k_noalloc_tail<<<(tail_words + 255) / 256, 256, 0, st>>>(d_map, bp.nblk, bp.wpc);
     e = cudaGetLastError();

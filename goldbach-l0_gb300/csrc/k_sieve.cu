@@ -278,31 +278,23 @@ __device__ __forceinline__ void tile_body(const BatchParams &bp, const GroupInfo
             }
         }
     } else {
-        // the rest: a thread per prime, the next prime's three loads issued
-        // before the current prime's marks
-        const uint32_t *pr = bp.primes, *mg = bp.magic;
+        // the rest: four primes per thread and round, their loads all issued
+        // before any of their marks
         const uint32_t n = bp.n_mid;
-        uint32_t i = bp.i_warp + tid;
-        uint32_t p = 0, x = kNone, m = 0;
-        if (i < n) {
-            p = __ldg(pr + i);
-            x = __ldg(xk + i);
-            m = __ldg(mg + i);
-        }
-        while (i < n) {
-            const uint32_t j = i + bs;
-            uint32_t pn = 0, xn = kNone, mn = 0;
-            if (j < n) {
-                pn = __ldg(pr + j);
-                xn = __ldg(xk + j);
-                mn = __ldg(mg + j);
+        for (uint32_t i = bp.i_warp + tid; i < n; i += 4 * bs) {
+            uint32_t pv[4], xv[4], mv[4];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) {
+                const uint32_t j = min(i + u * bs, n - 1);
+                pv[u] = __ldg(bp.primes + j);
+                xv[u] = i + u * bs < n ? __ldg(xk + j) : kNone;
+                mv[u] = __ldg(bp.magic + j);
             }
-            const uint32_t l = local_start(x, t0, p, m, tl);
-            if (l < tl) clear_stride(s, l, p, tl);
-            i = j;
-            p = pn;
-            x = xn;
-            m = mn;
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) {
+                const uint32_t l = local_start(xv[u], t0, pv[u], mv[u], tl);
+                if (l < tl) clear_stride(s, l, pv[u], tl);
+            }
         }
     }
     // a binned batch: the hit-list marks of this tile (offsets within it,
@@ -432,15 +424,15 @@ template __global__ void k_tile<kTbStages[0]>(BatchDesc, GroupInfo, uint32_t);
 template __global__ void k_tile<kTbStages[1]>(BatchDesc, GroupInfo, uint32_t);
 template __global__ void k_tile<kTbStages[2]>(BatchDesc, GroupInfo, uint32_t);
 
-// one run by value: grid (tiles_pc, 8), full tiles (wpc = tiles_pc tiles)
+// one run by value: grid (ceil(32 wpc / tile_bits), 8), the last tile of a class array cut short
 __global__ void __launch_bounds__(1024, 1) k_tile1(BatchParams bp, GroupInfo gi)
 {
     extern __shared__ uint32_t sm[];
-    const uint32_t tb = 1u << bp.tile_log2;
+    const uint32_t tb = bp.tile_bits, t0 = blockIdx.x * tb;
     uint32_t *pat = sm + (tb >> 5);
     for (uint32_t i = threadIdx.x; i < gi.words; i += blockDim.x) pat[i] = bp.pat[i];
     __syncthreads();
-    tile_body<false>(bp, gi, pat, sm, blockIdx.y, blockIdx.x, blockIdx.x << bp.tile_log2, tb, tb);
+    tile_body<false>(bp, gi, pat, sm, blockIdx.y, blockIdx.x, t0, min(tb, bp.wpc * 32 - t0), tb);
 }
 
 // The packed large-prime tier (the reference's pack_large_primes,
@@ -1063,7 +1055,7 @@ static size_t tile_smem_staged(uint32_t tile_bits, uint32_t stage, const gbk::Gr
     return tile_smem(tile_bits, gi) + size_t(stage) * 4;
 }
 
-bool tile_attributes(uint32_t tile_bits, uint32_t tile_log2, const gbk::GroupInfo &gi, int device, uint32_t *stage)
+bool tile_attributes(uint32_t tile_bits, const gbk::GroupInfo &gi, int device, uint32_t *stage)
 {
     int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
@@ -1080,8 +1072,6 @@ bool tile_attributes(uint32_t tile_bits, uint32_t tile_log2, const gbk::GroupInf
     if (c == 0) cudaFuncSetAttribute(gbk::k_tile<gbk::kTbStages[0]>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (c == 1) cudaFuncSetAttribute(gbk::k_tile<gbk::kTbStages[1]>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (c == 2) cudaFuncSetAttribute(gbk::k_tile<gbk::kTbStages[2]>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaFuncSetAttribute(gbk::k_tile1, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(tile_smem(1u << tile_log2, gi)));
     return true;
 }
 
@@ -1137,10 +1127,15 @@ void launch_xfirst1(const gbk::BatchParams &bp, cudaStream_t st)
     gbk::k_xfirst1<<<blocks, 256, 0, st>>>(bp);
 }
 
-void launch_tile1(const gbk::BatchParams &bp, const gbk::GroupInfo &gi, cudaStream_t st)
+cudaError_t launch_tile1(const gbk::BatchParams &bp, uint32_t max_bits, const gbk::GroupInfo &gi, cudaStream_t st)
 {
-    dim3 grid(bp.tiles_pc, 8);
-    gbk::k_tile1<<<grid, 1024, tile_smem(1u << bp.tile_log2, gi), st>>>(bp, gi);
+    // the attribute of the largest tile, whatever this call's: the same for every caller
+    const cudaError_t e = cudaFuncSetAttribute(gbk::k_tile1, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               int(tile_smem(max_bits, gi)));
+    if (e != cudaSuccess) return e;
+    dim3 grid((bp.wpc * 32 + bp.tile_bits - 1) / bp.tile_bits, 8);
+    gbk::k_tile1<<<grid, 1024, tile_smem(bp.tile_bits, gi), st>>>(bp, gi);
+    return cudaSuccess;
 }
 
 void launch_wheel_bytes(const gbk::BatchParams &bp, uint32_t *out, cudaStream_t st)
