@@ -825,10 +825,12 @@ static void finish_desc(const gbc_ctx *ctx, DescImage &img)
     img.tile_pref[nrun] = h.tile_items;
     if (!nrun) h.n_mid_min = h.n_hl_min = 0;
     h.chk_vb = h.ver_vb = h.cnt_vb = h.nlow = 0;
-    uint64_t sampled_words = 0;  // class words of the exact checker's segments
+    uint64_t words = 0, sampled_words = 0;  // class words of the segments, and of the exact checker's
     for (uint32_t i = 0; i < nseg; ++i) {
         const gbk::SegParams &sp = img.segs[i];
-        if (sp.sampled && !sp.low) sampled_words += (sp.seg_end - sp.seg_start) / 960 + 2;
+        const uint64_t w = (sp.seg_end - sp.seg_start) / 960 + 2;
+        words += w;
+        if (sp.sampled && !sp.low) sampled_words += w;
     }
     for (uint32_t i = 0; i < nseg; ++i) {
         gbk::SegParams &sp = img.segs[i];
@@ -841,7 +843,7 @@ static void finish_desc(const gbc_ctx *ctx, DescImage &img)
         if (sp.low) ++h.nlow;
         else if (sp.sampled) h.chk_vb += sp.vbx;
         else h.ver_vb += sp.vbx;
-        h.cnt_vb += gbh::count_ranges(img.runs[sp.run].base, sp, sp.cr);
+        h.cnt_vb += gbh::count_ranges(img.runs[sp.run].base, sp, words, ctx->grids.sm);
     }
     img.chk_pref[nseg] = h.chk_vb;
     img.ver_pref[nseg] = h.ver_vb;

@@ -173,6 +173,7 @@ struct SegParams {
     uint32_t run;                 // the segment's run (class map) in the batch
     uint32_t vbx;                 // checker CTAs of the segment
     uint32_t cw;                  // words per chunk of the exact checker
+    uint32_t cnt_words, cnt_rounds;  // words per round and rounds per item of the count kernel
     CountRanges cr;
 };
 
@@ -497,6 +498,7 @@ void launch_xfirst1(const gbk::BatchParams &bp, cudaStream_t st);
 // tiles of bp.tile_bits <= max_bits bits
 cudaError_t launch_tile1(const gbk::BatchParams &bp, uint32_t max_bits, const gbk::GroupInfo &gi, cudaStream_t st);
 void launch_wheel_bytes(const gbk::BatchParams &bp, uint32_t *out, cudaStream_t st);
-// host geometry of the count kernel: CountRanges of a segment on its run's map, and its CTAs
-uint32_t count_ranges(uint64_t base, const gbk::SegParams &sp, gbk::CountRanges &cr);
+// host geometry of the count kernel: CountRanges of a segment on its run's
+// map, and its CTAs in a batch of `words` class words
+uint32_t count_ranges(uint64_t base, gbk::SegParams &sp, uint64_t words, int sm);
 }  // namespace gbh
