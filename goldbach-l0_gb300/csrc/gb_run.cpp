@@ -15,6 +15,7 @@
 #include "gb_run.hpp"
 
 #include <algorithm>
+#include <charconv>
 #include <chrono>
 #include <cinttypes>
 #include <cstdio>
@@ -53,26 +54,35 @@ std::string u128_str(u128 v)
     return s;
 }
 
-std::vector<uint16_t> candidates()
+// the candidates, sieved once per process
+const std::vector<uint16_t> &candidates()
 {
-    std::vector<uint16_t> c(GBC_NCAND);
-    gbc_candidates(c.data(), GBC_NCAND);
+    static const std::vector<uint16_t> c = [] {
+        std::vector<uint16_t> v(GBC_NCAND);
+        gbc_candidates(v.data(), GBC_NCAND);
+        return v;
+    }();
     return c;
 }
 
+// v in decimal at the end of s
+void put(std::string &s, uint64_t v)
+{
+    char b[20];
+    s.append(b, std::to_chars(b, b + sizeof b, v).ptr);
+}
+
 // comma-separated counts, an empty entry for 0, trailing zeros cut
-// (GoldbachStats::dense_list, include/gstats.hpp:890-903)
-std::string dense_list(const std::vector<uint64_t> &v, size_t from = 0)
+// (GoldbachStats::dense_list, include/gstats.hpp:890-903), at the end of s
+void put_dense(std::string &s, const std::vector<uint64_t> &v, size_t from = 0)
 {
     size_t last = 0;
     for (size_t i = from; i < v.size(); ++i)
         if (v[i]) last = i + 1;
-    std::string s;
     for (size_t i = from; i < last; ++i) {
         if (i > from) s += ',';
-        if (v[i]) s += std::to_string(v[i]);
+        if (v[i]) put(s, v[i]);
     }
-    return s;
 }
 
 }  // namespace
@@ -83,7 +93,6 @@ RunAccumulator::RunAccumulator(uint64_t start, uint64_t limit, uint32_t tail_t)
     cand_ = candidates();
     samp_.assign(size_t(GBC_NCLASS) * GBC_NCAND, 0);
     tail_.assign(GBC_NCAND, 0);
-    tail_cls_.assign(size_t(GBC_NCLASS) * GBC_NCAND, 0);
     tail_agg_.assign(GBC_NCAND, 0);
     first_all_.assign(GBC_NCAND, 0);
     first_tail_.assign(GBC_NCAND, 0);
@@ -154,24 +163,25 @@ void RunAccumulator::add_segment(const gbc_segment_result &r)
     // positive accounting: every even of the segment has a p(n) (or, in a
     // verified segment, was resolved by the funnels or has one in the tail)
     uint64_t found = r.nleft;
-    for (int cr = 0; cr < GBC_NCLASS; ++cr)
-        for (int i = 0; i < GBC_NCAND; ++i) found += r.hist[cr][i];
+    for (int cr = 0; cr < GBC_NCLASS; ++cr) {
+        uint64_t sum = 0;
+        for (int i = 0; i < GBC_NCAND; ++i) sum += r.hist[cr][i];
+        found += sum;
+    }
     const uint64_t want = r.sampled ? r.evens : r.pending;
     if (found != want || r.pending > r.evens)
         throw std::runtime_error("coverage: segment [" + std::to_string(r.seg_start) + ", " +
                                  std::to_string(r.seg_end) + "] accounts for " + std::to_string(found) + " of " +
                                  std::to_string(want) + (r.sampled ? " evens" : " pending evens"));
+    if (r.sampled)
+        for (int cr = 0; cr < GBC_NCLASS; ++cr)
+            for (int i = 0; i < GBC_NCAND; ++i) samp_[size_t(cr) * GBC_NCAND + i] += r.hist[cr][i];
+    const int t0 = int(std::lower_bound(cand_.begin(), cand_.end(), tail_t_) - cand_.begin());
     for (int cr = 0; cr < GBC_NCLASS; ++cr)
-        for (int i = 0; i < GBC_NCAND; ++i) {
-            const uint64_t c = r.hist[cr][i];
-            if (!c) continue;
-            if (r.sampled) samp_[size_t(cr) * GBC_NCAND + i] += c;
-            if (cand_[i] >= tail_t_) {
-                tail_[i] += c;
-                if (r.sampled) tail_cls_[size_t(cr) * GBC_NCAND + i] += c;
-                else tail_agg_[i] += c;
-            }
-        }
+        for (int i = t0; i < GBC_NCAND; ++i) tail_[i] += r.hist[cr][i];
+    if (!r.sampled)
+        for (int cr = 0; cr < GBC_NCLASS; ++cr)
+            for (int i = t0; i < GBC_NCAND; ++i) tail_agg_[i] += r.hist[cr][i];
     for (int i = 0; i < GBC_NCAND; ++i)
         if (r.first[i] != 0xFFFFFFFFu) {
             const uint64_t n = r.seg_start + 2ull * r.first[i];
@@ -291,30 +301,37 @@ std::string RunAccumulator::stats_ref_line() const
     }
     std::snprintf(b, sizeof b, " twins30=%" PRIu64 ",%" PRIu64 ",%" PRIu64, twins30_[11], twins30_[17], twins30_[29]);
     o += b;
-    // first occurrences of every p(n) value, ascending p
-    std::map<uint64_t, uint64_t> firsts;
+    // first occurrences of every p(n) value, ascending p (beyond_ ascends
+    // too; its p = 2 comes before the candidates, the others after them)
     std::vector<uint64_t> tot(GBC_NCAND, 0);
-    for (int i = 0; i < GBC_NCAND; ++i) {
-        for (int cr = 0; cr < GBC_NCLASS; ++cr) tot[i] += samp_[size_t(cr) * GBC_NCAND + i];
-        if (tot[i]) firsts[cand_[i]] = first_all_[i];
-    }
-    for (auto &bp : beyond_) {
-        auto it = firsts.find(bp.first);
-        if (it == firsts.end() || bp.second.second < it->second) firsts[bp.first] = bp.second.second;
-    }
+    for (int cr = 0; cr < GBC_NCLASS; ++cr)
+        for (int i = 0; i < GBC_NCAND; ++i) tot[i] += samp_[size_t(cr) * GBC_NCAND + i];
     o += " first=";
     bool f1 = true;
-    for (auto &f : firsts) {
-        std::snprintf(b, sizeof b, "%s%" PRIu64 ":%" PRIu64, f1 ? "" : ";", f.first, f.second);
-        o += b;
+    auto put_first = [&](uint64_t p, uint64_t n) {
+        if (!f1) o += ';';
+        put(o, p);
+        o += ':';
+        put(o, n);
         f1 = false;
+    };
+    auto bp = beyond_.begin();
+    for (int i = 0; i < GBC_NCAND; ++i) {
+        for (; bp != beyond_.end() && bp->first < cand_[i]; ++bp) put_first(bp->first, bp->second.second);
+        const bool also = bp != beyond_.end() && bp->first == cand_[i];
+        if (tot[i]) put_first(cand_[i], also ? std::min(first_all_[i], bp->second.second) : first_all_[i]);
+        else if (also) put_first(cand_[i], bp->second.second);
+        if (also) ++bp;
     }
+    for (; bp != beyond_.end(); ++bp) put_first(bp->first, bp->second.second);
     std::vector<uint64_t> hist(tot);
-    for (size_t i = 0; i < hist.size(); ++i) {
-        auto it = beyond_.find(cand_[i]);
-        if (it != beyond_.end()) hist[i] += it->second.first;
-    }
-    o += " hist=" + dense_list(hist);
+    if (!beyond_.empty())
+        for (size_t i = 0; i < hist.size(); ++i) {
+            auto it = beyond_.find(cand_[i]);
+            if (it != beyond_.end()) hist[i] += it->second.first;
+        }
+    o += " hist=";
+    put_dense(o, hist);
     // gaps: count, moments, largest, tail, histogram
     u128 m[4] = {odd_gaps_, odd_gaps_, odd_gaps_, odd_gaps_};  // g = 1
     uint64_t n = odd_gaps_;
@@ -338,7 +355,8 @@ std::string RunAccumulator::stats_ref_line() const
         o += b;
         t1 = false;
     }
-    o += " ghist=" + dense_list(ghist_);
+    o += " ghist=";
+    put_dense(o, ghist_);
     return o;
 }
 
@@ -360,7 +378,11 @@ RunRecord RunAccumulator::record(bool gaps_on) const
     r.evens_sampled = evens_sampled_;
     r.tail_t = tail_t_;
     r.samp = samp_;
-    r.tail_cls = tail_cls_;
+    // the sampled segments' tail by class: their histogram from the tail bound on
+    r.tail_cls = samp_;
+    const size_t t0 = size_t(std::lower_bound(cand_.begin(), cand_.end(), tail_t_) - cand_.begin());
+    for (size_t cr = 0; cr < GBC_NCLASS; ++cr)
+        std::fill_n(r.tail_cls.begin() + std::ptrdiff_t(cr * GBC_NCAND), t0, uint64_t(0));
     r.tail_agg = tail_agg_;
     r.first = first_tail_;
     r.beyond = beyond_list_;
@@ -426,7 +448,7 @@ void check(gbc_ctx *ctx, int rc, const char *what)
 }  // namespace
 
 RangeStats run_range(gbc_ctx *ctx, uint64_t start, uint64_t limit, uint64_t segment_even, uint32_t max_batch,
-                     uint16_t *pn, RunAccumulator *acc_out, uint32_t sample_every, bool per_segment)
+                     uint16_t *pn, RunAccumulator *acc_out, uint32_t sample_every, bool per_segment, bool both_lines)
 {
     RangeStats st;
     const auto t0 = std::chrono::steady_clock::now();
@@ -447,26 +469,25 @@ RangeStats run_range(gbc_ctx *ctx, uint64_t start, uint64_t limit, uint64_t segm
             f.push_back(pn ? 0u : segment_flag(sample_every, j));
         flags.push_back(f);
     }
-    std::vector<gbc_segment_result> out[2];
     double gpu_ms = 0;
     Outputs *outs = outputs_of(ctx);
-    const std::vector<uint16_t> cand = outs ? candidates() : std::vector<uint16_t>();
+    const std::vector<uint16_t> &cand = candidates();
     const uint64_t evens_total = (limit - start) / 2 + 1;
     auto t_last = std::chrono::steady_clock::now();
     auto collect = [&](size_t b) {
         const int slot = int(b & 1);
         const int n = int(batches[b].size());
-        out[slot].resize(n);
+        const gbc_segment_result *out = nullptr;  // the slot's own results, until its next batch
         gbc_batch_times tm{};
-        check(ctx, gbc_collect(ctx, slot, out[slot].data(), n, &tm, 600000), "collect");
+        check(ctx, gbh_collect(ctx, slot, &out, n, &tm, 600000), "collect");
         if (per_segment) {
             const auto now = std::chrono::steady_clock::now();
             const double wall = std::chrono::duration<double, std::milli>(now - t_last).count();
             t_last = now;
             uint64_t be = 0;
-            for (int i = 0; i < n; ++i) be += out[slot][i].evens;
+            for (int i = 0; i < n; ++i) be += out[i].evens;
             for (int i = 0; i < n; ++i) {
-                const auto &r = out[slot][i];
+                const auto &r = out[i];
                 const double f = double(r.evens) / double(be);
                 st.per_segment.push_back({r.seg_start, r.seg_end, r.evens, r.nleft, tm.ms_tile * f, tm.ms_large * f,
                                           (tm.ms_check + tm.ms_count) * f, wall * f});
@@ -478,10 +499,10 @@ RangeStats run_range(gbc_ctx *ctx, uint64_t start, uint64_t limit, uint64_t segm
         st.check_ms += tm.ms_check;
         st.count_ms += tm.ms_count;
         for (int i = 0; i < n; ++i) {
-            acc.add_segment(out[slot][i]);
-            if (outs) outs->add_segment(out[slot][i], cand);
+            acc.add_segment(out[i]);
+            if (outs) outs->add_segment(out[i], cand);
             if (pn) {
-                const auto &r = out[slot][i];
+                const auto &r = out[i];
                 check(ctx, gbc_copy_pn(ctx, slot, i, pn + (r.seg_start - start) / 2, r.evens), "copy p(n)");
             }
         }
@@ -514,7 +535,7 @@ RangeStats run_range(gbc_ctx *ctx, uint64_t start, uint64_t limit, uint64_t segm
     st.gpu_seconds = gpu_ms / 1e3;
     st.wall_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     st.stats_line = acc.stats_ref_line();
-    st.gbstats_line = acc.gbstats_line(kVersion);
+    if (both_lines || st.stats_line.empty()) st.gbstats_line = acc.gbstats_line(kVersion);
     st.ridges = acc.ridges();
     // the passed run into the campaign state, once (GoldbachStats::commit)
     if (StatsCampaign *camp = campaign_of(ctx); camp && start >= kStatsMinStart) {
@@ -577,7 +598,7 @@ extern "C" int gbc_verify_range(gbc_ctx *ctx, uint64_t start, uint64_t limit, gb
         gbc_config cfg{};
         if (gbc_get_config(ctx, &cfg) != GBC_OK) return GBC_E_ARG;
         gb::RangeStats st =
-            gb::run_range(ctx, start, limit, cfg.segment_even, cfg.max_batch, pn, nullptr, cfg.sample_every);
+            gb::run_range(ctx, start, limit, cfg.segment_even, cfg.max_batch, pn, nullptr, cfg.sample_every, false, false);
         if (res) {
             res->start = st.start;
             res->limit = st.limit;

@@ -18,6 +18,11 @@
 #include "../../include/gbc.h"
 #include "gb_stats.hpp"
 
+// gbc_collect without its copy (gbc_api.cu): *out points at the slot's own
+// results in host memory, valid until the slot's next batch is enqueued.
+int gbh_collect(gbc_ctx *ctx, int slot, const gbc_segment_result **out, int nseg, gbc_batch_times *times,
+                int timeout_ms);
+
 namespace gb {
 
 struct GbcError : std::runtime_error {
@@ -52,7 +57,8 @@ struct RangeStats {
     double gpu_seconds = 0, wall_seconds = 0;
     double tile_ms = 0, large_ms = 0, check_ms = 0, count_ms = 0;
     std::string stats_line;       // tests/stats_ref.cpp's line (every segment sampled), else empty
-    std::string gbstats_line;     // the GBSTATS v2 log line of the run (include/gstats.hpp:913-969)
+    std::string gbstats_line;     // the GBSTATS v2 log line of the run (include/gstats.hpp:913-969); without
+                                  // both_lines only where stats_line is empty
     std::vector<Ridge> ridges;    // the run's top 30 ridges
     bool stats_committed = false; // merged into the context's campaign state (gbc_set_stats)
     std::vector<SegRecord> per_segment;  // filled when run_range is asked for it
@@ -97,7 +103,6 @@ private:
     std::vector<uint16_t> cand_;
     std::vector<uint64_t> samp_;                                  // [15][NCAND], sampled segments
     std::vector<uint64_t> tail_;                                  // [NCAND], p >= tail_t, every segment
-    std::vector<uint64_t> tail_cls_;                              // [15][NCAND], p >= tail_t, sampled segments
     std::vector<uint64_t> tail_agg_;                              // [NCAND], p >= tail_t, other segments
     std::vector<std::pair<uint64_t, uint64_t>> beyond_list_;      // (n, p) beyond 9781, in run order
     std::vector<uint64_t> first_all_;                             // first n per candidate, sampled segments
@@ -201,7 +206,8 @@ inline uint32_t segment_flag(uint32_t sample_every, size_t j)
 // nullptr. sample_every: every sample_every-th segment (segment 0 always)
 // gets p(n) of every even, the others the funnel verify + exact tail.
 RangeStats run_range(gbc_ctx *ctx, uint64_t start, uint64_t limit, uint64_t segment_even, uint32_t max_batch,
-                     uint16_t *pn, RunAccumulator *acc_out, uint32_t sample_every = 1, bool per_segment = false);
+                     uint16_t *pn, RunAccumulator *acc_out, uint32_t sample_every = 1, bool per_segment = false,
+                     bool both_lines = true);
 
 // The reference's --csv key=value line of a run (src/main.cpp:191-215).
 std::string csv_line(const RangeStats &st, uint64_t segment);

@@ -49,7 +49,7 @@ RangeStats Window::stats() const
     st.tail_evens = acc.tail_evens();
     st.pending = acc.pending();
     st.stats_line = acc.stats_ref_line();
-    st.gbstats_line = acc.gbstats_line("gb300-1.0");
+    if (st.stats_line.empty()) st.gbstats_line = acc.gbstats_line("gb300-1.0");
     st.ridges = acc.ridges();
     st.wall_seconds = std::chrono::duration<double>(t_done - t_submit).count();
     return st;
@@ -59,7 +59,6 @@ Scheduler::Scheduler(gbc_ctx *ctx) : ctx_(ctx)
 {
     check(ctx, gbc_get_config(ctx, &cfg_), "config");
     for (int s = int(cfg_.nslots) - 1; s >= 0; --s) free_slots_.push_back(s);
-    out_.resize(cfg_.max_batch);
 }
 
 void Scheduler::add(std::shared_ptr<Window> w)
@@ -114,13 +113,14 @@ std::vector<std::shared_ptr<Window>> Scheduler::finish(InFlight &f)
 {
     const int n = int(f.items.size());
     gbc_batch_times tm{};
-    check(ctx_, gbc_collect(ctx_, f.slot, out_.data(), n, &tm, 600000), "collect");
+    const gbc_segment_result *out = nullptr;  // the slot's own results, until its next batch
+    check(ctx_, gbh_collect(ctx_, f.slot, &out, n, &tm, 600000), "collect");
     st_.gpu_ms += tm.ms_total;
     free_slots_.push_back(f.slot);
     std::vector<std::shared_ptr<Window>> done;
     for (int i = 0; i < n; ++i) {
         auto &w = f.items[i].w;
-        w->acc.add_segment(out_[i]);
+        w->acc.add_segment(out[i]);
         if (++w->done == w->segs.size()) {
             w->t_done = Clock::now();
             st_.windows += 1;
@@ -270,6 +270,7 @@ void serve(gbc_server *srv)
 {
     gb::Scheduler sch(srv->ctx);
     std::vector<std::shared_ptr<gb::Window>> fresh;
+    gb::Clock::time_point last = gb::Clock::now();  // something arrived or finished
     try {
         for (;;) {
             {
@@ -283,6 +284,7 @@ void serve(gbc_server *srv)
                     srv->inbox.pop_front();
                 }
             }
+            if (!fresh.empty()) last = gb::Clock::now();
             for (auto &w : fresh) sch.add(std::move(w));
             fresh.clear();
             sch.launch_ready();
@@ -295,8 +297,11 @@ void serve(gbc_server *srv)
                 }
                 srv->stats = sch.stats();
                 srv->cv_done.notify_all();
+                last = gb::Clock::now();
             } else if (!sch.idle()) {
-                std::this_thread::sleep_for(std::chrono::microseconds(20));
+                // a sleep takes about 70 us: short batches are watched instead
+                if (gb::Clock::now() - last < std::chrono::milliseconds(1)) std::this_thread::yield();
+                else std::this_thread::sleep_for(std::chrono::microseconds(20));
             }
         }
     } catch (const gb::GbcError &e) {

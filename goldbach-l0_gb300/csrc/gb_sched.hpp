@@ -77,7 +77,6 @@ private:
     std::deque<std::shared_ptr<Window>> queue_;  // windows with unscheduled segments
     std::deque<InFlight> inflight_;
     std::vector<int> free_slots_;
-    std::vector<gbc_segment_result> out_;
     SchedStats st_;
 };
 

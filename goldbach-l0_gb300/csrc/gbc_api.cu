@@ -289,6 +289,8 @@ static int slot_alloc(gbc_ctx *ctx, Slot &s)
     CK(dev_alloc(ctx, &s.xfirst, s.xfirst_words * 4));
     CK(dev_alloc(ctx, &s.res, size_t(cfg.max_batch) * sizeof(gbc_segment_result)));
     CK(dev_alloc(ctx, &s.err, 4));
+    CK(cudaMallocHost(&s.res_host, size_t(cfg.max_batch) * sizeof(gbc_segment_result)));
+    CK(cudaMallocHost(&s.err_host, 4));
     if (cfg.want_pn) {
         s.pn_stride = cfg.segment_even / 2 + 1;
         CK(dev_alloc(ctx, &s.pn, size_t(cfg.max_batch) * s.pn_stride * 2));
@@ -349,6 +351,8 @@ static void slot_free(Slot &s)
     cudaFree(s.tb_cnt);
     cudaFree(s.ovf_buf);
     cudaFree(s.ovf_cnt);
+    if (s.res_host) cudaFreeHost(s.res_host);
+    if (s.err_host) cudaFreeHost(s.err_host);
     if (s.desc_host) cudaFreeHost(s.desc_host);
     if (s.win_host) cudaFreeHost(s.win_host);
     cudaFree(s.chk_map);
@@ -1311,6 +1315,9 @@ static int enqueue_planned(gbc_ctx *ctx, Slot &s)
         }
     }
     CK(cudaEventRecord(s.ev[5], st));
+    CK(cudaMemcpyAsync(s.res_host, s.res, img.h->nseg * sizeof(gbc_segment_result), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(s.err_host, s.err, 4, cudaMemcpyDeviceToHost, st));
+    CK(cudaEventRecord(s.ev[6], st));
     CK(cudaGetLastError());
     s.nseg = int(img.h->nseg);
     s.nrun = int(img.h->nrun);
@@ -1346,32 +1353,37 @@ extern "C" int gbc_poll(gbc_ctx *ctx, int slot)
     if (bad_slot(ctx, slot)) return fail(ctx, GBC_E_ARG, "bad context or slot");
     Slot &s = ctx->slot[slot];
     if (!s.pending) return 0;
-    const cudaError_t q = cudaEventQuery(s.ev[5]);
+    const cudaError_t q = cudaEventQuery(s.ev[6]);
     if (q == cudaSuccess) return 1;
     if (q == cudaErrorNotReady) return 0;
     return fail(ctx, GBC_E_CUDA, std::string("batch: ") + cudaGetErrorString(q));
 }
 
-extern "C" int gbc_collect(gbc_ctx *ctx, int slot, gbc_segment_result *out, int nseg, gbc_batch_times *times,
-                           int timeout_ms)
+// gbc_collect without its copy (gb_run.hpp): the slot's own results, copied to
+// host memory behind the batch
+int gbh_collect(gbc_ctx *ctx, int slot, const gbc_segment_result **res, int nseg, gbc_batch_times *times,
+                int timeout_ms)
 {
-    if (bad_slot(ctx, slot) || !out) return fail(ctx, GBC_E_ARG, "bad context, slot or output");
+    if (bad_slot(ctx, slot)) return fail(ctx, GBC_E_ARG, "bad context, slot or output");
     Slot &s = ctx->slot[slot];
     if (!s.pending) return fail(ctx, GBC_E_STATE, "collect without an enqueued batch");
     if (nseg != s.nseg) return fail(ctx, GBC_E_ARG, "nseg differs from the enqueued batch");
     const auto t0 = std::chrono::steady_clock::now();
     for (;;) {
-        const cudaError_t q = cudaEventQuery(s.ev[5]);
+        const cudaError_t q = cudaEventQuery(s.ev[6]);
         if (q == cudaSuccess) break;
         if (q != cudaErrorNotReady) return fail(ctx, GBC_E_CUDA, std::string("batch: ") + cudaGetErrorString(q));
-        if (timeout_ms >= 0 &&
-            std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(timeout_ms))
+        const auto waited = std::chrono::steady_clock::now() - t0;
+        if (timeout_ms >= 0 && waited > std::chrono::milliseconds(timeout_ms))
             return fail(ctx, GBC_E_TIMEOUT, "batch not finished within the timeout");
-        std::this_thread::sleep_for(std::chrono::microseconds(20));
+        // a sleep takes about 70 us: short batches are watched instead
+        if (waited < std::chrono::microseconds(500)) std::this_thread::yield();
+        else std::this_thread::sleep_for(std::chrono::microseconds(20));
     }
-    CK(cudaMemcpy(out, s.res, size_t(nseg) * sizeof(gbc_segment_result), cudaMemcpyDeviceToHost));
-    uint32_t berr = 0, bad_words = 0;
-    CK(cudaMemcpy(&berr, s.err, 4, cudaMemcpyDeviceToHost));
+    gbc_segment_result *const out = s.res_host;
+    *res = out;
+    const uint32_t berr = *s.err_host;
+    uint32_t bad_words = 0;
     if (s.did_selfcheck) CK(cudaMemcpy(&bad_words, s.chk_count, 4, cudaMemcpyDeviceToHost));
     if (ctx->cfg.hl_cap_pct < 100 && s.img.h->nrun && gbk::hl_binned(s.img.runs[0])) {
         uint32_t ov = 0;
@@ -1425,6 +1437,16 @@ extern "C" int gbc_collect(gbc_ctx *ctx, int slot, gbc_segment_result *out, int 
             return fail(ctx, GBC_E_OVERFLOW, "leftover, gap-tail, ridge or pending list overflow");
     }
     return GBC_OK;
+}
+
+extern "C" int gbc_collect(gbc_ctx *ctx, int slot, gbc_segment_result *out, int nseg, gbc_batch_times *times,
+                           int timeout_ms)
+{
+    if (!out) return fail(ctx, GBC_E_ARG, "bad context, slot or output");
+    const gbc_segment_result *res = nullptr;
+    const int rc = gbh_collect(ctx, slot, &res, nseg, times, timeout_ms);
+    if (res) std::memcpy(out, res, size_t(nseg) * sizeof(gbc_segment_result));
+    return rc;
 }
 
 extern "C" int gbc_copy_pn(gbc_ctx *ctx, int slot, int seg, uint16_t *out, uint64_t evens)

@@ -36,14 +36,17 @@ struct Slot {
     cudaStream_t st = nullptr;
     // 0 start, 1 hit lists harvested and sorted, 2 map done (tiles, large
     // primes, direct and overflow marks), 3 checker done, 4 counts done (end
-    // of the pipeline), 5 end of the batch (after a self-check)
-    cudaEvent_t ev[6] = {};
+    // of the pipeline), 5 end of the batch (after a self-check), 6 its results
+    // in host memory
+    cudaEvent_t ev[7] = {};
     uint32_t *map = nullptr;           // class maps of the batch's runs, back to back
     size_t map_words = 0;              // capacity (words, without the pad)
     uint32_t *xfirst = nullptr;        // first class bits of the runs, back to back
     size_t xfirst_words = 0;
     gbc_segment_result *res = nullptr; // max_batch results
     uint32_t *err = nullptr;
+    gbc_segment_result *res_host = nullptr; // the batch's results and error word, copied at its end (pinned)
+    uint32_t *err_host = nullptr;
     uint16_t *pn = nullptr;            // max_batch * pn_stride p(n), or nullptr
     uint64_t pn_stride = 0;
     uint2 *pend = nullptr;             // max_batch * pend_cap phase-A pending words
