@@ -39,6 +39,8 @@ __host__ __device__ __forceinline__ constexpr uint32_t unit30(uint32_t k)
 constexpr uint32_t kUnits30 = (1u << 1) | (1u << 7) | (1u << 11) | (1u << 13) | (1u << 17) | (1u << 19) |
                               (1u << 23) | (1u << 29);
 
+constexpr uint64_t kUnits60 = uint64_t(kUnits30) | uint64_t(kUnits30) << 30;
+
 // class array index of a residue mod 30, or 8 when it is not coprime to 30
 __host__ __device__ __forceinline__ constexpr uint32_t class_of(uint32_t u)
 {

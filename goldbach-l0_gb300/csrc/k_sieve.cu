@@ -615,10 +615,11 @@ __global__ void __launch_bounds__(256) k_large(BatchDesc d)
     }
 }
 
-// floor(2^64 / p), or up to four less, for 3 <= p < 2^32: the hit lists' reciprocal. From 2^20 on
-// without a division: a float estimate of 2^52 / p (error below 2^13 of it),
-// scaled by 2^12 and corrected by the float estimate of what it leaves; the
-// corrected value is within two of 2^64 / p, so two less never exceeds it.
+// floor(2^64 / p), or up to four less, for a prime 3 <= p < 2^32: the hit lists'
+// reciprocal. From 2^20 on without a division: a float estimate of 2^52 / p
+// (error below 2^13 of it), scaled by 2^12 and corrected by the float estimate
+// of what it leaves; the corrected value is within two of 2^64 / p, so two less
+// never exceeds it.
 __device__ __forceinline__ uint64_t recip64(uint32_t p, float rp)
 {
     if (p < (1u << 20)) return 0xFFFFFFFFFFFFFFFFull / p;
@@ -628,8 +629,21 @@ __device__ __forceinline__ uint64_t recip64(uint32_t p, float rp)
     return (uint64_t(q1) << 12) + uint64_t(int64_t(c)) - 2;
 }
 
+// floor(2^64 / p) itself, from recip64
+__device__ __forceinline__ uint64_t recip64_exact(uint32_t p, uint64_t inv)
+{
+    uint64_t e = 0 - inv * p;  // 2^64 - inv p < 5 p
+#pragma unroll
+    for (uint32_t step = 2; step; step >>= 1)
+        if (e >= uint64_t(p) * step) {
+            e -= uint64_t(p) * step;
+            inv += step;
+        }
+    return e >= p ? inv + 1 : inv;
+}
+
 // floor(x / p) and x mod p for x < 2^60 and inv = recip64(p): the high half
-// of x inv is the quotient or one less (x (2^64 / p - inv) / 2^64 < 1 / 4).
+// of x inv is the quotient or one less (x (2^64 / p - inv) / 2^64 < 1 / 2).
 // The remainder before the correction is below 2 p: 32 bits hold it for
 // p < 2^31.
 __device__ __forceinline__ uint64_t divmod_recip(uint64_t x, uint32_t p, uint64_t inv, uint32_t &rem)
@@ -659,36 +673,38 @@ __device__ __forceinline__ uint64_t divmod_recip(uint64_t x, uint32_t p, uint64_
 // + rho, places every mark: byte b holds the bits p (b - b0) + v_k - rho,
 // v_k = floor(p u_k / 30) = (p / 30) u_k + floor((p mod 30) u_k / 30), in
 // 32-bit arithmetic, and a mark belongs to the run iff its bit is below
-// nblk (no masks over the end bytes). A run narrower than p / 32 bits holds
-// at most one multiple of p: its multiplier is 30 b0 + j, j the least with
-// floor(p j / 30) >= rho, and most pairs of such a run end there, with j not
-// a unit or the bit past the run, before any table read.
+// nblk (no masks over the end bytes). A run narrower than p / 4 bits holds a
+// few multiples of p, from m = 30 b0 + j on, j the least with floor(p j / 30)
+// >= rho (at most one where it is narrower than p / 32): a pair reads the table
+// only for those that are units and inside the run, and most pairs of a narrow
+// run end without a read.
 __device__ __forceinline__ void ovf_push(const BatchParams &bp, uint32_t k, uint32_t t)
 {
     const uint32_t slot = atomicAdd(bp.ovf_cnt, 1u);
     if (slot < bp.ovf_cap) bp.ovf_buf[slot] = make_uint2(k, t);
 }
 
-// Bound by issue (68% on one 467.5M segment, 176 instructions per prime, of
-// them about 70 for a pair that ends in the narrow test) and, where p is
-// below the run's width, by the table's random sectors. Measured against a
-// pair that divided base and base + span apart, took byte bounds and masks
-// with 64-bit divisions by 30 and placed each mark with 64-bit arithmetic
-// (one GB300, harvest and sort): one segment 1.27 -> 0.75 ms, 128 segments
-// 8.13 -> 7.04 ms, 16 runs of 1e6 integers at 4e18..5e18 0.23 ms a run, 292
-// segments of uneven windows 75.1 -> 46.6 ms. Few, large CTAs: every CTA
+// Bound by issue (68% on one 467.5M segment) and, where p is below the run's
+// width, by the table's random sectors. Measured against a pair that divided
+// base and base + span apart, took byte bounds and masks with 64-bit divisions
+// by 30 and placed each mark with 64-bit arithmetic (one GB300, harvest and
+// sort): one segment 1.27 -> 0.70 ms, 8 segments 1.63 -> 1.24, 128 segments
+// 8.13 -> 7.0, 292 segments of uneven windows 75.1 -> 42.1. Of that the units
+// tested before the table is read (runs narrower than p / 4): one segment 0.75
+// -> 0.70, 8 segments 1.40 -> 1.24, the windows 46.6 -> 42.5. Few, large CTAs: every CTA
 // writes one stream per region bin, and the streams share the L2: 2 x 768
 // threads 7.04 ms per 128 segments, 3 x 512 7.37, 4 x 384 8.17, 5 x 256
 // 8.38, 1 x 1024 7.76.
 constexpr int kHlThreads = 768, kHlCtas = 2;
 
-// What the harvest reads of a run, two 16-byte shared-memory loads.
+// What the harvest reads of a run: of most pairs the first 16 bytes.
 struct __align__(16) HlRun {
+    uint64_t below;      // base - 1
+    uint32_t span;       // 30 nblk - 1, or 2^32 - 1 where that is more
+    uint32_t n_all;      // 0: no hit-listed prime
     uint64_t B;          // base / 30
-    uint32_t nblk, n_hl;
-    uint32_t n_all;
+    uint32_t nblk;
     uint32_t vbase;      // the run's first virtual bit (binned)
-    uint32_t pad[2];
 };
 
 // direct = 0: a binned batch's harvest (launched before the tiles); direct =
@@ -700,7 +716,7 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
     const bool binned = hl_binned(d.runs[0]);
     if (binned == (direct != 0)) return;
     const BatchParams &run0 = d.runs[0];
-    const uint32_t i_lo = d.h->n_hl_min, nhi = d.h->n_all_max;
+    const uint32_t nhi = d.h->n_all_max;
     const uint32_t quota = binned ? run0.hl_quota : 0u;
     const uint32_t rlog = run0.hl_rlog, nreg = run0.hl_nreg, nbin = 8 * nreg;
     // per (class of p, class of m): u_m | floor((p mod 30) u_m / 30) << 8 |
@@ -710,6 +726,9 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
     __shared__ uint8_t s_res[32];
     __shared__ uint32_t s_hcnt[kHlMaxBins];
     __shared__ HlRun s_run[256];
+    __shared__ uint32_t s_lo;
+    if (threadIdx.x == 0) s_lo = kNone;
+    __syncthreads();
     if (threadIdx.x < 64) {
         const uint32_t a = threadIdx.x >> 3, b = threadIdx.x & 7;
         const uint32_t x = unit30(a) * unit30(b), kq = class_of(x % 30);
@@ -721,14 +740,17 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
     for (uint32_t r = threadIdx.x; r < nrun; r += blockDim.x) {
         const BatchParams &bp = d.runs[r];
         HlRun x{};
+        x.below = bp.base - 1;  // (base 0: a run of a few small q, wide against every p)
+        x.span = uint32_t(min(30ull * bp.nblk - 1, 0xFFFFFFFFull));
+        x.n_all = bp.n_hl < bp.n_all ? bp.n_all : 0u;
         x.B = bp.base / 30;
         x.nblk = bp.nblk;
-        x.n_hl = bp.n_hl;
-        x.n_all = bp.n_all;
+        if (x.n_all) atomicMin(&s_lo, bp.n_hl);  // the same for every run that has some
         x.vbase = bp.tb_vt0 * run0.tile_bits;
         s_run[r] = x;
     }
     __syncthreads();
+    const uint32_t i_lo = min(s_lo, nhi);
     // a binned batch files its marks in region bins (k_binsort takes them on)
     uint32_t *const hl_mine = quota ? run0.hl_buf + size_t(blockIdx.x) * nbin * quota : nullptr;
     const uint32_t rmask = (1u << rlog) - 1u;
@@ -754,17 +776,39 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
         const uint32_t *const cls = s_cls[s_res[pr]];
         uint32_t rho;
         const uint64_t b = divmod_recip(run.B, p, inv, rho) - tb0;  // byte b0 in the table
+        // m = 30 b0 + j from j = ceil(30 rho / p) on, the estimate lowered by
+        // 0.01, far above its error
         if (run.nblk <= (p >> 5)) {
-            // at most one multiple: m = 30 b0 + j, j = ceil(30 rho / p).
-            // The estimate is lowered by 0.01, far above its error: when
-            // that gives j - 1, the first multiple is at least 0.99 p / 30
-            // > nblk bits up, and j - 1 itself is below the run.
+            // at most one multiple: when the estimate gives j - 1, the first
+            // multiple is at least 0.99 p / 30 > nblk bits up, and j - 1
+            // itself is below the run
             const uint32_t j = __float2uint_ru(fmaxf(__uint2float_rn(rho) * (30.0f * rp) - 0.01f, 0.0f));
             const uint32_t t = pq * j + ((pr * j * 2185u) >> 16) - rho;  // floor(pr j / 30): pr j < 900
             if (((kUnits30 >> j) & 1u) && t < run.nblk) {
                 const uint32_t k = __popc(kUnits30 & ((1u << j) - 1u));
                 if (b >= tbn) atomicOr(run0.err, kErrTable);
                 else if ((__ldg(mtab + (b >> 2)) >> (8 * (uint32_t(b) & 3u) + k)) & 1u) mark(ri, run.vbase, cls[k], t);
+            }
+            return;
+        }
+        if (run.nblk <= (p >> 2) && !(p >> 31)) {
+            // a few: the units among the next 30 nblk / p + 2 j (10 at most),
+            // the table read only for one inside the run
+            const float f30 = 30.0f * rp;
+            const uint32_t j0 = __float2uint_ru(fmaxf(__uint2float_rn(rho) * f30 - 0.01f, 0.0f));
+            const uint32_t n = __float2uint_rz(__uint2float_rn(run.nblk) * f30) + 3u;
+            for (uint32_t v = uint32_t(kUnits60 >> j0) & ((1u << n) - 1u); v; v &= v - 1u) {
+                uint32_t j = j0 + __ffs(v) - 1u;
+                const bool next = j >= 30;  // a unit of the byte after b0
+                j -= next ? 30u : 0u;
+                const uint32_t t = (next ? p : 0u) + pq * j + ((pr * j * 2185u) >> 16) - rho;
+                if (t < run.nblk) {
+                    const uint64_t at = b + (next ? 1u : 0u);
+                    const uint32_t k = __popc(kUnits30 & ((1u << j) - 1u));
+                    if (b >= tbn || at >= tbn) atomicOr(run0.err, kErrTable);
+                    else if ((__ldg(mtab + (at >> 2)) >> (8 * (uint32_t(at) & 3u) + k)) & 1u)
+                        mark(ri, run.vbase, cls[k], t);
+                }
             }
             return;
         }
@@ -844,11 +888,32 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
         const uint32_t p = p_next;
         if (i + stride < nhi) p_next = __ldg(primes + i + stride);  // its latency behind this prime's work
         const float rp = __fdividef(1.0f, __uint2float_rn(p));
-        const uint64_t inv = recip64(p, rp);
+        uint64_t inv = recip64(p, rp);
         const uint32_t pq = p / 30, pr = p - 30 * pq;
+        // A run of several narrower than p / 64: a pair goes on only if one of
+        // its integers is a multiple of p, which the remainder r of base - 1
+        // tells (the next multiple is base + p - 1 - r), so most warps stop
+        // there: 16 runs of 1e6 integers at 4e18..5e18 0.225 -> 0.146 ms a run.
+        // (A run alone would pay the exact reciprocal for one remainder; p >=
+        // 2^31: r takes 33 bits.)
+        uint32_t narrow = 0;
+        if (nrun > 1) {
+            inv = recip64_exact(p, inv);
+            narrow = p >> 31 ? 0u : p >> 6;
+        }
         for (uint32_t ri = 0; ri < nrun; ++ri) {
-            const HlRun run = s_run[ri];
-            if (i >= run.n_hl && i < run.n_all) pair(ri, p, rp, inv, pq, pr, run);
+            const uint64_t below = s_run[ri].below;
+            const uint32_t span = s_run[ri].span;
+            bool go = i < s_run[ri].n_all;
+            if (span < narrow) {
+                uint32_t r = uint32_t(below) - uint32_t(__umul64hi(below, inv)) * p;  // below 2 p
+                r = min(r, r - p);
+                go = go && r >= p - 1 - span;
+            }
+            if (go) {
+                const HlRun run = s_run[ri];  // in registers: the marks' atomics would have it read again
+                pair(ri, p, rp, inv, pq, pr, run);
+            }
             __syncwarp();
         }
     }

@@ -1,8 +1,8 @@
 """The hit-list harvest's placement of a prime's multiples (k_hitlist in
 goldbach-l0_gb300/csrc/k_sieve.cu), restated in exact float32 and integer
 arithmetic and compared with the general definition: the multiples q = p m of
-a run, m coprime to 30, as class bits, for runs narrower than p / 32 bits (one
-candidate multiplier), primes from 2^31 on (64-bit bits) and the word loop
+a run, m coprime to 30, as class bits, for runs narrower than p / 4 bits (a few
+candidate multipliers), primes from 2^31 on (64-bit bits) and the word loop
 (32-bit bits). A CPU test of the algorithm; the GPU tests check the kernel
 through every map bit."""
 import math
@@ -28,30 +28,56 @@ def recip64(p):
     return (q1 << 12) + c - 2
 
 
-def divmod_recip(x, p):
-    q = x * recip64(p) >> 64
+def recip64_exact(p):
+    inv = recip64(p)
+    e = 2**64 - inv * p
+    assert 0 <= e < 5 * p
+    for step in (2, 1):
+        if e >= p * step:
+            e -= p * step
+            inv += step
+    return inv + 1 if e >= p else inv
+
+
+def divmod_recip(x, p, recip=recip64):
+    q = x * recip(p) >> 64
     r = x - q * p
     assert 0 <= r < 2 * p
     return (q + 1, r - p) if r >= p else (q, r)
 
 
-def marks(base, nblk, p):
+def marks(base, nblk, p, several=False):
     """(class residue, bit) of every multiple p m in the run, m coprime to 30,
-    by the kernel's steps, every table bit taken as set."""
+    by the kernel's steps (several: of a batch of several runs), every table
+    bit taken as set."""
     rp = rn32(F(1, int(rn32(F(p)))))
-    b0, rho = divmod_recip(base // 30, p)
+    span = min(30 * nblk - 1, M32)
+    if several and span < p >> 6 and not p >> 31:
+        r = ((base - 1) - ((base - 1) * recip64_exact(p) >> 64) * p) & M32
+        assert r < 2 * p
+        r = min(r, (r - p) & M32)
+        if r < p - 1 - span:
+            return None, set()
+    b0, rho = divmod_recip(base // 30, p, recip64_exact if several else recip64)
     pq, pr = divmod(p, 30)
     out = set()
 
     def v(u):
         return pq * u + pr * u // 30
 
-    if nblk <= p >> 5:
+    one = nblk <= p >> 5
+    if one or (nblk <= p >> 2 and not p >> 31):
         a = rn32(rn32(F(rho)) * rn32(30 * rp))
-        j = math.ceil(max(rn32(a - rn32(F(1, 100))), 0))
-        t = (pq * j + ((pr * j * 2185) >> 16) - rho) & M32
-        if j in U30 and t < nblk:
-            out.add((p * j % 30, t))
+        j0 = math.ceil(max(rn32(a - rn32(F(1, 100))), 0))
+        n = 1 if one else f2u_rz(rn32(rn32(F(nblk)) * rn32(30 * rp))) + 3
+        assert j0 <= 30 and n <= 10
+        for j in range(j0, j0 + n):
+            nxt, j = j >= 30, j % 30
+            if j not in U30 or (nxt and one):
+                continue
+            t = ((p if nxt else 0) + pq * j + ((pr * j * 2185) >> 16) - rho) & M32
+            if t < nblk:
+                out.add((p * j % 30, t))
         return b0, out
     if p >> 31:
         for nb in range(2 if rho + nblk > p else 1):
@@ -89,7 +115,7 @@ PRIMES = [131, 1009, 65537, 1048573, 1048583, 1703941, 4194319, 16777259, 999999
 @pytest.mark.parametrize("p", PRIMES)
 def test_division_by_the_reciprocal(p):
     rnd = random.Random(p)
-    assert 0 <= 2**64 - recip64(p) * p < 5 * p + p
+    assert recip64_exact(p) == 2**64 // p and 0 <= 2**64 - recip64(p) * p < 6 * p
     top = (2**64 - 2**40) // 30
     for x in [0, 1, p - 1, p, top, top // p * p, top // p * p - 1] + [rnd.randrange(top) for _ in range(200)]:
         assert divmod_recip(x, p) == divmod(x, p)
@@ -98,7 +124,8 @@ def test_division_by_the_reciprocal(p):
 @pytest.mark.parametrize("p", PRIMES)
 def test_marks_equal_the_general_form(p):
     rnd = random.Random(p + 1)
-    widths = {1, 2, 33, max(p >> 5, 1), (p >> 5) + 1, p // 30 + 1, p // 2 + 1, p - 1, p, p + 1, 40 * p}
+    widths = {1, 2, 33, max(p >> 5, 1), (p >> 5) + 1, p // 30 + 1, p // 8, max(p >> 2, 1), (p >> 2) + 1, p // 2 + 1, p - 1,
+              p, p + 1, 40 * p}
     for nblk in sorted(w for w in widths if 0 < w < 2**31 and w < 4096 * p):
         if nblk // p > 50:
             continue
@@ -106,8 +133,9 @@ def test_marks_equal_the_general_form(p):
             # bases whose first multiple sits at either end of the run or anywhere
             m = rnd.randrange(p, max(p + 1, min(2**63 // p, 1 << 42)))
             off = rnd.choice((0, 30, -30, 30 * nblk, 30 * (nblk - 1), rnd.randrange(30 * p)))
-            base = max(0, p * m - off) // 30 * 30
-            assert marks(base, nblk, p)[1] == general(base, nblk, p), (p, nblk, base)
+            base = max(30, p * m - off) // 30 * 30
+            want = general(base, nblk, p)
+            assert marks(base, nblk, p)[1] == want and marks(base, nblk, p, True)[1] == want, (p, nblk, base)
 
 
 def test_small_product_division_by_30():
