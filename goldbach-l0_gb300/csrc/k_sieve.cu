@@ -843,10 +843,18 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
         }
         const uint32_t sh = uint32_t(b) & 3u, eb = sh + nb;  // the end byte from the first word's first
         const uint32_t *tw = mtab + (b >> 2);
-        const uint32_t hi_mask = 0xFFFFFFFFu >> (24 - 8 * (eb & 3u));
+        // the end bytes without most of the units outside the run: those below
+        // 30 rho / p, and from 30 (x - nb p + 1) / p on (estimates that err by
+        // 0.01 at most towards keeping one: a mark's own bit decides)
+        const float f30 = 30.0f * rp;
+        const uint32_t ja = __float2uint_ru(fmaxf(__uint2float_rn(rho) * f30 - 0.01f, 0.0f));
+        const uint32_t jb = __float2uint_rz(__uint2float_rn(x - nb * p + 1) * f30 + 0.01f);
+        const uint32_t lo8 = 0xFFu << __popc(kUnits30 & ((1u << ja) - 1u));
+        const uint32_t hi8 = (1u << __popc(kUnits30 & ((2u << jb) - 1u))) - 1u;
+        const uint32_t hi_mask = (0x00FFFFFFu >> (24 - 8 * (eb & 3u))) | (hi8 << (8 * (eb & 3u)));
         uint32_t left = eb >> 2;                             // words after the current one
         uint32_t tb = 0u - rho - p * sh;                     // bit of the word's byte 0, less its v_k
-        uint32_t v = __ldg(tw) & (0xFFFFFFFFu << (8 * sh));
+        uint32_t v = __ldg(tw) & ((0xFFFFFF00u | (lo8 & 0xFFu)) << (8 * sh));
         if (!left) v &= hi_mask;
         // the next table word loaded before this word's marks (its
         // latency hidden behind them); one mark per trip, whichever word

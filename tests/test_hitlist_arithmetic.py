@@ -91,8 +91,14 @@ def marks(base, nblk, p, several=False):
     elif x - nb * p >= p:
         nb += 1
     assert nb == x // p
+    f30 = rn32(30 * rp)
+    ja = math.ceil(max(rn32(rn32(rn32(F(rho)) * f30) - rn32(F(1, 100))), 0))
+    jb = f2u_rz(rn32(rn32(rn32(F(x - nb * p + 1)) * f30) + rn32(F(1, 100))))
+    assert ja <= 30 and jb <= 30
     for b in range(nb + 1):
         for u in U30:
+            if (b == 0 and u < ja) or (b == nb and u > jb):  # outside the end bytes' masks
+                continue
             t = (b * p + v(u) - rho) & M32
             if t < nblk:
                 out.add((p * u % 30, t))
