@@ -529,6 +529,15 @@ extern "C" int gbc_create(const gbc_config *cfg_in, gbc_ctx **out)
             uint2 &m = ck_mask[size_t(cr) * gbk::kCkWindows + w];
             (b < 32 ? m.y : m.x) |= 1u << (31 - b % 32);
         }
+    std::vector<uint16_t> ck_rank(size_t(GBC_NCLASS) * gbk::kCkFirst, 0);
+    ctx->ct.word = (cfg.test_flags & GBC_TEST_RETRY_LIMIT) ? 0 : 1;
+    for (uint32_t cr = 0; ctx->ct.word && cr < GBC_NCLASS; ++cr) {
+        for (uint32_t i = 0; i < gbk::kCkFirst; ++i) ck_rank[cr * gbk::kCkFirst + i] = list[list_off[cr] + i];
+        for (uint32_t n : {gbk::kCkFirst, gbk::kCkFew}) {
+            const uint32_t p = cand[list[list_off[cr] + n]], u = (2 * cr + 30 - p % 30) % 30;
+            (n == gbk::kCkFirst ? ctx->ct.w0 : ctx->ct.w0_few) |= uint64_t((p + u - 2 * cr) / 240) << (4 * cr);
+        }
+    }
     // verify plan (the reference's make_plan30, include/check30.hpp:88-174,
     // with our own greedy order): per class, the useful candidates below
     // GBC_TAIL_T in ascending order, each uncovered one p opening a funnel
@@ -628,10 +637,9 @@ extern "C" int gbc_create(const gbc_config *cfg_in, gbc_ctx **out)
     ctx->ct.cand = ctx->d_cand;
     ctx->ct.ci = ctx->d_ck_ci;
     ctx->ct.mask = ctx->d_ck_mask;
-    for (int cr = 0; cr < GBC_NCLASS; ++cr) {
-        ctx->ct.m0[cr] = ck_mask[size_t(cr) * gbk::kCkWindows];
-        ctx->ct.m1[cr] = ck_mask[size_t(cr) * gbk::kCkWindows + 1];
-    }
+    CK(dev_alloc(ctx, &ctx->d_ck_rank, ck_rank.size() * 2));
+    CK(cudaMemcpy(ctx->d_ck_rank, ck_rank.data(), ck_rank.size() * 2, cudaMemcpyHostToDevice));
+    ctx->ct.rank = ctx->d_ck_rank;
     ctx->ct.ridge_min = cfg.ridge_min;
     ctx->ct.ridge_w = cfg.ridge_min < 240 ? 0 : std::min<uint32_t>((cfg.ridge_min - 237) / 240, gbk::kCkWindows);
     // the plan's funnels as k_verify reads them: per class those the word form
@@ -690,6 +698,7 @@ extern "C" void gbc_destroy(gbc_ctx *ctx)
     cudaFree(ctx->d_cand);
     cudaFree(ctx->d_ck_ci);
     cudaFree(ctx->d_ck_mask);
+    cudaFree(ctx->d_ck_rank);
     delete ctx;
 }
 
@@ -842,6 +851,7 @@ static void finish_desc(const gbc_ctx *ctx, DescImage &img)
         img.ver_pref[i] = h.ver_vb;
         img.cnt_pref[i] = h.cnt_vb;
         const uint64_t evens = (sp.seg_end - sp.seg_start) / 2 + 1;
+        sp.ck_few = gbh::check_few(sp.seg_start) ? 1 : 0;
         if (sp.sampled) gbh::check_split(evens, sampled_words, ctx->grids.sm, &sp.cw, &sp.vbx);
         else sp.vbx = gbh::verify_vbx(evens, ctx->grids.sm);
         if (sp.low) ++h.nlow;

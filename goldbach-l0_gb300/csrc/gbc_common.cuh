@@ -175,6 +175,7 @@ struct SegParams {
     uint32_t run;                 // the segment's run (class map) in the batch
     uint32_t vbx;                 // checker CTAs of the segment
     uint32_t cw;                  // words per chunk of the exact checker
+    uint32_t ck_few;              // 1: the exact checker's word form takes kCkFew candidates
     uint32_t cnt_words, cnt_rounds;  // words per round and rounds per item of the count kernel
     CountRanges cr;
 };
@@ -272,8 +273,10 @@ __device__ __forceinline__ void transpose_word(const uint32_t (&h)[8], uint32_t 
     }
 }
 
-// windows of eight blocks the exact checker reads below an even: p <= 9781
+// windows of eight blocks the exact checker reads below an even: p <= 9781;
+// candidates of a class its word form takes (kCkFew in segments below 1e17)
 constexpr uint32_t kCkWindows = 41;
+constexpr uint32_t kCkFirst = 40, kCkFew = 24;
 
 // Candidate tables of the exact checker (uploaded once per context). Window
 // w of class c = r / 2 holds the blocks T - 8 w - 7 .. T - 8 w of the even
@@ -282,10 +285,12 @@ constexpr uint32_t kCkWindows = 41;
 struct CheckTables {
     const uint16_t *cand;   // odd primes 3..9781
     const uint16_t *ci;     // [c][64 w + b]: the candidate's index
+    const uint16_t *rank;   // [c][i]: the class's i-th candidate's index, i < kCkFirst
     const uint2 *mask;      // [c][w]: the window's candidate bits (x: low, y: high word)
-    uint2 m0[GBC_NCLASS], m1[GBC_NCLASS];  // mask[c][0], mask[c][1]
+    uint64_t w0, w0_few;    // 4 bits per class: the window of candidate kCkFirst, of kCkFew
     uint32_t ridge_min;     // evens with p(n) >= ridge_min are listed with their p(n)
     uint32_t ridge_w;       // the first window with a candidate >= ridge_min
+    uint32_t word;          // 1: the candidates are the word form's (0: cut short for a test)
 };
 
 // Funnel plan of the verify (phase A) checker and the ascending rest lists
@@ -494,6 +499,7 @@ void query_verify_grids(Grids &g);
 bool verify_word_funnel(uint32_t r, uint32_t p0, uint32_t members);
 void query_count_grids(Grids &g);
 void check_split(uint64_t evens, uint64_t words, int sm, uint32_t *cw, uint32_t *vbx);
+bool check_few(uint64_t seg_start);
 uint32_t verify_vbx(uint64_t evens, int sm);
 // single-run forms (the allocation-free entry point and the table build)
 void launch_xfirst1(const gbk::BatchParams &bp, cudaStream_t st);

@@ -91,7 +91,7 @@ struct gbc_ctx {
     uint32_t wpc_cap = 0;              // class-array words of max_batch full segments in one run
     DescLayout layout;
     uint32_t *d_primes = nullptr, *d_magic = nullptr, *d_pat = nullptr;
-    uint16_t *d_wheel = nullptr, *d_cand = nullptr, *d_ck_ci = nullptr;
+    uint16_t *d_wheel = nullptr, *d_cand = nullptr, *d_ck_ci = nullptr, *d_ck_rank = nullptr;
     uint8_t *d_pk_gap = nullptr;   // packed large primes from n_mid: half gaps
     uint32_t *d_pk_base = nullptr; // and the first prime of each group
     uint2 *d_ev = nullptr, *d_ck_mask = nullptr;

@@ -14,6 +14,7 @@
 
 #include <algorithm>
 #include <cstddef>
+#include <utility>
 
 #include "gbc_common.cuh"
 
@@ -39,45 +40,154 @@ __device__ __forceinline__ void append_ridge(gbc_segment_result *res, uint64_t n
 
 // ---- p(n) of every even of a sampled segment -----------------------------------
 //
-// In class bits of a run the even n = base + 30 T + r and the prime q = base +
-// 30 (T - i) + u_k meet in p = 30 i + r - u_k: the largest q below n whose
-// distance is a candidate is the witness of p(n). So the class arrays are
-// transposed to one byte per block of 30 (bit k: class k), where q ascends, and
-// a 64-bit window of eight blocks ending at T is ANDed with the class's mask
-// of the candidates it reaches: its highest bit is p(n). The window of T serves
-// all fifteen classes (classes with few candidates in it take the next one
-// too); about 96 evens in a hundred are settled. The others go to a queue of the
-// warp, which takes the windows below (kCkWindows in all, the candidates to
-// 9781) one T per lane.
+// Word form. In class bits of a run (base a multiple of 30) the even n = base +
+// 30 T + r of class r and the candidate p = s + 30 d meet in bit T - o of array
+// (r - s) mod 30, o = d + [r < s], so the evens T = 32 j .. 32 j + 31 of every
+// class sit in word j. A lane takes word j of all eight arrays and settles the
+// class's first candidates in ascending order, each a funnel shift and an AND
+// over 32 evens; their counts are the differences of the evens still open after
+// each (a popcount, two of them per warp reduction). Offsets and arrays are
+// constants. A candidate settles 3.75 / ln q of the open evens: kCkFirst of them
+// from 1e17 on (about 97 evens in a hundred settled), kCkFew below, where that
+// many settle as much and the later ones are too rare to have been seen.
 //
-// A mark in the histogram is a shared-memory atomic at (class, bit of the
-// window), for the first kCkHist windows; at the item's end the bits become
-// candidates. First occurrences need a look only at candidates not seen
-// before the present part: an item's evens ascend from part to part.
+// Even form. The class arrays of a chunk are transposed to one byte per block
+// of 30 (bit k: class k), where q ascends, and a 64-bit window of eight blocks
+// ending at T is ANDed with the class's mask of the candidates it reaches: the
+// largest q below n whose distance is a candidate is the witness of p(n), so the
+// highest bit is it. The words the word form leaves open go to a queue of the
+// warp and are taken from there, a word per lane, even by even through the
+// windows from the class's next candidate on (kCkWindows in all, the candidates
+// to 9781).
 //
-// Bound by the ALU pipe (18 ALU of 32 instructions per 32 evens, issue 76%).
-// One GB300, p(n) of every even: 48 segments of 467.5M at 4e18 11.8 ms
-// against 17.6 for candidates tested over words of 32 evens until the last
-// even of 4096 was settled; 195 segments of uneven windows 36.5 against 53.4;
-// 1e7 evens at 1e12 with the p(n) array 0.08 against 1.45.
+// An item's evens ascend from part to part (a few words, the rest of the first
+// chunk, the other chunks), so a candidate seen before a part cannot come first
+// in it. Words of classes with an unseen candidate among the first ones, the
+// words at a segment's ends, and every word where p(n) or a low ridge floor
+// wants each even, take the even form alone, a T per lane.
+//
+// __BOUND__
 constexpr int kCkThreads = 512;
 constexpr int kCkCtas = 2;                         // CTAs per SM
 constexpr uint32_t kCkWarps = kCkThreads / 32;
 constexpr uint32_t kCkHalo = 11;                   // words below a chunk: 41 windows of 8 blocks reach 335 back
 constexpr uint32_t kCkWords = kCkThreads - kCkHalo;  // words of a full chunk: one word per thread staged
 constexpr uint32_t kCkHist = 8;                    // windows counted in shared memory
-constexpr uint32_t kCkRow = 64 * kCkHist + 2;
+constexpr uint32_t kCkQueue = 32 * GBC_NCLASS;     // words of a warp's queue: a block's of every class
 static_assert(32 * kCkHalo >= 8 * kCkWindows + 7, "the last window is staged");
+static_assert(kCkWords <= 512 && kCkFirst % 2 == 0 && kCkFew % 2 == 0, "queue entries and candidate pairs");
 
 struct CkShared {
-    uint32_t hist[GBC_NCLASS][kCkRow];             // the windows' bits, after windows 0 and 1 one entry for none
+    uint32_t hist[GBC_NCLASS][64 * kCkHist];       // even form: marks by bit of the windows
+    uint32_t open[GBC_NCLASS][kCkFirst + 1];       // word form: evens taken, and those open after each candidate
     uint4 mask[GBC_NCLASS][kCkWindows];            // x, y: the window's candidates; z, w: those seen before the part
     uint32_t first[GBC_NCAND];
-    uint32_t slow;                                 // classes with a window-0 candidate not seen yet
+    uint32_t w0[GBC_NCLASS];                       // CheckTables::w0
+    uint32_t slow;                                 // classes that take the even form alone
     uint32_t vb;
-    uint32_t queue[kCkWarps][32];                  // a step's T with open classes: classes << 16 | block in the chunk
+    uint32_t q_bits[kCkWarps][kCkQueue];           // open evens of a word ...
+    uint16_t q_at[kCkWarps][kCkQueue];             // ... class << 9 | word in the chunk
     __align__(16) uint32_t bytes[8 * kCkThreads + 4];  // one byte per block, halo first; a window reads three words
 };
+
+namespace ckw {
+
+struct Cand {
+    uint32_t k, o, p;
+};
+// the i-th candidate of class r: ascending odd primes p with r - p a unit
+constexpr Cand cand(uint32_t r, uint32_t i)
+{
+    for (uint32_t p = 3;; p += 2) {
+        bool prime = true;
+        for (uint32_t d = 3; d * d <= p; d += 2) prime = prime && p % d != 0;
+        const uint32_t k = class_of((r + 30 - p % 30) % 30);
+        if (prime && k < 8 && i-- == 0) return Cand{k, p / 30 + (r < p % 30 ? 1u : 0u), p};
+    }
+}
+template <uint32_t R, uint32_t I>
+struct Of {
+    static constexpr Cand c = cand(R, I);
+    static_assert(c.o <= 32, "the candidate reads words j - 1 and j");
+};
+
+// words j - 1 (x) and j (y) of the eight arrays (members, not an array: every
+// access is by a constant, and an array went to local memory)
+struct Words {
+    uint2 a0, a1, a2, a3, a4, a5, a6, a7;
+};
+template <uint32_t K>
+__device__ __forceinline__ uint2 words_of(const Words &w)
+{
+    if constexpr (K == 0) return w.a0;
+    else if constexpr (K == 1) return w.a1;
+    else if constexpr (K == 2) return w.a2;
+    else if constexpr (K == 3) return w.a3;
+    else if constexpr (K == 4) return w.a4;
+    else if constexpr (K == 5) return w.a5;
+    else if constexpr (K == 6) return w.a6;
+    else return w.a7;
+}
+
+// the bits T - O of array K for the evens T of word j
+template <uint32_t K, uint32_t O>
+__device__ __forceinline__ uint32_t bits_at(const Words &w)
+{
+    const uint2 a = words_of<K>(w);
+    if constexpr (O == 0) return a.y;
+    else if constexpr (O == 32) return a.x;
+    else return __funnelshift_l(a.x, a.y, O);
+}
+
+template <uint32_t R, uint32_t I>
+__device__ __forceinline__ void two(const Words &w, uint32_t &un, uint32_t *open, uint32_t lane)
+{
+    un &= ~bits_at<Of<R, I>::c.k, Of<R, I>::c.o>(w);
+    const uint32_t n0 = __popc(un);
+    un &= ~bits_at<Of<R, I + 1>::c.k, Of<R, I + 1>::c.o>(w);
+    const uint32_t n = __reduce_add_sync(~0u, n0 | (__popc(un) << 16));  // at most 1024 each
+    if (lane < 2) atomicAdd(open + I + 1 + lane, lane ? n >> 16 : n & 0xFFFFu);
+}
+
+// class R's candidates From, ... over a word per lane; un: its evens, then those still open
+template <uint32_t R, uint32_t From, size_t... H>
+__device__ __forceinline__ void run(const Words &w, uint32_t &un, uint32_t *open, uint32_t lane,
+                                    std::index_sequence<H...>)
+{
+    (two<R, From + 2 * H>(w, un, open, lane), ...);
+}
+
+// the same for class C, and its words with open evens into the queue (place:
+// the lane's word in the chunk)
+template <uint32_t C>
+__device__ __forceinline__ void one(const Words &w, bool inner, uint32_t taken, uint32_t slow, bool few, CkShared &sh,
+                                     uint32_t *q_bits, uint16_t *q_at, uint32_t place,
+                                    uint32_t lane, uint32_t &qn)
+{
+    if (slow >> C & 1u) return;
+    uint32_t un = inner ? ~0u : 0u;
+    if (lane == 0) atomicAdd(&sh.open[C][0], taken);
+    run<2 * C, 0>(w, un, sh.open[C], lane, std::make_index_sequence<kCkFew / 2>());
+    if (!few) run<2 * C, kCkFew>(w, un, sh.open[C], lane, std::make_index_sequence<(kCkFirst - kCkFew) / 2>());
+    const uint32_t bal = __ballot_sync(~0u, un != 0);
+    if (un) {
+        const uint32_t at = qn + __popc(bal & ((1u << lane) - 1u));
+        q_bits[at] = un;
+        q_at[at] = uint16_t((C << 9) | place);
+    }
+    qn += __popc(bal);
+}
+
+template <size_t... C>
+__device__ __forceinline__ void all(const Words &w, bool inner, uint32_t slow, bool few, CkShared &sh,
+                                     uint32_t *q_bits, uint16_t *q_at, uint32_t place, uint32_t lane,
+                                    uint32_t &qn, std::index_sequence<C...>)
+{
+    const uint32_t taken = 32 * __popc(__ballot_sync(~0u, inner));
+    (one<C>(w, inner, taken, slow, few, sh, q_bits, q_at, place, lane, qn), ...);
+}
+
+}  // namespace ckw
 
 // bytes at - 7 .. at of the staged blocks as two words (byte `at` topmost)
 __device__ __forceinline__ void ck_window(const uint32_t *bytes, uint32_t at, uint32_t &lo, uint32_t &hi)
@@ -89,17 +199,18 @@ __device__ __forceinline__ void ck_window(const uint32_t *bytes, uint32_t at, ui
     hi = __funnelshift_r(w1, w2, s);
 }
 
-// Class c = r / 2 takes windows 0 and 1 at once, for every T: r is prime to 3
-// (19 or 26 candidates in a window, 39 or 50 in the others').
-__host__ __device__ __forceinline__ constexpr bool ck_wide(uint32_t c) { return c % 3 != 0; }
-
 __global__ void __launch_bounds__(kCkThreads, kCkCtas) k_check(BatchDesc d, CheckTables ct)
 {
     extern __shared__ __align__(16) uint8_t s_ck[];
     CkShared &sh = *reinterpret_cast<CkShared *>(s_ck);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t total = d.h->chk_vb, nseg = d.h->nseg;
-    uint32_t *const queue = sh.queue[warp];
+    uint32_t *const q_bits = sh.q_bits[warp];
+    uint16_t *const q_at = sh.q_at[warp];
+    // (locals: the lambdas below would take the address of a copy of ct)
+    const uint16_t *const ct_ci = ct.ci, *const ct_cand = ct.cand;
+    const uint32_t ridge_w = ct.ridge_w, ridge_min = ct.ridge_min;
+    const bool words = ct.word != 0;
     for (uint32_t i = tid; i < GBC_NCLASS * kCkWindows; i += kCkThreads) {
         const uint2 m = ct.mask[i];
         sh.mask[0][i] = make_uint4(m.x, m.y, 0u, 0u);
@@ -123,40 +234,42 @@ __global__ void __launch_bounds__(kCkThreads, kCkCtas) k_check(BatchDesc d, Chec
         const uint32_t jlo = A >> 5, jhi = B >> 5;
         const uint32_t nch = (jhi - jlo) / cw + 1;
         const uint32_t c0 = uint32_t(uint64_t(nch) * bx / sp.vbx), c1 = uint32_t(uint64_t(nch) * (bx + 1) / sp.vbx);
-        for (uint32_t i = tid; i < GBC_NCLASS * kCkRow; i += kCkThreads) sh.hist[0][i] = 0;
+        const bool few = sp.ck_few != 0;
+        if (tid < GBC_NCLASS) sh.w0[tid] = uint32_t((few ? ct.w0_few : ct.w0) >> (4 * tid)) & 15u;
+        for (uint32_t i = tid; i < GBC_NCLASS * 64 * kCkHist; i += kCkThreads) sh.hist[0][i] = 0;
+        for (uint32_t i = tid; i < GBC_NCLASS * (kCkFirst + 1); i += kCkThreads) sh.open[0][i] = 0;
         for (uint32_t i = tid; i < GBC_NCAND; i += kCkThreads) sh.first[i] = kNone;
         // everything of an even but its histogram mark: first occurrence, p(n), ridge
         auto note = [&](uint32_t c, uint32_t bit, uint32_t T) {
-            const uint32_t ci = __ldg(ct.ci + c * (64 * kCkWindows) + bit), idx = 15 * T + c - D;
+            const uint32_t ci = __ldg(ct_ci + c * (64 * kCkWindows) + bit), idx = 15 * T + c - D;
             if (sh.first[ci] > idx) atomicMin(&sh.first[ci], idx);
-            if (pn || bit >= 64 * ct.ridge_w) {
-                const uint32_t p = __ldg(ct.cand + ci);
+            if (pn || bit >= 64 * ridge_w) {
+                const uint32_t p = __ldg(ct_cand + ci);
                 if (pn) pn[idx] = uint16_t(p);
-                if (p >= ct.ridge_min) append_ridge(res, bp.base + 30ull * T + 2 * c, p);
+                if (p >= ridge_min) append_ridge(res, bp.base + 30ull * T + 2 * c, p);
             }
             return ci;
         };
-        // The candidates of the counted windows seen before word j (every one
-        // when notes are for first occurrences only: p(n) and ridges note all):
-        // theirs cannot come first from j on. Between barriers.
+        // The candidates of the counted windows seen before word j: theirs cannot
+        // come first from j on (none where p(n) or a ridge wants each even). And
+        // the classes not all of whose first candidates are. Between barriers.
         auto look = [&](uint32_t j) {
             if (tid == 0) sh.slow = 0;
             __syncthreads();
             const uint32_t idx0 = j == jlo ? 0u : 15 * 32 * j - D;  // no even from word j on has a smaller index
             for (uint32_t i = warp; i < GBC_NCLASS * kCkHist; i += kCkWarps) {
                 const uint32_t c = i / kCkHist, w = i % kCkHist;
-                const uint16_t *ci = ct.ci + c * (64 * kCkWindows) + 64 * w;
+                const uint16_t *ci = ct_ci + c * (64 * kCkWindows) + 64 * w;
                 const uint4 m = sh.mask[c][w];
                 // lane l: bits l and 32 + l from the top
                 const bool hi = (m.y >> (31 - lane) & 1u) && sh.first[__ldg(ci + lane)] < idx0;
                 const bool lo = (m.x >> (31 - lane) & 1u) && sh.first[__ldg(ci + 32 + lane)] < idx0;
                 const uint32_t sy = __brev(__ballot_sync(~0u, hi)), sx = __brev(__ballot_sync(~0u, lo));
-                const bool all = pn || w >= ct.ridge_w;
+                const bool all = pn || w >= ridge_w || !words;
                 if (lane == 0) {
                     sh.mask[c][w].z = all ? 0u : sx;
                     sh.mask[c][w].w = all ? 0u : sy;
-                    if ((w == 0 || (w == 1 && ck_wide(c))) && (all || sx != m.x || sy != m.y))
-                        atomicOr(&sh.slow, 1u << c);
+                    if (w <= sh.w0[c] && (all || sx != m.x || sy != m.y)) atomicOr(&sh.slow, 1u << c);
                 }
             }
             __syncthreads();
@@ -170,128 +283,155 @@ __global__ void __launch_bounds__(kCkThreads, kCkCtas) k_check(BatchDesc d, Chec
                 uint32_t h[8];
 #pragma unroll
                 for (uint32_t k = 0; k < 8; ++k) h[k] = j < wpc ? __ldg(map + size_t(k) * wpc + j) : 0u;
-                uint4 o[2];
-                uint32_t *t = reinterpret_cast<uint32_t *>(o);
+                uint32_t t[8];
                 transpose_word(h, t);
                 uint4 *dst = reinterpret_cast<uint4 *>(sh.bytes + 8 * tid);
-                dst[0] = o[0];
-                dst[1] = o[1];
+                dst[0] = make_uint4(t[0], t[1], t[2], t[3]);
+                dst[1] = make_uint4(t[4], t[5], t[6], t[7]);
             }
             look(j0);
-            // The classes of one T left open by window 0, one T per lane: the
-            // open classes qm, its block in the chunk, and for the highest open
-            // class the next window. A lane that is done takes the queue's last
-            // T. Ends with the queue empty (a T may stay with a lane), or with
-            // all settled.
-            uint32_t qn = 0, qm = 0, qt = 0, qw = 0;  // qw 0: the class's first queue window
+            // The queue's words, one per lane, even by even: the word's open evens
+            // qm, its class and place, and for the highest open even the next
+            // window from q0 (+ the class's first) on. A lane that is done takes
+            // the queue's last word. Ends with the queue empty (words may stay
+            // with lanes), or with all settled.
+            uint32_t qn = 0, qm = 0, qc = 0, qj = 0, qw = 0;
             auto settle = [&](bool finish) {
+                __syncwarp();
                 for (;;) {
                     const uint32_t idle = __ballot_sync(~0u, qm == 0);
                     if (qn) {
                         const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
                         if (qm == 0 && rank < qn) {
-                            const uint32_t e = queue[qn - 1 - rank];
-                            qm = e >> 16;
-                            qt = e & 0xFFFFu;
+                            const uint32_t at = q_at[qn - 1 - rank];
+                            qm = q_bits[qn - 1 - rank];
+                            qc = at >> 9;
+                            qj = at & 511u;
+                            qw = sh.w0[qc];
                         }
                         qn -= min(qn, uint32_t(__popc(idle)));
                     } else if (!finish || idle == ~0u) {
                         break;
                     }
-                    // (an idle lane goes through the motions of class 0 without a mark)
+                    // (an idle lane goes through the motions of its last even without a mark)
                     const bool busy = qm != 0;
-                    const uint32_t c = busy ? 31u - __clz(qm) : 0u;
-                    if (!qw) qw = ck_wide(c) ? 2u : 1u;
+                    const uint32_t eb = busy ? 31u - __clz(qm) : 0u, qt = 32 * qj + eb;
                     uint32_t lo, hi;
                     ck_window(sh.bytes, 32 * kCkHalo + qt - 8 * qw, lo, hi);
-                    const uint4 m = sh.mask[c][qw];
+                    const uint4 m = sh.mask[qc][qw];
                     lo &= m.x;
                     hi &= m.y;
                     const uint32_t z = hi ? hi : lo, b = __clz(z);
                     const bool hit = busy && z;
                     const uint32_t bit = 64 * qw + b + (hi ? 0u : 32u);
-                    if (hit && qw < kCkHist) atomicAdd(&sh.hist[c][bit + min(qw, 2u)], 1u);
+                    if (hit && qw < kCkHist) atomicAdd(&sh.hist[qc][bit], 1u);
                     const bool seen = (hi ? m.w : m.z) << b >> 31;
-                    bool last = qw + 1 == kCkWindows;
+                    const bool last = qw + 1 == kCkWindows;
                     if ((hit && !seen) || (busy && last)) {  // rare
                         if (hit) {
-                            const uint32_t ci = note(c, bit, 32 * j0 + qt);
-                            if (qw >= kCkHist) atomicAdd(&res->hist[c][ci], 1u);
+                            const uint32_t ci = note(qc, bit, 32 * j0 + qt);
+                            if (qw >= kCkHist) atomicAdd(&res->hist[qc][ci], 1u);
                         } else {
-                            append_leftover(res, bp.base + 30ull * (32 * j0 + qt) + 2 * c);
+                            append_leftover(res, bp.base + 30ull * (32 * j0 + qt) + 2 * qc);
                         }
                     }
                     __syncwarp();
-                    const bool done = hit || last;
-                    qw = done || !busy ? 0u : qw + 1;
-                    if (done) qm &= ~(1u << c);
+                    const bool done = busy && (hit || last);
+                    if (done) qm &= ~(1u << eb);
+                    qw = done ? sh.w0[qc] : busy ? qw + 1 : qw;
                 }
                 __syncwarp();
             };
+            // word j of the classes in `classes` in the even form, a T per lane:
+            // the windows to the class's w0; the others' evens into the queue
+            auto even_word = [&](uint32_t j, uint32_t classes) {
+                const uint32_t T = 32 * j + lane, tl = T - 32 * j0;
+#pragma unroll 1
+                for (; classes; classes &= classes - 1u) {
+                    const uint32_t c = __ffs(classes) - 1u;
+                    bool open = T >= A + (2 * c < ra ? 1u : 0u) && T <= B - (2 * c > rb ? 1u : 0u);
+                    for (uint32_t w = 0; w <= sh.w0[c]; ++w) {
+                        uint32_t lo, hi;
+                        ck_window(sh.bytes, 32 * kCkHalo + tl - 8 * w, lo, hi);
+                        const uint4 m = sh.mask[c][w];
+                        lo &= m.x;
+                        hi &= m.y;
+                        if (open && (lo | hi)) {
+                            const uint32_t b = hi ? __clz(hi) : __clz(lo), bit = 64 * w + b + (hi ? 0u : 32u);
+                            atomicAdd(&sh.hist[c][bit], 1u);
+                            if (!((hi ? m.w : m.z) << b >> 31)) note(c, bit, T);
+                            open = false;
+                        }
+                        __syncwarp();
+                    }
+                    const uint32_t left = __ballot_sync(~0u, open);
+                    if (left) {
+                        if (lane == 0) {
+                            q_bits[qn] = left;
+                            q_at[qn] = uint16_t((c << 9) | (j - j0));
+                        }
+                        ++qn;
+                    }
+                }
+            };
             // the item's first chunk in two parts: a few words, after which the
-            // window-0 candidates have been seen, then the others
+            // first candidates have been seen, then the others
             const uint32_t jm = ch == c0 ? min(j0 + 4 * kCkWarps, j1) : j1;
             for (uint32_t part = 0, ja = j0, jb = jm; ja < jb; ++part, ja = jm, jb = part == 1 ? j1 : jm) {
                 if (part) {
                     __syncthreads();
                     look(ja);
                 }
+                constexpr uint32_t kAll = (1u << GBC_NCLASS) - 1u;
                 const uint32_t slow = sh.slow;
-                for (uint32_t j = ja + warp; j < jb; j += kCkWarps) {
-                    const uint32_t T = 32 * j + lane, tl = T - 32 * j0;
-                    uint32_t lo, hi, lo1, hi1, open = 0;  // open: classes these windows leave open at T
-                    ck_window(sh.bytes, 32 * kCkHalo + tl, lo, hi);
-                    ck_window(sh.bytes, 32 * kCkHalo + tl - 8, lo1, hi1);
-                    if (j > jlo && j < jhi && !slow) {
-#pragma unroll
-                        for (uint32_t c = 0; c < GBC_NCLASS; ++c) {
-                            // branchless: an even left open marks the row's entry for none
-                            const uint32_t y = lo & ct.m0[c].x;
-                            uint32_t z = hi & ct.m0[c].y, at = z ? 0u : 32u;
-                            z = z ? z : y;
-                            if (ck_wide(c)) {
-                                const uint32_t u = hi1 & ct.m1[c].y, v = lo1 & ct.m1[c].x;
-                                at = z ? at : 65u;
-                                z = z ? z : u;
-                                at = z ? at : 97u;
-                                z = z ? z : v;
-                            }
-                            atomicAdd(&sh.hist[c][at + __clz(z)], 1u);
-                            open |= z ? 0u : 1u << c;
-                        }
-                    } else {
-                        // a word at the segment's ends, or candidates not all seen yet
-#pragma unroll 1
-                        for (uint32_t c = 0; c < GBC_NCLASS; ++c) {
-                            const bool in = T >= A + (2 * c < ra ? 1u : 0u) && T <= B - (2 * c > rb ? 1u : 0u);
-                            const uint4 m = sh.mask[c][0], m1 = sh.mask[c][1];
-                            const uint32_t x = hi & m.y, y = lo & m.x;
-                            const uint32_t u = ck_wide(c) ? hi1 & m1.y : 0u, v = ck_wide(c) ? lo1 & m1.x : 0u;
-                            if (in && (x | y | u | v)) {
-                                const uint32_t bit =
-                                    x ? __clz(x) : y ? 32u + __clz(y) : u ? 64u + __clz(u) : 96u + __clz(v);
-                                atomicAdd(&sh.hist[c][bit + (bit >> 6)], 1u);
-                                if (slow >> c & 1u) note(c, bit, T);
-                            } else if (in) {
-                                open |= 1u << c;
-                            }
-                            __syncwarp();
-                        }
+                if (slow == kAll) {
+                    for (uint32_t j = ja + warp; j < jb; j += kCkWarps) {
+                        even_word(j, kAll);
+                        settle(false);
                     }
-                    const uint32_t any = __ballot_sync(~0u, open != 0);
-                    if (open) queue[__popc(any & ((1u << lane) - 1u))] = (open << 16) | tl;
-                    qn = __popc(any);
-                    __syncwarp();
-                    settle(j + kCkWarps >= jb);
+                } else {
+                    for (uint32_t jw = ja + 32 * warp; jw < jb; jw += 32 * kCkWarps) {
+                        // a word per lane; the segment's end words and slow classes apart
+                        const uint32_t j = jw + lane;
+                        const bool inner = j < jb && j > jlo && j < jhi;
+                        const uint32_t *const at = map + (inner ? j : jlo + 1);
+                        auto pair = [&](uint32_t k) {
+                            return make_uint2(__ldg(at + size_t(k) * wpc - 1), __ldg(at + size_t(k) * wpc));
+                        };
+                        const ckw::Words w{pair(0), pair(1), pair(2), pair(3), pair(4), pair(5), pair(6), pair(7)};
+                        ckw::all(w, inner, slow, few, sh, q_bits, q_at, j - j0, lane, qn,
+                                 std::make_index_sequence<GBC_NCLASS>());
+                        settle(false);
+                        const uint32_t je = min(jw + 32, jb);
+                        if (slow)
+                            for (uint32_t i = jw; i < je; ++i)
+                                if (i > jlo && i < jhi) {
+                                    even_word(i, slow);
+                                    settle(false);
+                                }
+                        if (jlo >= jw && jlo < je) even_word(jlo, kAll);
+                        if (jhi >= jw && jhi < je && jhi != jlo) {
+                            settle(false);
+                            even_word(jhi, kAll);
+                        }
+                        settle(false);
+                    }
                 }
+                settle(true);
             }
         }
         __syncthreads();
-        for (uint32_t i = tid; i < GBC_NCLASS * kCkRow; i += kCkThreads) {
-            const uint32_t v = sh.hist[0][i], c = i / kCkRow, at = i % kCkRow;
-            if (!v || at == 64 || at == 129) continue;
-            const uint32_t bit = at - (at > 129 ? 2u : at > 64 ? 1u : 0u);
-            atomicAdd(&res->hist[c][__ldg(ct.ci + c * (64 * kCkWindows) + bit)], v);
+        for (uint32_t i = tid; i < GBC_NCLASS * 64 * kCkHist; i += kCkThreads) {
+            const uint32_t v = sh.hist[0][i];
+            if (!v) continue;
+            const uint32_t c = i / (64 * kCkHist), bit = i % (64 * kCkHist);
+            atomicAdd(&res->hist[c][__ldg(ct_ci + c * (64 * kCkWindows) + bit)], v);
+        }
+        for (uint32_t i = tid; i < GBC_NCLASS * kCkFirst; i += kCkThreads) {
+            const uint32_t c = i / kCkFirst, at = i % kCkFirst;
+            if (few && at >= kCkFew) continue;
+            const uint32_t v = sh.open[c][at] - sh.open[c][at + 1];
+            if (v) atomicAdd(&res->hist[c][__ldg(ct.rank + i)], v);
         }
         for (uint32_t i = tid; i < GBC_NCAND; i += kCkThreads)
             if (sh.first[i] != kNone) atomicMin(&res->first[i], sh.first[i]);
@@ -504,6 +644,9 @@ void check_split(uint64_t evens, uint64_t words, int sm, uint32_t *cw, uint32_t 
     const uint64_t per = std::min<uint64_t>(16, std::max<uint64_t>(1, words / *cw / (3 * want)));
     *vbx = uint32_t((nch + per - 1) / per);
 }
+
+// whether a segment takes the word form's kCkFew candidates
+bool check_few(uint64_t seg_start) { return seg_start < 100000000000000000ull; }
 
 void launch_check(const gbk::BatchDesc &d, const gbk::CheckTables &ct, const Grids &g, cudaStream_t st)
 {
