@@ -66,7 +66,12 @@ __device__ __forceinline__ void append_ridge(gbc_segment_result *res, uint64_t n
 // words at a segment's ends, and every word where p(n) or a low ridge floor
 // wants each even, take the even form alone, a T per lane.
 //
-// __BOUND__
+// Bound by issue. One GB300, p(n) of every even: 48 segments of 467.5M at 4e18
+// 8.0 ms (36 candidates in the word form 8.3, 48 8.6; the even form alone, two
+// windows a T, 11.8) against 17.6 for candidates tested over words of 32 evens
+// until the last even of 4096 was settled; 195 segments of uneven windows 24.5
+// against 53.4; 5e8 evens at 1e12 0.45 against 0.69 (with 40 candidates there
+// 1.04: the last ones are seen late); 1e7 with the p(n) array 0.10 against 1.45.
 constexpr int kCkThreads = 512;
 constexpr int kCkCtas = 2;                         // CTAs per SM
 constexpr uint32_t kCkWarps = kCkThreads / 32;
@@ -140,21 +145,22 @@ __device__ __forceinline__ uint32_t bits_at(const Words &w)
 }
 
 template <uint32_t R, uint32_t I>
-__device__ __forceinline__ void two(const Words &w, uint32_t &un, uint32_t *open, uint32_t lane)
+__device__ __forceinline__ void two(const Words &w, uint32_t &un, uint32_t *open, uint32_t lane, uint32_t half)
 {
     un &= ~bits_at<Of<R, I>::c.k, Of<R, I>::c.o>(w);
     const uint32_t n0 = __popc(un);
     un &= ~bits_at<Of<R, I + 1>::c.k, Of<R, I + 1>::c.o>(w);
-    const uint32_t n = __reduce_add_sync(~0u, n0 | (__popc(un) << 16));  // at most 1024 each
-    if (lane < 2) atomicAdd(open + I + 1 + lane, lane ? n >> 16 : n & 0xFFFFu);
+    const uint32_t n = __reduce_add_sync(~0u, n0 + (__popc(un) << 16));  // at most 1024 each
+    // lanes 0 and 1 add a half each
+    if (lane < 2) atomicAdd(open + I + 1, __byte_perm(n, 0u, half));
 }
 
 // class R's candidates From, ... over a word per lane; un: its evens, then those still open
 template <uint32_t R, uint32_t From, size_t... H>
-__device__ __forceinline__ void run(const Words &w, uint32_t &un, uint32_t *open, uint32_t lane,
+__device__ __forceinline__ void run(const Words &w, uint32_t &un, uint32_t *open, uint32_t lane, uint32_t half,
                                     std::index_sequence<H...>)
 {
-    (two<R, From + 2 * H>(w, un, open, lane), ...);
+    (two<R, From + 2 * H>(w, un, open, lane, half), ...);
 }
 
 // the same for class C, and its words with open evens into the queue (place:
@@ -167,8 +173,10 @@ __device__ __forceinline__ void one(const Words &w, bool inner, uint32_t taken, 
     if (slow >> C & 1u) return;
     uint32_t un = inner ? ~0u : 0u;
     if (lane == 0) atomicAdd(&sh.open[C][0], taken);
-    run<2 * C, 0>(w, un, sh.open[C], lane, std::make_index_sequence<kCkFew / 2>());
-    if (!few) run<2 * C, kCkFew>(w, un, sh.open[C], lane, std::make_index_sequence<(kCkFirst - kCkFew) / 2>());
+    const uint32_t half = lane ? 0x4432u : 0x4410u;
+    uint32_t *const open = sh.open[C] + (lane & 1u);
+    run<2 * C, 0>(w, un, open, lane, half, std::make_index_sequence<kCkFew / 2>());
+    if (!few) run<2 * C, kCkFew>(w, un, open, lane, half, std::make_index_sequence<(kCkFirst - kCkFew) / 2>());
     const uint32_t bal = __ballot_sync(~0u, un != 0);
     if (un) {
         const uint32_t at = qn + __popc(bal & ((1u << lane) - 1u));
@@ -376,7 +384,7 @@ __global__ void __launch_bounds__(kCkThreads, kCkCtas) k_check(BatchDesc d, Chec
             };
             // the item's first chunk in two parts: a few words, after which the
             // first candidates have been seen, then the others
-            const uint32_t jm = ch == c0 ? min(j0 + 4 * kCkWarps, j1) : j1;
+            const uint32_t jm = ch == c0 ? min(j0 + 3 * kCkWarps, j1) : j1;
             for (uint32_t part = 0, ja = j0, jb = jm; ja < jb; ++part, ja = jm, jb = part == 1 ? j1 : jm) {
                 if (part) {
                     __syncthreads();
