@@ -780,12 +780,22 @@ static void set_residues(gbk::BatchParams &bp)
     for (int j = 0; j < 8; ++j) bp.bres[j] = uint8_t(bp.base % f[j]);
 }
 
+// sieving primes of the integers up to qmax
+static uint32_t primes_to(const gbc_ctx *ctx, uint64_t qmax)
+{
+    const auto &pr = ctx->primes;
+    return uint32_t(std::upper_bound(pr.begin(), pr.end(), isqrt64(qmax)) - pr.begin());
+}
+
+// sieving primes past the tiles per integer of a run that is tested instead,
+// and the primes whose division takes as long as the tests' first results
+constexpr uint64_t kTestPrimes = 5, kTestSpare = 3'000'000;
+
 // One run (class map) of a batch: geometry, primes that reach it, and the
 // shared tables (the reference's segment_geometry / class_geometry,
 // src/host_math.cpp:13-78, for one map per run).
 static void plan_run(const gbc_ctx *ctx, gbk::BatchParams &bp, uint64_t s0, uint64_t sN)
 {
-    const auto &pr = ctx->primes;
     const uint64_t qlo = s0 > GBC_MAX_CAND + 30 ? s0 - GBC_MAX_CAND : 0;
     bp.base = qlo / 30 * 30;
     bp.qmax = sN + 3;
@@ -804,11 +814,24 @@ static void plan_run(const gbc_ctx *ctx, gbk::BatchParams &bp, uint64_t s0, uint
     bp.pk_gap = ctx->d_pk_gap;
     bp.pk_base = ctx->d_pk_base;
     bp.pk_i0 = ctx->n_mid;
-    const uint64_t root = isqrt64(bp.qmax);
-    bp.n_all = uint32_t(std::upper_bound(pr.begin(), pr.end(), root) - pr.begin());
+    bp.n_all = primes_to(ctx, bp.qmax);
     bp.i0 = std::min(ctx->i0, bp.n_all);
     bp.n_mid = std::max(std::min(ctx->n_mid, bp.n_all), bp.i0);
     bp.i_warp = std::min(std::max(ctx->i_warp, bp.i0), bp.n_mid);
+    // A narrow run: every prime past the tiles costs its division, the test of
+    // what the tiles leave goes with the width. Measured on one GB300, test
+    // against lists, ms: 16 runs a batch at 4e18 (98M primes) 2.39 and 4.61
+    // with 1e7 integers each, 6.54 and 5.90 with 3e7; at 1e17 (16M) .89 and
+    // .93 with 3e6. One run: at 4e18 .33 and .72 with 1e7, at 1e16 (5.6M) .143
+    // and .153 with 1e5, .187 and .173 with 1e6; at 1e15 (1.8M) .130 and .127
+    // with 1e4. (Not where the caller turned the hit lists on or off, nor in
+    // the plain form, whose tiles come segment by segment.)
+    const uint64_t past = bp.n_all - bp.n_mid;
+    if (ctx->cfg.hl_mode == 0 && ctx->cfg.launch_mode != 3 && bp.base >> 33 && past > kTestSpare &&
+        30ull * bp.nblk <= (past - kTestSpare) / kTestPrimes) {
+        bp.test = 1;
+        bp.n_all = bp.n_mid;
+    }
     bp.n_hl = ctx->hl_on ? std::min(std::max(ctx->n_hl, bp.n_mid), bp.n_all) : bp.n_all;
     set_residues(bp);
 }
@@ -825,8 +848,10 @@ static void finish_desc(const gbc_ctx *ctx, DescImage &img)
     h.n_hl_max = 0;
     h.n_hl_min = UINT32_MAX;
     h.n_all_max = 0;
+    uint64_t test_words = 0;
     for (uint32_t r = 0; r < nrun; ++r) {
         const gbk::BatchParams &bp = img.runs[r];
+        if (bp.test) test_words += 8 * ((bp.nblk + 31) / 32);
         img.tile_pref[r] = h.tile_items;
         h.tile_items += 8 * bp.tiles_pc;
         h.n_mid_max = std::max(h.n_mid_max, bp.n_mid);
@@ -836,6 +861,7 @@ static void finish_desc(const gbc_ctx *ctx, DescImage &img)
         h.n_all_max = std::max(h.n_all_max, bp.n_all);
     }
     img.tile_pref[nrun] = h.tile_items;
+    h.test_words = gbh::test_words(test_words, ctx->grids.sm);
     if (!nrun) h.n_mid_min = h.n_hl_min = 0;
     h.chk_vb = h.ver_vb = h.cnt_vb = h.nlow = 0;
     uint64_t words = 0, sampled_words = 0;  // class words of the segments, and of the exact checker's
@@ -1064,7 +1090,6 @@ static int ensure_mtab(gbc_ctx *ctx, uint64_t need0, uint64_t need1)
     CK(cudaMalloc(&tmp, size_t(8) * wpc * 4 + kMapPadBytes));
     CK(cudaMalloc(&xf, std::max<size_t>(size_t(8) * ctx->n_mid * 4, 4)));
     CK(cudaMalloc(&ddev, host.size()));
-    const auto &pr = ctx->primes;
     std::vector<gbk::BatchParams> runs(nchunk);
     for (uint64_t c = 0; c < nchunk; ++c) {
         DescImage img;
@@ -1090,8 +1115,7 @@ static int ensure_mtab(gbc_ctx *ctx, uint64_t need0, uint64_t need1)
         bb.pk_i0 = ctx->n_mid;
         bb.err = ctx->slot[0].err;
         bb.spin0 = gbk::kStageSpin;
-        const uint64_t root = isqrt64(bb.qmax);
-        bb.n_all = uint32_t(std::upper_bound(pr.begin(), pr.end(), root) - pr.begin());
+        bb.n_all = primes_to(ctx, bb.qmax);
         bb.i0 = std::min(ctx->i0, bb.n_all);
         bb.n_mid = std::max(std::min(ctx->n_mid, bb.n_all), bb.i0);
         bb.i_warp = std::min(std::max(ctx->i_warp, bb.i0), bb.n_mid);
@@ -1179,7 +1203,7 @@ static int issue_plain(gbc_ctx *ctx, Slot &s)
         gbh::launch_tile(d, ctx->gi, ctx->tile_bits, ctx->tile_stage, g, st);
         gbh::launch_large(d, g, st);
         gbh::launch_hitlist(d, true, g, st);
-        gbh::launch_hl_overflow(d, g, st);
+        gbh::launch_map_finish(d, g, st);
         gbh::launch_check(d, ctx->ct, g, st);
         gbh::launch_verify(d, ctx->vt, g, st);
         gbh::launch_tail(d, ctx->vt, g, st);
@@ -1214,7 +1238,7 @@ static int issue_pipeline(gbc_ctx *ctx, Slot &s, bool capture)
     gbh::launch_tile(d, ctx->gi, ctx->tile_bits, ctx->tile_stage, g, st);  // with the tile bins' marks
     gbh::launch_large(d, g, st);
     gbh::launch_hitlist(d, true, g, st);   // other batches: direct marks
-    gbh::launch_hl_overflow(d, g, st);
+    gbh::launch_map_finish(d, g, st);
     CK(cudaEventRecordWithFlags(s.ev[2], st, rec));
     gbh::launch_check(d, ctx->ct, g, st);
     gbh::launch_verify(d, ctx->vt, g, st);
@@ -1268,9 +1292,11 @@ static int issue_selfcheck(gbc_ctx *ctx, Slot &s)
     for (uint32_t r = 0; r < ci.h->nrun; ++r) {
         gbk::BatchParams &bp = ci.runs[r];
         bp.map = s.chk_map + (bp.map - s.map);
+        bp.n_all = primes_to(ctx, bp.qmax);  // a run whose rest was tested is sieved to the end here
         bp.n_hl = bp.n_all;
         bp.hl_quota = 0;
         bp.tb_cap = 0;
+        ci.h->n_all_max = std::max(ci.h->n_all_max, bp.n_all);
     }
     ci.h->n_hl_max = ci.h->n_all_max;
     ci.h->n_hl_min = ci.h->n_all_max;
@@ -1316,7 +1342,7 @@ static int enqueue_planned(gbc_ctx *ctx, Slot &s)
     }
     ctx->launches += kPipelineKernels;
     s.did_selfcheck = false;
-    if (hl) {
+    if (hl || img.h->test_words) {
         ctx->hl_batches += 1;
         const uint32_t every = ctx->cfg.selfcheck_every;
         if (every && ctx->hl_batches % every == 0) {

@@ -121,6 +121,7 @@ struct BatchParams {
     uint2 *ovf_buf;           // (class, virtual bit) of each overflow mark
     uint32_t *ovf_cnt;
     uint32_t spin0;           // try_wait rounds of the first wait on a tile bin's bulk copies (kStageSpin)
+    uint32_t test;            // 1: no prime past the tiles' sieves the run, what they leave is tested one by one
 };
 
 // t / tile_bits for t < 2^31 (the estimate umulhi(t, rcp) is exact or one
@@ -201,7 +202,7 @@ struct BatchHeader {
     // and limits
     uint32_t seg0;
     uint32_t win_b0, win_b1;
-    uint32_t pad;
+    uint32_t test_words;           // class words a warp tests at a time (runs with BatchParams::test; 0: none)
     // work counters of the persistent kernels (CTAs take their next item
     // with an atomic add); zero in the host image, so every batch's
     // descriptor copy resets them
@@ -481,7 +482,9 @@ void launch_large(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st);
 // marks of every other batch (after the tiles)
 void launch_hitlist(const gbk::BatchDesc &d, bool direct, const Grids &g, cudaStream_t st);
 void launch_binsort(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st);
-void launch_hl_overflow(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st);
+// after the tiles: the overflow marks, the narrow runs' primality tests
+uint32_t test_words(uint64_t words, int sm);
+void launch_map_finish(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st);
 void query_sieve_grids(Grids &g);
 void launch_check(const gbk::BatchDesc &d, const gbk::CheckTables &ct, const Grids &g, cudaStream_t st);
 void launch_verify(const gbk::BatchDesc &d, const gbk::VerifyTables &vt, const Grids &g, cudaStream_t st);

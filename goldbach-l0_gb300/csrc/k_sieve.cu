@@ -1049,10 +1049,8 @@ __global__ void __launch_bounds__(256, 6) k_binsort(BatchDesc d)
 }
 
 // The overflow list of a binned batch, cleared after the tiles.
-__global__ void __launch_bounds__(256) k_hl_overflow(BatchDesc d)
+__device__ __forceinline__ void overflow_marks(const BatchDesc &d, uint32_t nrun)
 {
-    const uint32_t nrun = d.h->nrun;
-    if (!nrun || !hl_binned(d.runs[0])) return;
     const BatchParams &bp0 = d.runs[0];
     const uint32_t cnt = *bp0.ovf_cnt, tb = bp0.tile_bits;
     if (cnt > bp0.ovf_cap && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(bp0.err, kErrHlOverflow);
@@ -1073,6 +1071,211 @@ __global__ void __launch_bounds__(256) k_hl_overflow(BatchDesc d)
         if (t < bp.nblk && t >= b0 && t < b1)
             atomicAnd(bp.map + size_t(e.x) * bp.wpc + (t >> 5), ~(1u << (t & 31)));
     }
+}
+
+// The primality test of one odd n, 2^33 < n < 2^64, without a prime factor
+// below 128 (Baillie and Wagstaff, Mathematics of Computation 35, 1980): a
+// strong probable prime to base 2, then an extra strong Lucas probable prime
+// (Grantham, Mathematics of Computation 70, 2001; the first P from 3 on whose
+// P^2 - 4 has Jacobi symbol -1, Q = 1). No composite below 2^64 is both: every
+// base-2 pseudoprime of J. Feitsma's complete list fails the second. A square
+// ends at base 2 (of a prime: only 1093^2 and 3511^2 pass, both below 2^33),
+// so a P exists. Numbers are in Montgomery form, x 2^64 mod n.
+struct Bpsw {
+    uint64_t n, ninv, one;
+    __device__ __forceinline__ explicit Bpsw(uint64_t q) : n(q)
+    {
+        ninv = n;  // n^-1 mod 2^64 (Newton: correct bits 3, 6, 12, ...)
+#pragma unroll
+        for (int i = 0; i < 5; ++i) ninv *= 2 - n * ninv;
+        one = (0 - n) % n;  // 2^64 mod n
+    }
+    __device__ __forceinline__ uint64_t sub(uint64_t x, uint64_t y) const { return x >= y ? x - y : x - y + n; }
+    __device__ __forceinline__ uint64_t twice(uint64_t x) const { return sub(x, n - x); }
+    // x y / 2^64: the product less the multiple of n with the same low half
+    __device__ __forceinline__ uint64_t mul(uint64_t x, uint64_t y) const
+    {
+        return sub(__umul64hi(x, y), __umul64hi(x * y * ninv, n));
+    }
+
+    // 2^d = 1, or 2^(d 2^r) = -1 for an r < s (n - 1 = d 2^s, d odd)
+    __device__ __forceinline__ bool base2() const
+    {
+        const int s = __ffsll(static_cast<long long>(n - 1)) - 1;
+        const uint64_t d = (n - 1) >> s, minus = n - one;
+        uint64_t x = twice(one);
+#pragma unroll 1
+        for (int b = 62 - __clzll(static_cast<long long>(d)); b >= 0; --b) {
+            x = mul(x, x);
+            if (d >> b & 1) x = twice(x);
+        }
+        bool ok = x == one || x == minus;
+        for (int r = 1; r < s && !ok; ++r) {
+            x = mul(x, x);
+            ok = x == minus;
+        }
+        return ok;
+    }
+
+    // The Jacobi symbol (a | n) is -1; 0 < a < 2^31 without a common factor with n.
+    __device__ __noinline__ static bool jacobi_minus(uint32_t a, uint64_t n)
+    {
+        bool neg = false;
+        const int z = __ffs(a) - 1;
+        if (z & 1) neg ^= (n & 7) == 3 || (n & 7) == 5;
+        a >>= z;
+        neg ^= (a & n & 3) == 3;
+        uint32_t m = a;  // (n mod m | m)
+        a = uint32_t(n % m);
+        while (a) {
+            const int y = __ffs(a) - 1;
+            if (y & 1) neg ^= (m & 7) == 3 || (m & 7) == 5;
+            a >>= y;
+            neg ^= (a & m & 3) == 3;
+            const uint32_t t = m % a;
+            m = a;
+            a = t;
+        }
+        return neg;
+    }
+
+    // The first P: the symbols of the primes up to 23 as a sign per k <= 24
+    // give those of (P - 2)(P + 2) up to P = 22; one n in a thousand or so
+    // needs more.
+    template <uint32_t F>
+    __device__ __forceinline__ static uint32_t signs(uint32_t r, uint64_t n)
+    {
+        constexpr uint32_t non = [] {
+            uint32_t m = 0;
+            for (uint32_t x = 1; x < F; ++x) m |= 1u << x;
+            for (uint32_t x = 1; x < F; ++x) m &= ~(1u << (x * x % F));
+            return m;
+        }();
+        constexpr uint32_t odd = [] {  // bit k: F divides k an odd number of times
+            uint32_t m = 0;
+            for (uint32_t k = F; k <= 24; ++k) {
+                uint32_t v = 0, x = k;
+                for (; x % F == 0; x /= F) ++v;
+                m |= (v & 1u) << k;
+            }
+            return m;
+        }();
+        bool neg = non >> (r % F) & 1u;
+        if ((F & 3) == 3) neg ^= (n & 3) == 3;
+        return neg ? odd : 0u;
+    }
+    __device__ __forceinline__ uint32_t lucas_p() const
+    {
+        const uint32_t r = uint32_t(n % (3u * 5 * 7 * 11 * 13 * 17 * 19 * 23));
+        uint32_t k = signs<3>(r, n) ^ signs<5>(r, n) ^ signs<7>(r, n) ^ signs<11>(r, n) ^ signs<13>(r, n) ^
+                     signs<17>(r, n) ^ signs<19>(r, n) ^ signs<23>(r, n);
+        if ((n & 7) == 3 || (n & 7) == 5) k ^= 1u << 2 | 1u << 6 | 1u << 8 | 1u << 10 | 1u << 14 | 1u << 18 | 1u << 22 | 1u << 24;
+        const uint32_t p = (k ^ k >> 4) & 0x1FFFFEu;  // bit P - 2
+        if (p) return uint32_t(__ffs(p)) + 1u;
+        uint32_t x = 23;
+        while (x < 30000 && !jacobi_minus(x * x - 4, n)) ++x;
+        return x;
+    }
+
+    // V_d = 2 and U_d = 0 (then V_(d+1) = P), the same with both signs turned,
+    // or V_(d 2^r) = 0 for an r < s - 1 (n + 1 = d 2^s, d odd)
+    __device__ __forceinline__ bool lucas() const
+    {
+        const uint32_t p = lucas_p();
+        uint64_t pm = 0;
+#pragma unroll 1
+        for (int b = 31 - __clz(p); b >= 0; --b) {
+            pm = twice(pm);
+            if (p >> b & 1) pm = sub(pm, n - one);
+        }
+        const int s = __ffsll(static_cast<long long>(n + 1)) - 1;
+        const uint64_t d = (n + 1) >> s, two = twice(one);
+        uint64_t v = pm, w = sub(mul(pm, pm), two);  // V_1, V_2
+#pragma unroll 1
+        for (int b = 62 - __clzll(static_cast<long long>(d)); b >= 0; --b) {
+            const bool up = d >> b & 1;
+            const uint64_t x = sub(mul(v, w), pm), y = up ? w : v, y2 = sub(mul(y, y), two);
+            v = up ? x : y2;
+            w = up ? y2 : x;
+        }
+        bool ok = v == 0 || (v == two && w == pm) || (v == n - two && w == n - pm);
+        for (int r = 1; r < s - 1 && !ok; ++r) {
+            v = sub(mul(v, v), two);
+            ok = v == 0;
+        }
+        return ok;
+    }
+};
+
+// Narrow runs (BatchParams::test): what the tiles leave has no factor up to
+// p_mid, one integer in 25 or so, and each is settled by its own primality
+// test instead of every larger sieving prime being divided into the run. A
+// warp takes test_words words of a class array: their bits to a list, base 2
+// for all, the Lucas test for those that pass (three in five, nearly all of
+// them prime), 32 numbers at a time. Bound by the integer multipliers (11 of a
+// product's 22 instructions, wide ones at a quarter of the issue rate): 13 ps
+// an integer of the run at 4e18, where Miller-Rabin to seven bases takes 51.
+// From kTestMinWords on a warp's first list has about 32 numbers: 16 runs of
+// 1e4 integers at 4e18 take .23 ms with 6 words at least, .25 with 1 (2.59
+// through the hit lists).
+constexpr uint32_t kTestWords = 32, kTestMinWords = 6;
+constexpr int kTestThreads = 128, kTestCtas = 8;
+
+__device__ __forceinline__ void test_runs(const BatchDesc &d, uint32_t nrun)
+{
+    __shared__ uint16_t s_list[kTestThreads / 32][32 * kTestWords];
+    const uint32_t lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5), tw = d.h->test_words;
+    uint16_t *const list = s_list[threadIdx.x >> 5];
+    uint32_t task = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    for (uint32_t r = 0; r < nrun; ++r) {
+        const BatchParams &bp = d.runs[r];
+        if (!bp.test) continue;
+        const uint32_t nw = (bp.nblk + 31) / 32, per = (nw + tw - 1) / tw, tasks = 8 * per;
+        for (; task < tasks; task += warps) {
+            const uint32_t k = task / per, w0 = (task - k * per) * tw;
+            uint32_t *const words = bp.map + size_t(k) * bp.wpc + w0;
+            uint32_t v = lane < tw && w0 + lane < nw ? words[lane] : 0u;
+            if (w0 + lane + 1 == nw && (bp.nblk & 31u)) v &= (1u << (bp.nblk & 31u)) - 1u;
+            uint32_t at = __popc(v);
+#pragma unroll
+            for (uint32_t o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(~0u, at, o);
+                if (lane >= o) at += y;
+            }
+            uint32_t n = __shfl_sync(~0u, at, 31);
+            at -= __popc(v);
+            for (; v; v &= v - 1u) list[at++] = uint16_t(32 * lane + __ffs(v) - 1u);
+            __syncwarp();
+            const uint64_t q0 = bp.base + 30ull * 32 * w0 + unit30(k);
+            for (uint32_t pass = 0; pass < 2; ++pass) {
+                uint32_t kept = 0;
+                for (uint32_t i = lane; i - lane < n; i += 32) {
+                    const uint32_t bit = list[i < n ? i : 0u];
+                    bool prime = false;
+                    if (i < n) {
+                        const Bpsw t(q0 + 30ull * bit);
+                        prime = pass ? t.lucas() : t.base2();
+                        if (!prime) atomicAnd(words + (bit >> 5), ~(1u << (bit & 31u)));
+                    }
+                    const uint32_t bal = __ballot_sync(~0u, prime);
+                    if (prime) list[kept + __popc(bal & ((1u << lane) - 1u))] = uint16_t(bit);
+                    kept += __popc(bal);
+                    __syncwarp();
+                }
+                n = kept;
+            }
+        }
+        task -= tasks;  // the next run's tasks go on from here
+    }
+}
+
+// After the tiles: the overflow marks of a binned batch, and the narrow runs' tests.
+__global__ void __launch_bounds__(kTestThreads) k_map_finish(BatchDesc d)
+{
+    const uint32_t nrun = d.h->nrun;
+    if (!nrun) return;
+    if (hl_binned(d.runs[0])) overflow_marks(d, nrun);
+    if (d.h->test_words) test_runs(d, nrun);
 }
 
 // The class arrays of a sieved range, rewritten as one byte per block of 30
@@ -1202,9 +1405,16 @@ void launch_binsort(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st)
     gbk::k_binsort<<<g.sm * 6, 256, 0, st>>>(d);
 }
 
-void launch_hl_overflow(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st)
+uint32_t test_words(uint64_t words, int sm)
 {
-    gbk::k_hl_overflow<<<g.sm * 2, 256, 0, st>>>(d);
+    const uint64_t warps = uint64_t(sm) * gbk::kTestCtas * (gbk::kTestThreads / 32);
+    const uint64_t share = std::max<uint64_t>((words + warps - 1) / warps, gbk::kTestMinWords);
+    return words ? uint32_t(std::min<uint64_t>(share, gbk::kTestWords)) : 0u;
+}
+
+void launch_map_finish(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st)
+{
+    gbk::k_map_finish<<<g.sm * gbk::kTestCtas, gbk::kTestThreads, 0, st>>>(d);
 }
 
 void launch_xfirst1(const gbk::BatchParams &bp, cudaStream_t st)

@@ -72,7 +72,8 @@ typedef struct gbc_config {
                                 with one class map; windows that do not touch are separate runs);
                                 default max_batch, at most max_batch */
     uint32_t hl_mode;        /* prime-multiplier hit lists: 0 auto (on when a batch spans >= 1e9
-                                integers), 1 on, 2 off */
+                                integers; a run narrow for its height is finished by primality
+                                tests instead), 1 on, 2 off */
     uint32_t mtab_max_gb;    /* HBM budget of the prime-multiplier table (default 48 GB); primes below
                                 limit / (30 * budget) keep the read-before-mark kernel */
     uint32_t nslots;         /* independent slots (default 2, 2..GBC_MAX_SLOTS) */
@@ -95,8 +96,8 @@ typedef struct gbc_config {
                                 pipeline, src/verifier.cpp:2487-2517): a batch's hit lists harvested
                                 once, then each segment by its own launches of the sieve, large-prime,
                                 checker and count kernels (batches of several runs: as 2) */
-    uint32_t selfcheck_every;/* every selfcheck_every-th batch that uses hit lists rebuilds its maps
-                                without them and compares every word (src/verifier.cpp:2057-2112);
+    uint32_t selfcheck_every;/* every selfcheck_every-th batch that uses hit lists (or the primality
+                                tests of hl_mode 0) rebuilds its maps without them and compares every word (src/verifier.cpp:2057-2112);
                                 a mismatch fails the batch closed. 0: never (default) */
     uint32_t verify_funnels; /* accepted and reported for callers that set it (default 3; at most
                                 plan_funnels): the verify kernel takes three funnels of every class
