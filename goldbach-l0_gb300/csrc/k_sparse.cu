@@ -20,17 +20,18 @@
 //   k_sp_large  a thread per prime from 2^20: its twelve first bits, each mark
 //               a read of the word and an atomic AND only where the bit is set
 //   k_sp_popc   set bits of the map
-//   k_sp_check  persistent CTAs over (chunk of 4096 evens per class, block of
-//               1024 even classes) items; each item's twelve row windows are
-//               staged in shared memory by bulk copies (two buffers: the next
-//               item's copies land while this one is checked); a warp takes an
-//               even class, each lane four words of its evens, and ORs in the
-//               entries (class, window word, up to six packed offsets) of the
-//               plan's first three groups; the evens still open, about one in
-//               a hundred, are then taken one per lane, a group as one 32-bit window
-//               of its row ANDed with the group's candidates; evens no group
-//               verifies go to the pending list, which the host resolves by an
-//               ascending Miller-Rabin scan.
+//   k_sp_pattern  rows that hold the OR of a map row's bits at a few offsets
+//   k_sp_check  persistent CTAs over (chunk of 8192 evens per class, block of
+//               even classes) items; each item's row windows are staged in
+//               shared memory by bulk copies (two buffers: the next item's
+//               copies land while this one is checked); a warp takes an even
+//               class, each lane eight words of its evens, and ORs in the
+//               shifts of map and pattern rows that test the plan's first two
+//               groups; the evens still open, about one in 25, are then taken
+//               one per lane, a group as one 32-bit window of its row ANDed
+//               with the group's candidates; evens no group verifies go to
+//               the pending list, which the host resolves by an ascending
+//               Miller-Rabin scan.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -52,16 +53,31 @@ constexpr uint32_t kM = 30030, kHalfM = 15015, kK = 12;
 constexpr uint32_t kTileLog2 = 20, kTileBits = 1u << kTileLog2, kTileWords = kTileBits / 32;
 constexpr uint32_t kSplit = 1u << 20;        // sieving primes below: tiles; from: k_sp_large
 constexpr uint32_t kWarpPrime = 1024;        // below: a warp per prime in the tile
-constexpr uint32_t kV = 4;                   // words per lane in the checker
+constexpr uint32_t kV = 8;                   // words per lane in the checker
 constexpr uint32_t kChunkWords = 32 * kV;    // words (of evens) per class and checker item
 constexpr uint32_t kChunkEvens = 32 * kChunkWords;
-constexpr uint32_t kCheckWarps = 8, kCheckThreads = 32 * kCheckWarps;
-constexpr uint32_t kClassBlock = 128 * kCheckWarps;  // even classes per checker item
-constexpr uint32_t kClassBlocks = (kHalfM + kClassBlock - 1) / kClassBlock;
+constexpr uint32_t kCheckWarps = 32, kCheckThreads = 32 * kCheckWarps;
+constexpr uint32_t kMinBlock = 4 * kCheckWarps, kMaxBlock = 32 * kCheckWarps;  // even classes per checker item
 constexpr uint32_t kPendCap = 1u << 20;      // pending words per segment
 constexpr uint32_t kErrStaging = 1u << 0;    // a bulk copy missed its wait limit
 constexpr uint32_t kEntryMax = 6;            // candidates per plan entry
-constexpr uint32_t kWordGroups = 3;          // plan groups every word takes before its open evens
+constexpr uint32_t kWordGroups = 2;          // plan groups every word takes before its open evens
+
+constexpr uint32_t kMaskEnd = 1u << 31;      // a class's masks end here
+
+// shared memory for the checker's staged rows, beside its queues (40 KB)
+constexpr uint32_t kCheckWindows = 184 * 1024;
+
+// Pattern rows: row k of pattern g has bit t set where row k of the map has
+// any of the bits t + x, x in the pattern. One funnel shift of a pattern row
+// then tests all of the pattern's candidates. The sets are those that cover
+// the groups of the first four offsets a candidate at a time cheapest, found
+// one after the other among pairs, triples, quadruples and quintuples.
+constexpr uint32_t kPatterns = 4;
+__host__ __device__ constexpr uint32_t pattern(uint32_t g)
+{
+    return g == 0 ? 0x3u : g == 1 ? 0x29u : g == 2 ? 0x13u : 0x205u;
+}
 
 // A plan entry: up to six candidates of one class k and one window word o,
 // as x = k | o << 4 | count << 12 and y = their offsets within the word, 5
@@ -94,6 +110,8 @@ struct SpSeg {
     uint32_t dl, T, tb;       // evens per class; map bits per row (dl + TB); TB
     uint32_t tiles, chunks;   // tiles per row; checker chunks
     uint32_t stride, rw;      // words per map row; staged words per row and item
+    uint32_t rows;            // rows of the map and its patterns
+    uint32_t block, blocks;   // even classes per checker item, and items per chunk
     uint32_t group_cap;       // plan entries per class (all: ~0)
     uint32_t *map;
     SpCtr *ctr;
@@ -210,35 +228,59 @@ __global__ void __launch_bounds__(256) k_sp_popc(SpSeg s)
 // bits [0, x) of a word, x <= 32
 __device__ __forceinline__ uint32_t low_bits(uint32_t x) { return x >= 32 ? ~0u : (1u << x) - 1u; }
 
-// the twelve row windows of chunk c into buf: row k's words [c W, c W + rw)
+// the pattern rows of the map's words
+__global__ void __launch_bounds__(256) k_sp_pattern(SpSeg s)
+{
+    const uint64_t words = uint64_t(s.tiles) * kTileWords;
+    const uint32_t k = blockIdx.y;
+    const uint32_t *src = s.map + size_t(k) * s.stride;
+    for (uint64_t w = blockIdx.x * blockDim.x + threadIdx.x; w < words; w += uint64_t(gridDim.x) * blockDim.x) {
+        const uint32_t a = src[w], b = w + 1 < words ? src[w + 1] : 0u;
+#pragma unroll
+        for (uint32_t g = 0; g < kPatterns; ++g) {
+            if (kK * (g + 2) > s.rows) break;
+            uint32_t v = 0;
+#pragma unroll
+            for (uint32_t x = 0; x < 32; ++x)
+                if (pattern(g) >> x & 1u) v |= __funnelshift_r(a, b, x);
+            s.map[size_t(kK * (g + 1) + k) * s.stride + w] = v;
+        }
+    }
+}
+
+// the row windows of chunk c into buf: row k's words [c W, c W + rw)
 __device__ __forceinline__ void sp_stage(const SpSeg &s, uint32_t *buf, uint64_t *bar, uint32_t c)
 {
     gbk::fence_proxy_async();
-    gbk::mbar_arrive_expect_tx(bar, kK * s.rw * 4);
+    gbk::mbar_arrive_expect_tx(bar, s.rows * s.rw * 4);
 #pragma unroll 1
-    for (uint32_t k = 0; k < kK; ++k)
+    for (uint32_t k = 0; k < s.rows; ++k)
         gbk::bulk_copy_g2s(buf + k * s.rw, s.map + size_t(k) * s.stride + size_t(c) * kChunkWords, s.rw * 4, bar);
 }
 
 // The word form costs a word of 32 evens a funnel shift and half a three-input
-// OR per candidate, however many of its evens are open; the even form about 35
-// instructions for the 10 to 17 candidates of a group. An even is verified by
-// a candidate with probability 0.12 at 4e18, so after the 50 or so candidates
-// of the three fullest groups the even form is the cheaper one. With a
-// group_cap every word takes the capped entries, word by word.
-// Bound by the ALU pipe (83%). One GB300, 1.05e12 evens at 4e18: 244.0 ms
-// (two groups word by word: 251.7) against 321.6 for entries word by word
-// until every even of 4096 was verified.
-__global__ void __launch_bounds__(kCheckThreads, 4) k_sp_check(SpSeg s, const uint2 *groups, const uint32_t *goff,
-                                                            const uint2 *masks, const uint2 *cls, uint4 *pend)
+// OR per shift, however many of its evens are open; a shift of a pattern row
+// tests two or three candidates, so the 15 of a full group take 9 instead of
+// 15. The even form is about 35 instructions for the 10 to 15 candidates of a
+// group, with every lane at work: a lane keeps its word over the end of a
+// class. An even is verified by a candidate with probability 0.12 at 4e18:
+// about one in 25 is open after the two fullest groups. One CTA an SM, since
+// two buffers of 60 row windows take 144 KB.
+// Bound by the ALU pipe (75%) and issue (78%). One GB300, 1.05e12 evens at
+// 4e18: 125.1 ms (three groups word by word: 129.6; 3 patterns 147.3, 4 145.3,
+// 5 144.5, when the even form still began anew with each class; map rows only
+// and four words a lane: 244.0; entries word by word until every even of 4096
+// was verified: 321.6).
+__global__ void __launch_bounds__(kCheckThreads, 1) k_sp_check(SpSeg s, const uint2 *entries, const uint2 *masks,
+                                                            const uint4 *cls, uint4 *pend)
 {
-    extern __shared__ __align__(16) uint32_t win[];  // two buffers of kK * rw words
+    extern __shared__ __align__(16) uint32_t win[];  // two buffers of rows * rw words
     __shared__ uint32_t s_qbits[kCheckWarps][kChunkWords];  // a task's words with open evens: their bits
     __shared__ uint8_t s_qword[kCheckWarps][kChunkWords];   // and which word
     __shared__ uint64_t s_bar[2];
     __shared__ uint32_t s_j[2];  // alternate: no barrier separates two item fetches
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t items = s.chunks * kClassBlocks;
+    const uint32_t items = s.chunks * s.blocks;
     if (tid == 0) {
         gbk::mbar_init(&s_bar[0], 1);
         gbk::mbar_init(&s_bar[1], 1);
@@ -246,25 +288,24 @@ __global__ void __launch_bounds__(kCheckThreads, 4) k_sp_check(SpSeg s, const ui
     }
     uint32_t phase = 0, buf = 0;
     unsigned long long ngroups = 0, nevens = 0;
-    const bool capped = s.group_cap != ~0u;
     uint32_t *const q_bits = s_qbits[warp];
     uint8_t *const q_word = s_qword[warp];
     uint32_t j = gbk::next_item(&s.ctr->work_check, &s_j[0]);
-    if (j < items && tid == 0) sp_stage(s, win, &s_bar[0], j / kClassBlocks);
+    if (j < items && tid == 0) sp_stage(s, win, &s_bar[0], j / s.blocks);
     while (j < items) {
         // the next item's copies go into the other buffer, free since the
         // synchronization inside next_item
         const uint32_t jn = gbk::next_item(&s.ctr->work_check, &s_j[buf ^ 1u]);
-        if (jn < items && tid == 0) sp_stage(s, win + (buf ^ 1u) * kK * s.rw, &s_bar[buf ^ 1u], jn / kClassBlocks);
+        if (jn < items && tid == 0) sp_stage(s, win + (buf ^ 1u) * s.rows * s.rw, &s_bar[buf ^ 1u], jn / s.blocks);
         bool ok = gbk::mbar_wait(&s_bar[buf], (phase >> buf) & 1u);
         if (!ok) {
             atomicOr(&s.ctr->err, kErrStaging);
             ok = gbk::mbar_wait(&s_bar[buf], (phase >> buf) & 1u);
         }
         phase ^= 1u << buf;
-        const uint32_t c = j / kClassBlocks, cb = j - c * kClassBlocks;
-        const uint32_t *w0 = win + buf * kK * s.rw;
-        const uint32_t cr1 = min(kHalfM, (cb + 1) * kClassBlock);
+        const uint32_t c = j / s.blocks, cb = j - c * s.blocks;
+        const uint32_t *w0 = win + buf * s.rows * s.rw;
+        const uint32_t cr1 = min(kHalfM, (cb + 1) * s.block);
         // a chunk inside [start, limit] for every even class needs no
         // per-class range: the latest first even is class 0's, the earliest
         // last even class M - 2's
@@ -273,20 +314,38 @@ __global__ void __launch_bounds__(kCheckThreads, 4) k_sp_check(SpSeg s, const ui
         const uint64_t top = s.N + kM - 2;
         const uint64_t ihi_min = s.limit >= top ? min(uint64_t(s.dl), (s.limit - top) / kM + 1) : 0;
         const bool interior = ilo_max <= ci0 && ihi_min >= ci0 + kChunkEvens;
-        for (uint32_t q0 = cb * kClassBlock + warp; ok && q0 < cr1; q0 += 32 * kCheckWarps) {
-            // the group ranges of the warp's next 32 classes, one per lane
-            const uint32_t mine = q0 + lane * kCheckWarps;
-            uint32_t lg0 = 0, lg1 = 0;
-            uint2 lcls = make_uint2(0u, 0u);
-            if (mine < cr1) {
-                lg0 = __ldg(goff + mine);
-                lcls = __ldg(cls + mine);
-                lg1 = capped ? lg0 + min(__ldg(goff + mine + 1) - lg0, s.group_cap) : lg0 + (lcls.y >> 16);
+        // a lane's word of open evens: the next group's mask, the class's first
+        struct {
+            uint32_t m = 0, rest = 0, word = 0, at = 0, first = 0, cr = 0;
+        } ev;
+        auto step = [&] {
+            const uint2 e = __ldg(masks + ev.at);  // with kMaskEnd: every group tried (rare)
+            const uint32_t b = 31u - __clz(ev.m | 1u);
+            const uint32_t *row = w0 + (e.x & 0xFFFFu) + ev.word;
+            const bool hit = ((__funnelshift_r(row[0], row[1], b) & e.y) | (e.x & kMaskEnd)) != 0;
+            ++ev.at;
+            if (hit) {
+                const uint32_t bit = ev.m & (1u << b);
+                if (e.x & kMaskEnd) ev.rest |= bit;
+                ev.m ^= bit;
+                ev.at = ev.first;
+                if (ev.m == 0 && ev.rest) {
+                    const uint32_t slot = atomicAdd(&s.ctr->npend, 1u);
+                    if (slot < kPendCap) pend[slot] = make_uint4(ev.cr, c * kChunkWords + ev.word, ev.rest, 0u);
+                    ev.rest = 0;
+                }
             }
+            if (ev.m == 0) ev.at = ev.first;
+            __syncwarp();
+        };
+        for (uint32_t q0 = cb * s.block + warp; ok && q0 < cr1; q0 += 32 * kCheckWarps) {
+            // the plans of the warp's next classes, one per lane
+            const uint32_t mine = q0 + lane * kCheckWarps;
+            const uint4 lcls = mine < cr1 ? __ldg(cls + mine) : make_uint4(0u, 0u, 0u, 0u);
             const uint32_t nt = min(32u, (cr1 - q0 + kCheckWarps - 1) / kCheckWarps);
             for (uint32_t tj = 0; tj < nt; ++tj) {
                 const uint32_t cr = q0 + tj * kCheckWarps;
-                const uint32_t g0 = __shfl_sync(~0u, lg0, tj), g1 = __shfl_sync(~0u, lg1, tj);
+                const uint32_t g0 = __shfl_sync(~0u, lcls.x, tj), ng = __shfl_sync(~0u, lcls.y, tj);
                 uint32_t f[kV];
                 if (interior) {
 #pragma unroll
@@ -313,60 +372,29 @@ __global__ void __launch_bounds__(kCheckThreads, 4) k_sp_check(SpSeg s, const ui
                     }
                     if (__all_sync(~0u, all == ~0u)) continue;
                 }
-                // the groups in plan order, 32 entries per coalesced load
-                uint32_t g = g0, head = ~0u, a[kV] = {}, b[kV] = {};
-                bool done = false;
-                while (!done && g < g1) {
-                    const uint32_t ng = min(32u, g1 - g);
-                    uint2 le = make_uint2(0u, 0u);
-                    if (lane < ng) le = __ldg(groups + g + lane);
-                    uint32_t u = 0;
-                    while (u < ng) {
-                        const uint32_t ex = __shfl_sync(~0u, le.x, u), ey = __shfl_sync(~0u, le.y, u);
-                        ++u;
-                        // a group's entries share their window
-                        if ((ex & 0xFFFu) != head) {
-                            head = ex & 0xFFFu;
-                            const uint32_t *row = w0 + entry_k(ex) * s.rw + entry_o(ex) + lane;
+                // word by word: the first groups' entries, one per lane
+                const uint2 le = lane < ng ? __ldg(entries + g0 + lane) : make_uint2(0u, 0u);
+                ngroups += __shfl_sync(~0u, lcls.w, tj);
+                for (uint32_t u = 0; u < ng; ++u) {
+                    const uint32_t ex = __shfl_sync(~0u, le.x, u);
+                    uint32_t y = __shfl_sync(~0u, le.y, u);
+                    const uint32_t *row = w0 + (ex & 0xFFFFu) + lane;
+                    uint32_t a[kV], b[kV];
 #pragma unroll
-                            for (uint32_t v = 0; v < kV; ++v) {
-                                a[v] = row[32 * v];
-                                b[v] = row[32 * v + 1];
-                            }
-                        }
-                        // two candidates per step
-                        const uint32_t np = (entry_n(ex) + 1) >> 1;
-                        uint32_t y = ey;
-#pragma unroll
-                        for (uint32_t jp = 0; jp < (kEntryMax + 1) / 2; ++jp)
-                            if (jp < np) {
-                                const uint32_t y2 = y >> 5;
-#pragma unroll
-                                for (uint32_t v = 0; v < kV; ++v)
-                                    f[v] |= __funnelshift_r(a[v], b[v], y) | __funnelshift_r(a[v], b[v], y2);
-                                y >>= 10;
-                            }
-                        if (!capped) continue;
-                        uint32_t all = f[0];
-#pragma unroll
-                        for (uint32_t v = 1; v < kV; ++v) all &= f[v];
-                        if (__all_sync(~0u, all == ~0u)) {
-                            done = true;
-                            break;
-                        }
+                    for (uint32_t v = 0; v < kV; ++v) {
+                        a[v] = row[32 * v];
+                        b[v] = row[32 * v + 1];
                     }
-                    g += u;
-                }
-                ngroups += g - g0;
-                auto leave = [&](uint32_t word, uint32_t bits) {
-                    const uint32_t slot = atomicAdd(&s.ctr->npend, 1u);
-                    if (slot < kPendCap) pend[slot] = make_uint4(cr, c * kChunkWords + word, bits, 0u);
-                };
-                if (capped) {
+                    // two shifts per step
 #pragma unroll
-                    for (uint32_t v = 0; v < kV; ++v)
-                        if (f[v] != ~0u) leave(32 * v + lane, ~f[v]);
-                    continue;
+                    for (uint32_t jp = 0; jp < kEntryMax / 2; ++jp)
+                        if (jp < ex >> 16) {
+                            const uint32_t y2 = y >> 5;
+#pragma unroll
+                            for (uint32_t v = 0; v < kV; ++v)
+                                f[v] |= __funnelshift_r(a[v], b[v], y) | __funnelshift_r(a[v], b[v], y2);
+                            y >>= 10;
+                        }
                 }
                 // the words with open evens into the queue
                 uint32_t qn = 0;
@@ -381,42 +409,26 @@ __global__ void __launch_bounds__(kCheckThreads, 4) k_sp_check(SpSeg s, const ui
                     qn += __popc(bal);
                 }
                 __syncwarp();
-                // even by even: a lane takes a word, then the queue's last one;
-                // the class's next 32 groups one per lane
-                const uint32_t m0 = __shfl_sync(~0u, lcls.x, tj), mn = __shfl_sync(~0u, lcls.y, tj) & 0xFFFFu;
-                const uint2 lm = lane < mn ? __ldg(masks + m0 + lane) : make_uint2(0u, 0u);
-                uint32_t m = 0, word = 0, h = 0;
-                for (;;) {
-                    const uint32_t idle = __ballot_sync(~0u, m == 0);
-                    if (qn) {
-                        const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
-                        if (m == 0 && rank < qn) {
-                            m = q_bits[qn - 1 - rank];
-                            word = q_word[qn - 1 - rank];
-                        }
-                        qn -= min(qn, uint32_t(__popc(idle)));
-                    } else if (idle == ~0u) {
-                        break;
+                // even by even, as long as no lane is idle: an idle lane takes
+                // the queue's last word, what lanes hold at the queue's end
+                // goes on beside the next class's words
+                const uint32_t m0 = __shfl_sync(~0u, lcls.z, tj);
+                while (qn) {
+                    const uint32_t idle = __ballot_sync(~0u, ev.m == 0);
+                    const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
+                    if (ev.m == 0 && rank < qn) {
+                        ev.m = q_bits[qn - 1 - rank];
+                        ev.word = q_word[qn - 1 - rank];
+                        ev.at = m0;
+                        ev.first = m0;
+                        ev.cr = cr;
                     }
-                    uint2 e;
-                    e.x = __shfl_sync(~0u, lm.x, h & 31u);
-                    e.y = __shfl_sync(~0u, lm.y, h & 31u);
-                    if (h >= 32) e = h < mn ? __ldg(masks + m0 + h) : make_uint2(0u, 0u);
-                    const uint32_t b = 31u - __clz(m | 1u);
-                    const uint32_t *row = w0 + entry_k(e.x) * s.rw + entry_o(e.x) + word;
-                    const bool hit = (__funnelshift_r(row[0], row[1], b) & e.y) != 0;
-                    ++h;
-                    const bool lost = !hit && h >= mn;  // every group tried (rare)
-                    if (lost && m) leave(word, 1u << b);
-                    if (hit || lost) {
-                        m &= ~(1u << b);
-                        h = 0;
-                    }
-                    if (m == 0) h = 0;
+                    qn -= min(qn, uint32_t(__popc(idle)));
+                    step();
                 }
-                __syncwarp();
             }
         }
+        while (__any_sync(~0u, ev.m != 0)) step();
         j = jn;
         buf ^= 1u;
     }
@@ -464,7 +476,7 @@ using namespace gbs;
 struct gbc_sparse {
     gbc_sparse_config cfg{};
     std::string err;
-    uint32_t tb = 0, dlt = 0, rw = 0, stride = 0, tiles_max = 0, pmax = 0;
+    uint32_t tb = 0, dlt = 0, rw = 0, rows = 0, stride = 0, tiles_max = 0, pmax = 0;
     uint32_t c[kK] = {};
     uint64_t qbound = 0;                   // sieving primes up to isqrt(limit + M)
     std::vector<uint2> groups;             // plan entries (entry_k / entry_o / entry_n, packed offsets)
@@ -475,8 +487,9 @@ struct gbc_sparse {
     uint32_t *d_xf = nullptr;
     uint2 *d_groups = nullptr;
     uint32_t *d_goff = nullptr;
-    uint2 *d_masks = nullptr;              // the groups after the first kWordGroups: class | word << 4, offsets as a mask
-    uint2 *d_cls = nullptr;                // per even class: first mask, masks | entries of the first groups << 16
+    uint2 *d_entries = nullptr;            // the checker's plan (check_plan): the first kWordGroups groups,
+    uint2 *d_masks = nullptr;              // the others,
+    uint4 *d_cls = nullptr;                // per even class: first entry, entries, first mask, plan entries they stand for
     uint32_t *d_map = nullptr;
     uint32_t *d_out = nullptr;             // witness output
     uint32_t out_cap = 0;
@@ -691,28 +704,106 @@ bool validate_plan(const gbc_sparse *sp, const std::vector<uint8_t> &isp, std::s
     return true;
 }
 
-// The plan as the checker's even form reads it: per even class the entries of
-// its first kWordGroups groups counted, every later group as one mask.
-void group_masks(const gbc_sparse *sp, std::vector<uint2> &masks, std::vector<uint2> &cls)
+// The shifts of pattern rows that test the offsets of mask and no other, the
+// pattern at offset x tests pattern << x: the patterns' best first, a shift
+// that tests one more offset only is the map row's own. sh[0]: of the map row,
+// sh[g + 1]: of pattern g. Another row costs as much as 1.3 shifts (two loads
+// against a funnel shift and half an OR).
+void cover(uint32_t mask, uint32_t npat, std::vector<uint32_t> (&sh)[kPatterns + 1])
 {
-    cls.assign(kHalfM, make_uint2(0u, 0u));
-    for (uint32_t x = 0; x < kHalfM; ++x) {
-        uint32_t seen = 0, head = 0, entries = 0;
-        cls[x].x = uint32_t(masks.size());
-        for (uint32_t g = sp->goff[x]; g < sp->goff[x + 1]; ++g) {
-            const uint2 e = sp->groups[g];
-            const uint32_t h = e.x & 0xFFFu;  // class and window word
-            if (!seen || h != head) {
-                ++seen;
-                head = h;
-                if (seen > kWordGroups) masks.push_back(make_uint2(h, 0u));
+    constexpr double kRow = 1.3;
+    for (auto &v : sh) v.clear();
+    uint32_t seen = 0;
+    for (;;) {
+        double best = 0.0;
+        uint32_t best_g = 0, best_seen = 0;
+        std::vector<uint32_t> best_at;
+        for (uint32_t g = 0; g < npat; ++g) {
+            if (!sh[g + 1].empty()) continue;
+            uint32_t s = seen;
+            std::vector<uint32_t> at;
+            double gain = -kRow;
+            for (;;) {
+                int more = 1;
+                uint32_t x = 0;
+                for (uint32_t y = 0; y < 32; ++y) {
+                    const uint64_t t = uint64_t(pattern(g)) << y;
+                    if (t & ~uint64_t(mask)) continue;
+                    const int n = __builtin_popcount(uint32_t(t) & ~s);
+                    if (n > more) {
+                        more = n;
+                        x = y;
+                    }
+                }
+                if (more == 1) break;
+                s |= pattern(g) << x;
+                at.push_back(x);
+                gain += more - 1;
             }
-            if (seen <= kWordGroups) ++entries;
-            else
-                for (uint32_t q = 0; q < entry_n(e.x); ++q) masks.back().y |= 1u << ((e.y >> (5 * q)) & 31u);
+            if (gain > best) {
+                best = gain;
+                best_g = g;
+                best_seen = s;
+                best_at = at;
+            }
         }
-        cls[x].y = (uint32_t(masks.size()) - cls[x].x) | entries << 16;
+        if (best <= 0.0) break;
+        seen = best_seen;
+        sh[best_g + 1] = best_at;
     }
+    for (uint32_t m = mask & ~seen; m; m &= m - 1) sh[0].push_back(uint32_t(__builtin_ctz(m)));
+}
+
+// The plan as the checker reads it. Per even class: the first kWordGroups
+// groups as entries of one row and up to six shifts (x = word of the staged
+// rows | steps of two shifts << 16, y as in a plan entry), every later group
+// as one mask (x = word of the staged rows), and kMaskEnd. False if the entries of a group
+// do not test its candidates, all of them and no other.
+bool check_plan(const gbc_sparse *sp, std::vector<uint2> &entries, std::vector<uint2> &masks, std::vector<uint4> &cls)
+{
+    cls.assign(kHalfM, make_uint4(0u, 0u, 0u, 0u));
+    const uint32_t cap = sp->cfg.group_cap ? sp->cfg.group_cap : ~0u, npat = sp->rows / kK - 1;
+    std::vector<uint32_t> sh[kPatterns + 1];
+    for (uint32_t x = 0; x < kHalfM; ++x) {
+        const uint32_t end = sp->goff[x] + std::min(sp->goff[x + 1] - sp->goff[x], cap);
+        uint32_t plan = 0, seen = 0;
+        cls[x].x = uint32_t(entries.size());
+        cls[x].z = uint32_t(masks.size());
+        for (uint32_t g = sp->goff[x]; g < end; ++seen) {
+            const uint32_t h = sp->groups[g].x & 0xFFFu;  // class and window word
+            uint32_t mask = 0, n = 0;
+            for (; g < end && (sp->groups[g].x & 0xFFFu) == h; ++g, ++n)
+                for (uint32_t q = 0; q < entry_n(sp->groups[g].x); ++q)
+                    mask |= 1u << ((sp->groups[g].y >> (5 * q)) & 31u);
+            if (seen >= kWordGroups) {
+                masks.push_back(make_uint2(entry_k(h) * sp->rw + entry_o(h), mask));
+                continue;
+            }
+            plan += n;
+            cover(mask, npat, sh);
+            uint32_t tested = 0;
+            for (uint32_t r = 0; r <= npat; ++r)
+                for (size_t i = 0; i < sh[r].size(); i += kEntryMax) {
+                    const uint32_t c = uint32_t(std::min<size_t>(kEntryMax, sh[r].size() - i));
+                    uint32_t y = 0;
+                    for (uint32_t q = 0; q < c; ++q) {
+                        y |= sh[r][i + q] << (5 * q);
+                        const uint64_t t = uint64_t(r ? pattern(r - 1) : 1u) << sh[r][i + q];
+                        if (t >> 32) return false;
+                        tested |= uint32_t(t);
+                    }
+                    if (c & 1) y |= sh[r][i + c - 1] << (5 * c);
+                    entries.push_back(make_uint2(((r * kK + entry_k(h)) * sp->rw + entry_o(h)) | (c + 1) / 2 << 16, y));
+                }
+            if (tested != mask) return false;
+        }
+        masks.push_back(make_uint2(kMaskEnd, 0u));
+        const uint32_t n = uint32_t(entries.size()) - cls[x].x;
+        if (n > 32) return false;  // an entry a lane
+        cls[x].y = n;
+        cls[x].w = plan;
+    }
+    return true;
 }
 
 SpSeg make_seg(const gbc_sparse *sp, uint64_t N, uint32_t dl, uint64_t start, uint64_t limit)
@@ -730,6 +821,12 @@ SpSeg make_seg(const gbc_sparse *sp, uint64_t N, uint32_t dl, uint64_t start, ui
     s.tiles = uint32_t((std::max<uint64_t>(need, s.T) + kTileBits - 1) / kTileBits);
     s.stride = sp->stride;
     s.rw = sp->rw;
+    s.rows = sp->rows;
+    // sixteen items per SM where that leaves a warp its four classes, at most
+    // a class per lane
+    const uint64_t share = uint64_t(kHalfM) * s.chunks / (16 * uint64_t(std::max(sp->sms, 1)));
+    s.block = uint32_t(std::min<uint64_t>(std::max<uint64_t>(share, kMinBlock), kMaxBlock)) / kCheckWarps * kCheckWarps;
+    s.blocks = (kHalfM + s.block - 1) / s.block;
     s.group_cap = sp->cfg.group_cap ? sp->cfg.group_cap : ~0u;
     s.map = sp->d_map;
     s.ctr = sp->d_ctr;
@@ -800,6 +897,8 @@ extern "C" int gbc_sparse_create(const gbc_sparse_config *cfg_in, gbc_sparse **o
         sp->tiles_max = uint32_t((bits + kTileBits - 1) / kTileBits);
         sp->stride = sp->tiles_max * kTileWords;
     }
+    // as many pattern rows as leave two buffers of all rows in shared memory
+    sp->rows = kK * std::min(kPatterns + 1, kCheckWindows / (2 * kK * sp->rw * 4));
     make_residues(sp->c);
     uint32_t bad = 0;
     if (!check_cover(sp->c, &bad)) {
@@ -814,6 +913,12 @@ extern "C" int gbc_sparse_create(const gbc_sparse_config *cfg_in, gbc_sparse **o
     if (!validate_plan(sp, isp, &why)) {
         *out = sp;
         return sp_fail(sp, GBC_E_STATE, "sparse plan failed validation: " + why);
+    }
+    std::vector<uint2> entries, masks;
+    std::vector<uint4> cls;
+    if (!check_plan(sp, entries, masks, cls)) {
+        *out = sp;
+        return sp_fail(sp, GBC_E_STATE, "the checker's entries differ from the plan");
     }
     if (cfg.host_only) {
         *out = sp;
@@ -845,21 +950,20 @@ extern "C" int gbc_sparse_create(const gbc_sparse_config *cfg_in, gbc_sparse **o
         SPCK(cudaMemcpy(sp->d_groups, sp->groups.data(), sp->groups.size() * sizeof(uint2), cudaMemcpyHostToDevice));
     SPCK(cudaMalloc(&sp->d_goff, (kHalfM + 1) * 4));
     SPCK(cudaMemcpy(sp->d_goff, sp->goff.data(), (kHalfM + 1) * 4, cudaMemcpyHostToDevice));
-    {
-        std::vector<uint2> masks, cls;
-        group_masks(sp, masks, cls);
-        SPCK(cudaMalloc(&sp->d_masks, std::max<size_t>(masks.size(), 1) * sizeof(uint2)));
-        if (!masks.empty())
-            SPCK(cudaMemcpy(sp->d_masks, masks.data(), masks.size() * sizeof(uint2), cudaMemcpyHostToDevice));
-        SPCK(cudaMalloc(&sp->d_cls, cls.size() * sizeof(uint2)));
-        SPCK(cudaMemcpy(sp->d_cls, cls.data(), cls.size() * sizeof(uint2), cudaMemcpyHostToDevice));
-    }
-    SPCK(cudaMalloc(&sp->d_map, size_t(kK) * sp->stride * 4));
-    SPCK(cudaMemset(sp->d_map, 0, size_t(kK) * sp->stride * 4));
+    SPCK(cudaMalloc(&sp->d_entries, std::max<size_t>(entries.size(), 1) * sizeof(uint2)));
+    if (!entries.empty())
+        SPCK(cudaMemcpy(sp->d_entries, entries.data(), entries.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+    SPCK(cudaMalloc(&sp->d_masks, std::max<size_t>(masks.size(), 1) * sizeof(uint2)));
+    if (!masks.empty())
+        SPCK(cudaMemcpy(sp->d_masks, masks.data(), masks.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+    SPCK(cudaMalloc(&sp->d_cls, cls.size() * sizeof(uint4)));
+    SPCK(cudaMemcpy(sp->d_cls, cls.data(), cls.size() * sizeof(uint4), cudaMemcpyHostToDevice));
+    SPCK(cudaMalloc(&sp->d_map, size_t(sp->rows) * sp->stride * 4));
+    SPCK(cudaMemset(sp->d_map, 0, size_t(sp->rows) * sp->stride * 4));
     SPCK(cudaMalloc(&sp->d_ctr, sizeof(SpCtr)));
     SPCK(cudaMalloc(&sp->d_pend, size_t(kPendCap) * sizeof(uint4)));
     SPCK(cudaFuncSetAttribute(k_sp_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTileWords * 4)));
-    const int csmem = int(2 * kK * sp->rw * 4);
+    const int csmem = int(2 * sp->rows * sp->rw * 4);
     SPCK(cudaFuncSetAttribute(k_sp_check, cudaFuncAttributeMaxDynamicSharedMemorySize, csmem));
     int occ = 0;
     SPCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_sp_check, kCheckThreads, csmem));
@@ -876,6 +980,7 @@ extern "C" void gbc_sparse_destroy(gbc_sparse *sp)
     cudaFree(sp->d_xf);
     cudaFree(sp->d_groups);
     cudaFree(sp->d_goff);
+    cudaFree(sp->d_entries);
     cudaFree(sp->d_masks);
     cudaFree(sp->d_cls);
     cudaFree(sp->d_map);
@@ -938,8 +1043,12 @@ extern "C" int gbc_sparse_verify(gbc_sparse *sp, uint64_t start, uint64_t limit,
         const SpSeg s = make_seg(sp, N, dl, start, limit);
         if (s.tiles > sp->tiles_max) return sp_fail(sp, GBC_E_STATE, "segment larger than the map");
         if (int rc = build_map(sp, s)) return rc;
-        k_sp_check<<<sp->check_ctas, kCheckThreads, 2 * kK * sp->rw * 4, sp->st>>>(s, sp->d_groups, sp->d_goff,
-                                                                                 sp->d_masks, sp->d_cls, sp->d_pend);
+        if (s.rows > kK) {
+            k_sp_pattern<<<dim3(sp->sms, kK), 256, 0, sp->st>>>(s);
+            SPCK(cudaGetLastError());
+        }
+        k_sp_check<<<sp->check_ctas, kCheckThreads, 2 * s.rows * s.rw * 4, sp->st>>>(s, sp->d_entries, sp->d_masks,
+                                                                                   sp->d_cls, sp->d_pend);
         SPCK(cudaGetLastError());
         SPCK(cudaEventRecord(sp->ev[3], sp->st));
         SpCtr ctr{};

@@ -550,7 +550,7 @@ typedef struct gbc_sparse_result {
     uint64_t evens;      /* evens in [start, limit] */
     uint64_t pending;    /* evens the GPU left, each resolved on the CPU (the reference's leftovers) */
     uint64_t map_primes; /* set map bits summed over the segments */
-    uint64_t groups;     /* plan entries tested word by word, summed over the checker's warps */
+    uint64_t groups;     /* plan entries taken word by word, summed over the checker's warps */
     uint64_t segments;
     double ms_sieve;     /* GPU time: first bits and tiles (primes below 2^20) */
     double ms_large;     /* GPU time: primes from 2^20 */
