@@ -865,11 +865,15 @@ static void finish_desc(const gbc_ctx *ctx, DescImage &img)
     if (!nrun) h.n_mid_min = h.n_hl_min = 0;
     h.chk_vb = h.ver_vb = h.cnt_vb = h.nlow = 0;
     uint64_t words = 0, sampled_words = 0;  // class words of the segments, and of the exact checker's
+    uint64_t smallest = UINT64_MAX;         // of the latter's smallest
     for (uint32_t i = 0; i < nseg; ++i) {
         const gbk::SegParams &sp = img.segs[i];
         const uint64_t w = (sp.seg_end - sp.seg_start) / 960 + 2;
         words += w;
-        if (sp.sampled && !sp.low) sampled_words += w;
+        if (sp.sampled && !sp.low) {
+            sampled_words += w;
+            smallest = std::min(smallest, w);
+        }
     }
     for (uint32_t i = 0; i < nseg; ++i) {
         gbk::SegParams &sp = img.segs[i];
@@ -878,7 +882,7 @@ static void finish_desc(const gbc_ctx *ctx, DescImage &img)
         img.cnt_pref[i] = h.cnt_vb;
         const uint64_t evens = (sp.seg_end - sp.seg_start) / 2 + 1;
         sp.ck_few = gbh::check_few(sp.seg_start) ? 1 : 0;
-        if (sp.sampled) gbh::check_split(evens, sampled_words, ctx->grids.sm, &sp.cw, &sp.vbx);
+        if (sp.sampled) gbh::check_split(evens, sampled_words, smallest, ctx->grids.sm, &sp.cw, &sp.vbx);
         else sp.vbx = gbh::verify_vbx(evens, ctx->grids.sm);
         if (sp.low) ++h.nlow;
         else if (sp.sampled) h.chk_vb += sp.vbx;

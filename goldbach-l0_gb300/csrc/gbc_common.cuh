@@ -501,7 +501,7 @@ void query_check_grids(Grids &g);
 void query_verify_grids(Grids &g);
 bool verify_word_funnel(uint32_t r, uint32_t p0, uint32_t members);
 void query_count_grids(Grids &g);
-void check_split(uint64_t evens, uint64_t words, int sm, uint32_t *cw, uint32_t *vbx);
+void check_split(uint64_t evens, uint64_t words, uint64_t smallest, int sm, uint32_t *cw, uint32_t *vbx);
 bool check_few(uint64_t seg_start);
 uint32_t verify_vbx(uint64_t evens, int sm);
 // single-run forms (the allocation-free entry point and the table build)

@@ -70,7 +70,7 @@ __device__ __forceinline__ void append_ridge(gbc_segment_result *res, uint64_t n
 // 8.0 ms (36 candidates in the word form 8.3, 48 8.6; the even form alone, two
 // windows a T, 11.8) against 17.6 for candidates tested over words of 32 evens
 // until the last even of 4096 was settled; 195 segments of uneven windows 24.5
-// against 53.4; 5e8 evens at 1e12 0.45 against 0.69 (with 40 candidates there
+// against 53.4; 5e8 evens at 1e12 0.36 against 0.69 (with 40 candidates there
 // 1.04: the last ones are seen late); 1e7 with the p(n) array 0.10 against 1.45.
 constexpr int kCkThreads = 512;
 constexpr int kCkCtas = 2;                         // CTAs per SM
@@ -639,14 +639,34 @@ void launch_init(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st)
     gbk::k_init<<<g.sm * 2, 256, 0, st>>>(d);
 }
 
-// words per chunk and CTAs of a sampled segment: full chunks, up to 16 per CTA
-// while the batch (words: of all its sampled segments) keeps three CTAs per
-// resident one (a CTA clears and flushes 31 KB of counts); below that shorter
-// chunks, down to a word per warp: 5e5 evens take 0.03 ms, against 0.06 on one CTA a class.
-void check_split(uint64_t evens, uint64_t words, int sm, uint32_t *cw, uint32_t *vbx)
+// words per chunk and items of a sampled segment: full chunks, up to 16 per
+// item while the batch (words: of all its sampled segments) keeps three items
+// per resident CTA (an item clears and flushes 31 KB of counts, and takes its
+// first 48 words even by even); below that shorter chunks, down to a word per
+// warp: 5e5 evens take 0.03 ms, against 0.06 on one CTA a class.
+// A segment of eight CTAs' work or more in a batch of at most 48 chunks per CTA
+// has a fixed number of items per CTA instead, all of the same chunks: one or
+// two or three, the fewest with at most 16 chunks; two at least beside
+// segments of less (smallest), whose items come between. p(n) of every even,
+// one GB300: one segment of 467.5M at 4e18 0.30 ms (three items per CTA 0.43),
+// two 0.46 (0.61), eight 1.51 (1.61); 1e9 integers at 1e12 0.36 (0.45);
+// sixteen windows of 2e4 to 5e8 0.71 (0.79, one item per CTA 0.87).
+void check_split(uint64_t evens, uint64_t words, uint64_t smallest, int sm, uint32_t *cw, uint32_t *vbx)
 {
     const uint64_t mine = evens / 15 / 32 + 2, want = uint64_t(sm) * gbk::kCkCtas;
     const uint64_t w = (words + want - 1) / want;
+    const bool beside = 8 * words > smallest * want && w > 2 * gbk::kCkWords;
+    const uint64_t k = std::max<uint64_t>((w + 16 * gbk::kCkWords - 1) / (16 * gbk::kCkWords), beside ? 2 : 1),
+                   items = mine * want * k / words;
+    if (items >= 8 * k && k <= 3) {
+        const uint64_t m = (mine + gbk::kCkWords * items) / (gbk::kCkWords * items);
+        const uint64_t each = (mine + m * items) / (m * items);
+        if (each >= gbk::kCkWarps) {
+            *cw = uint32_t(each);
+            *vbx = uint32_t(items);
+            return;
+        }
+    }
     *cw = uint32_t(w < gbk::kCkWarps ? gbk::kCkWarps : w > gbk::kCkWords ? gbk::kCkWords : w);
     const uint64_t nch = (mine + *cw - 1) / *cw;
     const uint64_t per = std::min<uint64_t>(16, std::max<uint64_t>(1, words / *cw / (3 * want)));
