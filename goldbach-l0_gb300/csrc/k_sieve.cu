@@ -25,6 +25,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "gbc_common.cuh"
 
@@ -688,8 +689,8 @@ __device__ __forceinline__ void ovf_push(const BatchParams &bp, uint32_t k, uint
 // width, by the table's random sectors. Measured against a pair that divided
 // base and base + span apart, took byte bounds and masks with 64-bit divisions
 // by 30 and placed each mark with 64-bit arithmetic (one GB300, harvest and
-// sort): one segment 1.27 -> 0.70 ms, 8 segments 1.63 -> 1.24, 128 segments
-// 8.13 -> 7.0, 292 segments of uneven windows 75.1 -> 42.1. Of that the units
+// sort): one segment 1.27 -> 0.66 ms, 8 segments 1.63 -> 1.14, 128 segments
+// 8.13 -> 6.8, 292 segments of uneven windows 75.1 -> 36.9. Of that the units
 // tested before the table is read (runs narrower than p / 4): one segment 0.75
 // -> 0.70, 8 segments 1.40 -> 1.24, the windows 46.6 -> 42.5. Few, large CTAs: every CTA
 // writes one stream per region bin, and the streams share the L2: 2 x 768
@@ -704,7 +705,7 @@ struct __align__(16) HlRun {
     uint32_t n_all;      // 0: no hit-listed prime
     uint64_t B;          // base / 30
     uint32_t nblk;
-    uint32_t vbase;      // the run's first virtual bit (binned)
+    uint32_t place;      // the run's first virtual bit (binned), or its number
 };
 
 // direct = 0: a binned batch's harvest (launched before the tiles); direct =
@@ -725,7 +726,9 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
     __shared__ uint32_t s_cls[8][8];
     __shared__ uint8_t s_res[32];
     __shared__ uint32_t s_hcnt[kHlMaxBins];
+    // the runs, those that most primes reach first
     __shared__ HlRun s_run[256];
+    __shared__ uint32_t s_n[256];
     __shared__ uint32_t s_lo;
     if (threadIdx.x == 0) s_lo = kNone;
     __syncthreads();
@@ -737,16 +740,24 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
         s_res[threadIdx.x - 64] = uint8_t(class_of(threadIdx.x - 64));
     }
     if (threadIdx.x < kHlMaxBins) s_hcnt[threadIdx.x] = 0;
-    for (uint32_t r = threadIdx.x; r < nrun; r += blockDim.x) {
-        const BatchParams &bp = d.runs[r];
+    if (threadIdx.x < nrun) {
+        const BatchParams &bp = d.runs[threadIdx.x];
+        s_n[threadIdx.x] = bp.n_hl < bp.n_all ? bp.n_all : 0u;
+    }
+    __syncthreads();
+    if (threadIdx.x < nrun) {
+        const BatchParams &bp = d.runs[threadIdx.x];
+        const uint32_t n = s_n[threadIdx.x];
+        uint32_t r = 0;  // the run's place
+        for (uint32_t o = 0; o < nrun; ++o) r += s_n[o] > n || (s_n[o] == n && o < threadIdx.x) ? 1u : 0u;
         HlRun x{};
         x.below = bp.base - 1;  // (base 0: a run of a few small q, wide against every p)
         x.span = uint32_t(min(30ull * bp.nblk - 1, 0xFFFFFFFFull));
-        x.n_all = bp.n_hl < bp.n_all ? bp.n_all : 0u;
+        x.n_all = n;
         x.B = bp.base / 30;
         x.nblk = bp.nblk;
         if (x.n_all) atomicMin(&s_lo, bp.n_hl);  // the same for every run that has some
-        x.vbase = bp.tb_vt0 * run0.tile_bits;
+        x.place = binned ? bp.tb_vt0 * run0.tile_bits : threadIdx.x;
         s_run[r] = x;
     }
     __syncthreads();
@@ -757,23 +768,22 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
     // the table: bytes [tb0, tb0 + tbn) of the multiplier line (the same for every run)
     const uint32_t *const mtab = run0.mtab;
     const uint64_t tb0 = run0.m0 / 30, tbn = (run0.m1 - run0.m0 + 1) / 30;
-    // the marks of class cls of q at bit t of run ri (t < nblk)
-    auto mark = [&](uint32_t ri, uint32_t vbase, uint32_t e, uint32_t t) {
+    // the mark of class e >> 16 of q at bit t of a run (t < nblk)
+    auto mark = [&](uint32_t place, uint32_t e, uint32_t t) {
         if (quota) {
-            const uint32_t v = vbase + t;
+            const uint32_t v = place + t;
             const uint32_t bin = (e >> 20) + (v >> rlog);
             const uint32_t pos = atomicAdd(&s_hcnt[bin], 1u);
             if (pos < quota) hl_mine[bin * quota + pos] = v & rmask;
             else ovf_push(run0, (e >> 16) & 7u, v);
         } else {
-            const BatchParams &bp = d.runs[ri];
+            const BatchParams &bp = d.runs[place];
             atomicAnd(bp.map + size_t((e >> 16) & 7u) * bp.wpc + (t >> 5), ~(1u << (t & 31)));
         }
     };
-    // the pair (prime i = p, run ri): every path of a lane ends here, so the
+    // the pair (prime p, run): every path of a lane ends here, so the
     // warp meets again before its next pair
-    auto pair = [&](uint32_t ri, uint32_t p, float rp, uint64_t inv, uint32_t pq, uint32_t pr, const HlRun &run) {
-        const uint32_t *const cls = s_cls[s_res[pr]];
+    auto pair = [&](uint32_t p, float rp, uint64_t inv, uint32_t pq, uint32_t pr, const HlRun &run) {
         uint32_t rho;
         const uint64_t b = divmod_recip(run.B, p, inv, rho) - tb0;  // byte b0 in the table
         // m = 30 b0 + j from j = ceil(30 rho / p) on, the estimate lowered by
@@ -787,7 +797,8 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
             if (((kUnits30 >> j) & 1u) && t < run.nblk) {
                 const uint32_t k = __popc(kUnits30 & ((1u << j) - 1u));
                 if (b >= tbn) atomicOr(run0.err, kErrTable);
-                else if ((__ldg(mtab + (b >> 2)) >> (8 * (uint32_t(b) & 3u) + k)) & 1u) mark(ri, run.vbase, cls[k], t);
+                else if ((__ldg(mtab + (b >> 2)) >> (8 * (uint32_t(b) & 3u) + k)) & 1u)
+                    mark(run.place, s_cls[s_res[pr]][k], t);
             }
             return;
         }
@@ -807,11 +818,12 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
                     const uint32_t k = __popc(kUnits30 & ((1u << j) - 1u));
                     if (b >= tbn || at >= tbn) atomicOr(run0.err, kErrTable);
                     else if ((__ldg(mtab + (at >> 2)) >> (8 * (uint32_t(at) & 3u) + k)) & 1u)
-                        mark(ri, run.vbase, cls[k], t);
+                        mark(run.place, s_cls[s_res[pr]][k], t);
                 }
             }
             return;
         }
+        const uint32_t *const cls = s_cls[s_res[pr]];
         if (p >> 31) {
             // p >= 2^31 > nblk: at most two bytes, their bits in 64-bit arithmetic
             const uint32_t more = uint64_t(rho) + run.nblk > p ? 1u : 0u;
@@ -825,7 +837,7 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
                 for (; v; v &= v - 1u) {
                     const uint32_t e = cls[__ffs(v) - 1u];
                     const int64_t t = int64_t(nb ? uint64_t(p) : 0u) + int64_t(pq * (e & 0xFFu) + ((e >> 8) & 0xFFu)) - rho;
-                    if (t >= 0 && t < int64_t(run.nblk)) mark(ri, run.vbase, e, uint32_t(t));
+                    if (t >= 0 && t < int64_t(run.nblk)) mark(run.place, e, uint32_t(t));
                 }
             }
             return;
@@ -867,7 +879,7 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
                 v &= v - 1u;
                 const uint32_t e = cls[j & 7u];
                 const uint32_t t = tb + p * (j >> 3) + pq * (e & 0xFFu) + ((e >> 8) & 0xFFu);
-                if (t < run.nblk) mark(ri, run.vbase, e, t);
+                if (t < run.nblk) mark(run.place, e, t);
             }
             if (!v) {
                 if (!left) break;
@@ -889,42 +901,60 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
     // (the mean and 45%), and the overflow list does not hold the rest.
     // Warp-uniform loops: the warp's first prime bounds them.
     const bool deal = nhi - i_lo < 8 * stride;
-    uint32_t i = i_lo + (deal ? ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31u)
-                              : blockIdx.x * blockDim.x + threadIdx.x);
-    uint32_t p_next = i < nhi ? __ldg(primes + i) : 3u;
-    for (; i - (threadIdx.x & 31u) < nhi; i += stride) {
-        const uint32_t p = p_next;
-        if (i + stride < nhi) p_next = __ldg(primes + i + stride);  // its latency behind this prime's work
-        const float rp = __fdividef(1.0f, __uint2float_rn(p));
-        uint64_t inv = recip64(p, rp);
-        const uint32_t pq = p / 30, pr = p - 30 * pq;
-        // A run of several narrower than p / 64: a pair goes on only if one of
-        // its integers is a multiple of p, which the remainder r of base - 1
-        // tells (the next multiple is base + p - 1 - r), so most warps stop
-        // there: 16 runs of 1e6 integers at 4e18..5e18 0.225 -> 0.146 ms a run.
-        // (A run alone would pay the exact reciprocal for one remainder; p >=
-        // 2^31: r takes 33 bits.)
-        uint32_t narrow = 0;
-        if (nrun > 1) {
+    // Of several runs only those that the warp's primes reach: 292 segments of
+    // uneven windows at 1e15..5e18 39.3 -> 36.9 ms, 16 windows at 1e10..3e18 1.60
+    // -> 0.73. One run apart (kMany), since that loop's bound, which the
+    // compiler cannot tell to be the same for a warp's lanes, cost it 9%: one
+    // segment 0.70 ms with a loop over all runs, 0.77 with this one, 0.66.
+    auto harvest = [&](auto many) {
+        constexpr bool kMany = decltype(many)::value;
+        const uint32_t lane = threadIdx.x & 31u;
+        uint32_t i = i_lo + (deal ? ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + lane
+                                  : blockIdx.x * blockDim.x + threadIdx.x);
+        uint32_t p_next = i < nhi ? __ldg(primes + i) : 3u;
+        uint32_t live = nrun, reach = 0;  // the runs that the warp's primes reach: all of them below reach
+        for (; i - lane < nhi; i += stride) {
+            const uint32_t p = p_next;
+            if (i + stride < nhi) p_next = __ldg(primes + i + stride);  // its latency behind this prime's work
+            const float rp = __fdividef(1.0f, __uint2float_rn(p));
+            uint64_t inv = recip64(p, rp);
+            const uint32_t pq = p / 30, pr = p - 30 * pq;
+            if constexpr (!kMany) {
+                if (i < s_run[0].n_all) pair(p, rp, inv, pq, pr, s_run[0]);
+                __syncwarp();
+                continue;
+            }
+            if (i - lane >= reach) {
+                while (live && s_run[live - 1].n_all <= i - lane) --live;
+                reach = live ? s_run[live - 1].n_all : kNone;
+            }
+            // A run narrower than p / 64: a pair goes on only if one of its
+            // integers is a multiple of p, which the remainder r of base - 1
+            // tells (the next multiple is base + p - 1 - r), so most warps stop
+            // there: 16 runs of 1e6 integers at 4e18..5e18 0.225 -> 0.146 ms a run.
+            // (A run alone would pay the exact reciprocal for one remainder; p >=
+            // 2^31: r takes 33 bits.)
             inv = recip64_exact(p, inv);
-            narrow = p >> 31 ? 0u : p >> 6;
-        }
-        for (uint32_t ri = 0; ri < nrun; ++ri) {
-            const uint64_t below = s_run[ri].below;
-            const uint32_t span = s_run[ri].span;
-            bool go = i < s_run[ri].n_all;
-            if (span < narrow) {
-                uint32_t r = uint32_t(below) - uint32_t(__umul64hi(below, inv)) * p;  // below 2 p
-                r = min(r, r - p);
-                go = go && r >= p - 1 - span;
+            const uint32_t narrow = p >> 31 ? 0u : p >> 6;
+            for (uint32_t ri = 0; ri < live; ++ri) {
+                const uint64_t below = s_run[ri].below;
+                const uint32_t span = s_run[ri].span;
+                bool go = i < s_run[ri].n_all;
+                if (span < narrow) {
+                    uint32_t r = uint32_t(below) - uint32_t(__umul64hi(below, inv)) * p;  // below 2 p
+                    r = min(r, r - p);
+                    go = go && r >= p - 1 - span;
+                }
+                if (go) {
+                    const HlRun run = s_run[ri];  // in registers: the marks' atomics would have it read again
+                    pair(p, rp, inv, pq, pr, run);
+                }
+                __syncwarp();
             }
-            if (go) {
-                const HlRun run = s_run[ri];  // in registers: the marks' atomics would have it read again
-                pair(ri, p, rp, inv, pq, pr, run);
-            }
-            __syncwarp();
         }
-    }
+    };
+    if (nrun > 1) harvest(std::true_type{});
+    else harvest(std::false_type{});
     if (quota) {
         __syncthreads();
         for (uint32_t bi = threadIdx.x; bi < nbin; bi += blockDim.x) run0.hl_cnt[blockIdx.x * nbin + bi] = s_hcnt[bi];
