@@ -277,7 +277,7 @@ __device__ __forceinline__ void transpose_word(const uint32_t (&h)[8], uint32_t 
 // windows of eight blocks the exact checker reads below an even: p <= 9781;
 // candidates of a class its word form takes (kCkFew in segments below 1e17)
 constexpr uint32_t kCkWindows = 41;
-constexpr uint32_t kCkFirst = 40, kCkFew = 24;
+constexpr uint32_t kCkFirst = 40, kCkFew = 28;
 
 // Candidate tables of the exact checker (uploaded once per context). Window
 // w of class c = r / 2 holds the blocks T - 8 w - 7 .. T - 8 w of the even

@@ -46,7 +46,9 @@ __device__ __forceinline__ void append_ridge(gbc_segment_result *res, uint64_t n
 // class sit in word j. A lane takes word j of all eight arrays and settles the
 // class's first candidates in ascending order, each a funnel shift and an AND
 // over 32 evens; their counts are the differences of the evens still open after
-// each (a popcount, two of them per warp reduction). Offsets and arrays are
+// each: a popcount, two of them added to a counter in shared memory that two
+// lanes of every warp share (a reduction over the warp for two, on the popcounts'
+// own pipe, took 8.0 ms where this takes 6.5). Offsets and arrays are
 // constants. A candidate settles 3.75 / ln q of the open evens: kCkFirst of them
 // from 1e17 on (about 97 evens in a hundred settled), kCkFew below, where that
 // many settle as much and the later ones are too rare to have been seen.
@@ -66,25 +68,30 @@ __device__ __forceinline__ void append_ridge(gbc_segment_result *res, uint64_t n
 // words at a segment's ends, and every word where p(n) or a low ridge floor
 // wants each even, take the even form alone, a T per lane.
 //
-// Bound by issue. One GB300, p(n) of every even: 48 segments of 467.5M at 4e18
-// 8.0 ms (36 candidates in the word form 8.3, 48 8.6; the even form alone, two
-// windows a T, 11.8) against 17.6 for candidates tested over words of 32 evens
-// until the last even of 4096 was settled; 195 segments of uneven windows 24.5
-// against 53.4; 5e8 evens at 1e12 0.36 against 0.69 (with 40 candidates there
-// 1.04: the last ones are seen late); 1e7 with the p(n) array 0.10 against 1.45.
+// Bound by issue and the popcounts' pipe. One GB300, p(n) of every even: 48
+// segments of 467.5M at 4e18 6.5 ms (36 candidates in the word form 6.56, 44
+// 6.59, 48 6.80; the even form alone, two windows a T, 11.8) against 17.6 for
+// candidates tested over words of 32 evens until the last even of 4096 was
+// settled; 195 segments of uneven windows 19.9 against 53.4; 5e8 evens at 1e12
+// 0.31 against 0.69 (24 candidates there 0.32, 32 0.35, 40 1.04: the last ones
+// are seen late); 1e7 with the p(n) array 0.10 against 1.45.
 constexpr int kCkThreads = 512;
 constexpr int kCkCtas = 2;                         // CTAs per SM
 constexpr uint32_t kCkWarps = kCkThreads / 32;
 constexpr uint32_t kCkHalo = 11;                   // words below a chunk: 41 windows of 8 blocks reach 335 back
 constexpr uint32_t kCkWords = kCkThreads - kCkHalo;  // words of a full chunk: one word per thread staged
 constexpr uint32_t kCkHist = 8;                    // windows counted in shared memory
-constexpr uint32_t kCkQueue = 32 * GBC_NCLASS;     // words of a warp's queue: a block's of every class
+constexpr uint32_t kCkHalf = 8;                    // classes settled at a time
+constexpr uint32_t kCkQueue = 32 * kCkHalf;        // words of a warp's queue: a block's of that many classes
+constexpr uint32_t kCkLanes = 16;                  // counters of a pair of candidates (lanes l and l + 16 share one)
 static_assert(32 * kCkHalo >= 8 * kCkWindows + 7, "the last window is staged");
+static_assert(17 * kCkWarps * (32 / kCkLanes) * 32 < 65536, "a counter of 16 bits holds an item of 17 chunks");
 static_assert(kCkWords <= 512 && kCkFirst % 2 == 0 && kCkFew % 2 == 0, "queue entries and candidate pairs");
 
 struct CkShared {
     uint32_t hist[GBC_NCLASS][64 * kCkHist];       // even form: marks by bit of the windows
-    uint32_t open[GBC_NCLASS][kCkFirst + 1];       // word form: evens taken, and those open after each candidate
+    uint32_t open[GBC_NCLASS][kCkFirst + 1];       // word form: evens taken, and those open after each candidate,
+    __align__(16) uint32_t part[GBC_NCLASS * kCkFirst / 2][kCkLanes];  // the latter of two candidates by lane until the item's end
     uint4 mask[GBC_NCLASS][kCkWindows];            // x, y: the window's candidates; z, w: those seen before the part
     uint32_t first[GBC_NCAND];
     uint32_t w0[GBC_NCLASS];                       // CheckTables::w0
@@ -145,22 +152,19 @@ __device__ __forceinline__ uint32_t bits_at(const Words &w)
 }
 
 template <uint32_t R, uint32_t I>
-__device__ __forceinline__ void two(const Words &w, uint32_t &un, uint32_t *open, uint32_t lane, uint32_t half)
+__device__ __forceinline__ void two(const Words &w, uint32_t &un, uint32_t *part)
 {
     un &= ~bits_at<Of<R, I>::c.k, Of<R, I>::c.o>(w);
-    const uint32_t n0 = __popc(un);
+    const uint32_t n = __popc(un);
     un &= ~bits_at<Of<R, I + 1>::c.k, Of<R, I + 1>::c.o>(w);
-    const uint32_t n = __reduce_add_sync(~0u, n0 + (__popc(un) << 16));  // at most 1024 each
-    // lanes 0 and 1 add a half each
-    if (lane < 2) atomicAdd(open + I + 1, __byte_perm(n, 0u, half));
+    atomicAdd(part + (R / 2 * kCkFirst + I) / 2 * kCkLanes, n + (__popc(un) << 16));
 }
 
 // class R's candidates From, ... over a word per lane; un: its evens, then those still open
 template <uint32_t R, uint32_t From, size_t... H>
-__device__ __forceinline__ void run(const Words &w, uint32_t &un, uint32_t *open, uint32_t lane, uint32_t half,
-                                    std::index_sequence<H...>)
+__device__ __forceinline__ void run(const Words &w, uint32_t &un, uint32_t *part, std::index_sequence<H...>)
 {
-    (two<R, From + 2 * H>(w, un, open, lane, half), ...);
+    (two<R, From + 2 * H>(w, un, part), ...);
 }
 
 // the same for class C, and its words with open evens into the queue (place:
@@ -173,10 +177,9 @@ __device__ __forceinline__ void one(const Words &w, bool inner, uint32_t taken, 
     if (slow >> C & 1u) return;
     uint32_t un = inner ? ~0u : 0u;
     if (lane == 0) atomicAdd(&sh.open[C][0], taken);
-    const uint32_t half = lane ? 0x4432u : 0x4410u;
-    uint32_t *const open = sh.open[C] + (lane & 1u);
-    run<2 * C, 0>(w, un, open, lane, half, std::make_index_sequence<kCkFew / 2>());
-    if (!few) run<2 * C, kCkFew>(w, un, open, lane, half, std::make_index_sequence<(kCkFirst - kCkFew) / 2>());
+    uint32_t *const part = sh.part[0] + lane % kCkLanes;
+    run<2 * C, 0>(w, un, part, std::make_index_sequence<kCkFew / 2>());
+    if (!few) run<2 * C, kCkFew>(w, un, part, std::make_index_sequence<(kCkFirst - kCkFew) / 2>());
     const uint32_t bal = __ballot_sync(~0u, un != 0);
     if (un) {
         const uint32_t at = qn + __popc(bal & ((1u << lane) - 1u));
@@ -186,13 +189,14 @@ __device__ __forceinline__ void one(const Words &w, bool inner, uint32_t taken, 
     qn += __popc(bal);
 }
 
-template <size_t... C>
+// classes From, ...
+template <uint32_t From, size_t... C>
 __device__ __forceinline__ void all(const Words &w, bool inner, uint32_t slow, bool few, CkShared &sh,
                                      uint32_t *q_bits, uint16_t *q_at, uint32_t place, uint32_t lane,
                                     uint32_t &qn, std::index_sequence<C...>)
 {
     const uint32_t taken = 32 * __popc(__ballot_sync(~0u, inner));
-    (one<C>(w, inner, taken, slow, few, sh, q_bits, q_at, place, lane, qn), ...);
+    (one<From + C>(w, inner, taken, slow, few, sh, q_bits, q_at, place, lane, qn), ...);
 }
 
 }  // namespace ckw
@@ -245,7 +249,11 @@ __global__ void __launch_bounds__(kCkThreads, kCkCtas) k_check(BatchDesc d, Chec
         const bool few = sp.ck_few != 0;
         if (tid < GBC_NCLASS) sh.w0[tid] = uint32_t((few ? ct.w0_few : ct.w0) >> (4 * tid)) & 15u;
         for (uint32_t i = tid; i < GBC_NCLASS * 64 * kCkHist; i += kCkThreads) sh.hist[0][i] = 0;
-        for (uint32_t i = tid; i < GBC_NCLASS * (kCkFirst + 1); i += kCkThreads) sh.open[0][i] = 0;
+        const bool word_form = words && !pn;  // (else every class is slow)
+        if (tid < GBC_NCLASS) sh.open[tid][0] = 0;
+        if (word_form)
+            for (uint32_t i = tid; i < sizeof sh.part / 16; i += kCkThreads)
+                reinterpret_cast<uint4 *>(sh.part)[i] = make_uint4(0u, 0u, 0u, 0u);
         for (uint32_t i = tid; i < GBC_NCAND; i += kCkThreads) sh.first[i] = kNone;
         // everything of an even but its histogram mark: first occurrence, p(n), ridge
         auto note = [&](uint32_t c, uint32_t bit, uint32_t T) {
@@ -407,8 +415,11 @@ __global__ void __launch_bounds__(kCkThreads, kCkCtas) k_check(BatchDesc d, Chec
                             return make_uint2(__ldg(at + size_t(k) * wpc - 1), __ldg(at + size_t(k) * wpc));
                         };
                         const ckw::Words w{pair(0), pair(1), pair(2), pair(3), pair(4), pair(5), pair(6), pair(7)};
-                        ckw::all(w, inner, slow, few, sh, q_bits, q_at, j - j0, lane, qn,
-                                 std::make_index_sequence<GBC_NCLASS>());
+                        ckw::all<0>(w, inner, slow, few, sh, q_bits, q_at, j - j0, lane, qn,
+                                    std::make_index_sequence<kCkHalf>());
+                        settle(false);
+                        ckw::all<kCkHalf>(w, inner, slow, few, sh, q_bits, q_at, j - j0, lane, qn,
+                                          std::make_index_sequence<GBC_NCLASS - kCkHalf>());
                         settle(false);
                         const uint32_t je = min(jw + 32, jb);
                         if (slow)
@@ -429,13 +440,26 @@ __global__ void __launch_bounds__(kCkThreads, kCkCtas) k_check(BatchDesc d, Chec
             }
         }
         __syncthreads();
+        for (uint32_t i = tid; word_form && i < GBC_NCLASS * kCkFirst / 2; i += kCkThreads) {
+            const uint4 *v = reinterpret_cast<const uint4 *>(sh.part[i]);
+            uint32_t a = 0, b = 0;
+#pragma unroll
+            for (uint32_t l = 0; l < kCkLanes / 4; ++l) {
+                a += (v[l].x & 0xFFFFu) + (v[l].y & 0xFFFFu) + (v[l].z & 0xFFFFu) + (v[l].w & 0xFFFFu);
+                b += (v[l].x >> 16) + (v[l].y >> 16) + (v[l].z >> 16) + (v[l].w >> 16);
+            }
+            uint32_t *const at = sh.open[i / (kCkFirst / 2)] + 2 * (i % (kCkFirst / 2)) + 1;
+            at[0] = a;
+            at[1] = b;
+        }
+        __syncthreads();
         for (uint32_t i = tid; i < GBC_NCLASS * 64 * kCkHist; i += kCkThreads) {
             const uint32_t v = sh.hist[0][i];
             if (!v) continue;
             const uint32_t c = i / (64 * kCkHist), bit = i % (64 * kCkHist);
             atomicAdd(&res->hist[c][__ldg(ct_ci + c * (64 * kCkWindows) + bit)], v);
         }
-        for (uint32_t i = tid; i < GBC_NCLASS * kCkFirst; i += kCkThreads) {
+        for (uint32_t i = tid; word_form && i < GBC_NCLASS * kCkFirst; i += kCkThreads) {
             const uint32_t c = i / kCkFirst, at = i % kCkFirst;
             if (few && at >= kCkFew) continue;
             const uint32_t v = sh.open[c][at] - sh.open[c][at + 1];
@@ -648,9 +672,10 @@ void launch_init(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st)
 // has a fixed number of items per CTA instead, all of the same chunks: one or
 // two or three, the fewest with at most 16 chunks; two at least beside
 // segments of less (smallest), whose items come between. p(n) of every even,
-// one GB300: one segment of 467.5M at 4e18 0.30 ms (three items per CTA 0.43),
-// two 0.46 (0.61), eight 1.51 (1.61); 1e9 integers at 1e12 0.36 (0.45);
-// sixteen windows of 2e4 to 5e8 0.71 (0.79, one item per CTA 0.87).
+// one GB300, before the word form's counters: one segment of 467.5M at 4e18
+// 0.30 ms (three items per CTA 0.43), two 0.46 (0.61), eight 1.51 (1.61); 1e9
+// integers at 1e12 0.36 (0.45); sixteen windows of 2e4 to 5e8 0.71 (0.79, one
+// item per CTA 0.87).
 void check_split(uint64_t evens, uint64_t words, uint64_t smallest, int sm, uint32_t *cw, uint32_t *vbx)
 {
     const uint64_t mine = evens / 15 / 32 + 2, want = uint64_t(sm) * gbk::kCkCtas;

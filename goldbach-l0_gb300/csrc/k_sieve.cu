@@ -7,7 +7,7 @@
 //   k_xfirst  per tile-sieve prime, class and run: the first class bit of
 //             the run that is a multiple of p and >= p^2 (mid_setup's job,
 //             goldbach.cl:3528-3563; host_math.cpp:80-113).
-//   k_tile    one CTA per (run, class, tile) item: up to 2^tile_log2 bits in
+//   k_tile    one CTA per (run, class, tile) item: up to tile_bits bits in
 //             shared memory; the primes 7..67 by whole-word AND patterns of
 //             seven prime groups, then every prime 71..p_mid by shared-memory
 //             atomics (small primes warp-cooperatively, the rest one per
@@ -20,6 +20,9 @@
 //             stage clears (the 30030 wheel and the 17..43 skip of
 //             goldbach.cl:638-748).
 //   k_hitlist the primes above p_hl through the prime-multiplier table.
+//   k_map_finish the marks that no bin held; in runs narrow for their height
+//             primality tests of what the tiles leave, in place of every
+//             prime past them.
 // A thread reads its prime once and applies it to every run of the batch,
 // so a batch of many short windows streams the sieving primes once.
 #include <cuda_runtime.h>
