@@ -192,17 +192,55 @@ __global__ void __launch_bounds__(1024, 1) k_sp_tile(SpSeg s, const uint32_t *pr
     }
 }
 
+// The primes from 2^20 on, one per thread: most reach a row of dl + TB bits in
+// few of the twelve classes or none. With r = Q mod p the first multiplier mlo
+// gives p mlo - Q = e (0 or p - r), and class k's is mlo + d, d = (mu_k - mlo)
+// mod M: its bit (e + p d - c_k) / M lies below T only if d <= (M T + M - e) /
+// p, 32-bit arithmetic for all twelve (a float bound, two above its error);
+// only classes that pass take the exact first bit and its test.
+// Bound by issue. 98M primes at 4e18 on one GB300: 0.77 ms at T = 2^16 + TB
+// against 1.73 with a 64-bit division and the exact bit of every class (0.96
+// with the division), 4.50 against 7.4 at 2^26 + TB.
 __global__ void __launch_bounds__(256) k_sp_large(SpSeg s, const uint32_t *primes, uint32_t i0, uint32_t n,
                                                   const uint16_t *inv)
 {
+    __shared__ uint32_t s_c[kK];
+    if (threadIdx.x < kK) s_c[threadIdx.x] = s.c[threadIdx.x];
+    __syncthreads();
+    const float qf = __ull2float_rz(s.Q), span = __ull2float_ru(uint64_t(kM) * s.T + kM);
     for (uint32_t i = i0 + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t p = __ldg(primes + i);
-        uint64_t t[kK];
-        sp_first(s.Q, p, __ldg(inv + p % kM), s.c, t);
+        const uint32_t p = __ldg(primes + i), invp = __ldg(inv + p % kM);
+        // Q = p qd + r: two float estimates, the second of what the first
+        // leaves (below 2^54), then at most two steps
+        const float rp = __fdividef(1.0f, __uint2float_rn(p));
+        uint64_t qd = __float2ull_rz(qf * rp);
+        int64_t r = int64_t(s.Q - qd * p);
+        const int64_t more = __float2ll_rn(__ll2float_rn(r) * rp);
+        qd += uint64_t(more);
+        r -= more * int64_t(p);
+        while (r < 0) {
+            r += p;
+            --qd;
+        }
+        while (r >= int64_t(p)) {
+            r -= p;
+            ++qd;
+        }
+        const uint64_t mlo = qd + (r != 0 ? 1 : 0);
+        const uint32_t mm = uint32_t(mlo % kM);
+        const uint32_t dmax = __float2uint_ru(fminf(span * rp, float(kM))) + 2u;
+        uint32_t reach = 0;
 #pragma unroll
         for (uint32_t k = 0; k < kK; ++k) {
+            const uint32_t mu = (s.c[k] * invp) % kM;
+            const uint32_t d = mu >= mm ? mu - mm : mu + kM - mm;
+            reach |= d <= dmax ? 1u << k : 0u;
+        }
+        for (; reach; reach &= reach - 1u) {
+            const uint32_t k = __ffs(reach) - 1u, c = s_c[k], mu = (c * invp) % kM;
+            const uint32_t d = mu >= mm ? mu - mm : mu + kM - mm;
             uint32_t *row = s.map + size_t(k) * s.stride;
-            for (uint64_t x = t[k]; x < s.T; x += p) {
+            for (uint64_t x = ((p * (mlo + d) - s.Q - c) >> 1) * kInvHalfM; x < s.T; x += p) {
                 uint32_t *w = row + (x >> 5);
                 const uint32_t bit = 1u << (x & 31);
                 if (__ldcg(w) & bit) atomicAnd(w, ~bit);
