@@ -17,7 +17,8 @@
 //   k_sp_tile   persistent CTAs over (class, 2^20-bit tile) items: the tile
 //               in shared memory, primes below 2^10 warp-cooperatively, the
 //               rest a thread per prime, one coalesced store (bits >= T zero)
-//   k_sp_large  a thread per prime from 2^20: its twelve first bits, each mark
+//   k_sp_large  a thread per prime from 2^20: its first bits in the classes whose
+//               rows it can reach, each mark
 //               a read of the word and an atomic AND only where the bit is set
 //   k_sp_popc   set bits of the map
 //   k_sp_pattern  rows that hold the OR of a map row's bits at a few offsets
@@ -27,7 +28,7 @@
 //               copies land while this one is checked); a warp takes an even
 //               class, each lane eight words of its evens, and ORs in the
 //               shifts of map and pattern rows that test the plan's first two
-//               groups; the evens still open, about one in 25, are then taken
+//               groups; the evens still open, about one in 40, are then taken
 //               one per lane, a group as one 32-bit window of its row ANDed
 //               with the group's candidates; evens no group verifies go to
 //               the pending list, which the host resolves by an ascending
@@ -302,7 +303,7 @@ __device__ __forceinline__ void sp_stage(const SpSeg &s, uint32_t *buf, uint64_t
 // 15. The even form is about 35 instructions for the 10 to 15 candidates of a
 // group, with every lane at work: a lane keeps its word over the end of a
 // class. An even is verified by a candidate with probability 0.12 at 4e18:
-// about one in 25 is open after the two fullest groups. One CTA an SM, since
+// about one in 40 is open after the two fullest groups. One CTA an SM, since
 // two buffers of 60 row windows take 144 KB.
 // Bound by the ALU pipe (75%) and issue (78%). One GB300, 1.05e12 evens at
 // 4e18: 125.1 ms (three groups word by word: 129.6; 3 patterns 147.3, 4 145.3,
