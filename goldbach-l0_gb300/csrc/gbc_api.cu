@@ -882,11 +882,15 @@ static void finish_desc(const gbc_ctx *ctx, DescImage &img)
         img.cnt_pref[i] = h.cnt_vb;
         const uint64_t evens = (sp.seg_end - sp.seg_start) / 2 + 1;
         sp.ck_few = gbh::check_few(sp.seg_start) ? 1 : 0;
-        if (sp.sampled) gbh::check_split(evens, sampled_words, smallest, ctx->grids.sm, &sp.cw, &sp.vbx);
-        else sp.vbx = gbh::verify_vbx(evens, ctx->grids.sm);
-        if (sp.low) ++h.nlow;
-        else if (sp.sampled) h.chk_vb += sp.vbx;
-        else h.ver_vb += sp.vbx;
+        if (sp.low) {
+            ++h.nlow;  // the generic checker's: no items of the others
+        } else if (sp.sampled) {
+            gbh::check_split(evens, sampled_words, smallest, ctx->grids.sm, &sp.cw, &sp.vbx);
+            h.chk_vb += sp.vbx;
+        } else {
+            sp.vbx = gbh::verify_vbx(evens, ctx->grids.sm);
+            h.ver_vb += sp.vbx;
+        }
         h.cnt_vb += gbh::count_ranges(img.runs[sp.run].base, sp, words, ctx->grids.sm);
     }
     img.chk_pref[nseg] = h.chk_vb;

@@ -682,7 +682,7 @@ void check_split(uint64_t evens, uint64_t words, uint64_t smallest, int sm, uint
     const uint64_t w = (words + want - 1) / want;
     const bool beside = 8 * words > smallest * want && w > 2 * gbk::kCkWords;
     const uint64_t k = std::max<uint64_t>((w + 16 * gbk::kCkWords - 1) / (16 * gbk::kCkWords), beside ? 2 : 1),
-                   items = mine * want * k / words;
+                   items = words ? mine * want * k / words : 0;  // (0: no segment of the batch is the checker's)
     if (items >= 8 * k && k <= 3) {
         const uint64_t m = (mine + gbk::kCkWords * items) / (gbk::kCkWords * items);
         const uint64_t each = (mine + m * items) / (m * items);
