@@ -827,9 +827,12 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
             return;
         }
         const uint32_t *const cls = s_cls[s_res[pr]];
-        if (p >> 31) {
-            // p >= 2^31 > nblk: at most two bytes, their bits in 64-bit arithmetic
-            const uint32_t more = uint64_t(rho) + run.nblk > p ? 1u : 0u;
+        if ((p >> 31) || p > ~run.nblk) {
+            // p + nblk >= 2^32 (a run of 2^31 bits and the margin, p close to
+            // 2^31) or p >= 2^31: at most three bytes, their bits in 64-bit
+            // arithmetic
+            const uint64_t x = uint64_t(rho) + run.nblk - 1;
+            const uint32_t more = (x >= p ? 1u : 0u) + (x >= 2ull * p ? 1u : 0u);
             if (b >= tbn || b + more >= tbn) {
                 atomicOr(run0.err, kErrTable);
                 return;
@@ -839,7 +842,7 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
                 uint32_t v = (__ldg(mtab + (at >> 2)) >> (8 * (uint32_t(at) & 3u))) & 0xFFu;
                 for (; v; v &= v - 1u) {
                     const uint32_t e = cls[__ffs(v) - 1u];
-                    const int64_t t = int64_t(nb ? uint64_t(p) : 0u) + int64_t(pq * (e & 0xFFu) + ((e >> 8) & 0xFFu)) - rho;
+                    const int64_t t = int64_t(uint64_t(nb) * p) + int64_t(pq * (e & 0xFFu) + ((e >> 8) & 0xFFu)) - rho;
                     if (t >= 0 && t < int64_t(run.nblk)) mark(run.place, e, uint32_t(t));
                 }
             }
