@@ -425,7 +425,7 @@ extern "C" int gbc_create(const gbc_config *cfg_in, gbc_ctx **out)
     ctx->primes = gbh_cached_primes(std::max<uint64_t>(bound, 127));
     const auto &pr = ctx->primes;
     ctx->i0 = uint32_t(std::lower_bound(pr.begin(), pr.end(), gbk::kFirstSievePrime) - pr.begin());
-    ctx->n_mid = uint32_t(std::upper_bound(pr.begin(), pr.end(), cfg.p_mid) - pr.begin());
+    ctx->n_mid = uint32_t(std::upper_bound(pr.begin(), pr.end(), std::min(cfg.p_mid, gbk::kMaxTilePrime)) - pr.begin());
     ctx->tile_bits = cfg.tile_bits ? cfg.tile_bits : 1u << cfg.tile_log2;
     const uint32_t tb = ctx->tile_bits;
     // primes with at least 128 marks per tile: a warp per prime; above, a

@@ -26,6 +26,9 @@ constexpr uint32_t kWheelM = 1001;    // 7 * 11 * 13: the large-prime multiplier
 // the 720 unit gaps, the inverses mod 1001 (1001), the inverses mod 17..43
 // back to back (240)
 constexpr uint32_t kWheelTabWords = 1001 + 720 + 1001 + 240;
+// largest prime of the tile sieve: a mark's shared-memory bit (below 2^22) and
+// three strides of it stay below 2^32; larger primes are the large-prime kernel's
+constexpr uint32_t kMaxTilePrime = uint32_t(((1ull << 32) - (1u << 22)) / 3);
 constexpr uint32_t kPackGroup = 256;  // packed large primes per group (one warp decodes a group)
 
 // u_k, the residue of class array k

@@ -187,8 +187,11 @@ __device__ __forceinline__ void clear_bit(uint32_t b)
                  "r"(__funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, b)));
 }
 
-// Clears bits b, b + st, b + 2 st, ... below end (b < end + st, end + 4 st < 2^32):
-// four marks per bound check.
+// Clears bits b, b + st, b + 2 st, ... below end, four marks per bound check.
+// b + 3 st < 2^32: a lane's own prime has b < end < 2^22 and st <=
+// kMaxTilePrime, a prime of a whole warp b < end + st and st < 2^20.
+static_assert(8u * (228u << 10) + 1835008u < 1u << 22, "bits of the largest tile in shared memory");
+static_assert((1ull << 22) + 3ull * kMaxTilePrime <= 1ull << 32, "three strides past a tile's end");
 __device__ __forceinline__ void clear_stride(uint32_t b, uint32_t st, uint32_t end)
 {
     for (; b + 3u * st < end; b += 4u * st) {

@@ -65,7 +65,8 @@ typedef struct gbc_config {
     uint64_t segment_even;   /* integer span of a full segment (default 467.5M) */
     uint32_t max_batch;      /* segments per batch the slots are sized for (default 8, at most 256) */
     uint32_t tile_log2;      /* log2 of shared-memory tile bits per class (14..20, default 20); see tile_bits */
-    uint32_t p_mid;          /* primes <= p_mid: shared-memory tiles; above: large-prime kernel (default 2^22) */
+    uint32_t p_mid;          /* primes <= p_mid: shared-memory tiles (to 1.43e9 at most); above:
+                                large-prime kernel (default 2^22) */
     uint32_t want_pn;        /* 1: slots also hold a per-even u16 p(n) buffer */
     int32_t device;          /* CUDA device ordinal (default 0) */
     uint32_t max_runs;       /* runs per batch the slots are sized for (a run: consecutive segments
