@@ -184,7 +184,8 @@ __device__ __forceinline__ uint32_t tile_bit0(const uint32_t *s) { return 8u * s
 __device__ __forceinline__ void clear_bit(uint32_t b)
 {
     asm volatile("red.shared::cta.and.b32 [%0], %1;" ::"r"((b >> 3) & ~3u),
-                 "r"(__funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, b)));
+                 "r"(__funnelshift_l(0xFFFFFFFEu, 0xFFFFFFFEu, b))
+                 : "memory");
 }
 
 // Clears bits b, b + st, b + 2 st, ... below end, four marks per bound check.
