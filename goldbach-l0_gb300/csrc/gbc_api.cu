@@ -241,8 +241,8 @@ static void hl_regions(uint64_t nblk, uint32_t &rlog, uint32_t &nreg)
 // Offsets per (harvest CTA, bin): the expected marks of a whole region (not
 // the batch's average over bins: its last region is cut short) + 45%, + 64,
 // whole lines. marks_per_bit: marks per class bit. The margin covers the
-// harvest CTAs' uneven shares: CTA c takes primes in blocks of 256, and the
-// first blocks (the smallest primes, with the most marks) weigh most.
+// harvest CTAs' uneven shares, which hl_deal keeps below it: the first CTA's
+// primes are the smallest of every round and have the most marks.
 static uint32_t hl_quota(double marks_per_bit, uint64_t nblk, uint32_t rlog, uint32_t ctas)
 {
     const double region = double(std::min<uint64_t>(nblk, uint64_t(1) << rlog));
@@ -597,6 +597,9 @@ extern "C" int gbc_create(const gbc_config *cfg_in, gbc_ctx **out)
     gbh::query_verify_grids(ctx->grids);
     gbh::query_count_grids(ctx->grids);
     gbh::query_sieve_grids(ctx->grids);
+    if (ctx->hl_on)
+        gbh::hl_shares(pr.data(), ctx->n_hl, uint32_t(pr.size()), uint32_t(ctx->grids.sm) * uint32_t(ctx->grids.hitlist),
+                       &ctx->hl_shares);
     CK(dev_alloc(ctx, &ctx->d_primes, (pr.size() + kPrimePad) * 4));
     CK(cudaMemcpy(ctx->d_primes, pr.data(), pr.size() * 4, cudaMemcpyHostToDevice));
     CK(dev_alloc(ctx, &ctx->d_magic, (magic.size() + kPrimePad) * 4));
@@ -846,7 +849,6 @@ static void finish_desc(const gbc_ctx *ctx, DescImage &img)
     h.n_mid_max = 0;
     h.n_mid_min = UINT32_MAX;
     h.n_hl_max = 0;
-    h.n_hl_min = UINT32_MAX;
     h.n_all_max = 0;
     uint64_t test_words = 0;
     for (uint32_t r = 0; r < nrun; ++r) {
@@ -857,12 +859,15 @@ static void finish_desc(const gbc_ctx *ctx, DescImage &img)
         h.n_mid_max = std::max(h.n_mid_max, bp.n_mid);
         h.n_mid_min = std::min(h.n_mid_min, bp.n_mid);
         h.n_hl_max = std::max(h.n_hl_max, bp.n_hl);
-        h.n_hl_min = std::min(h.n_hl_min, bp.n_hl);
         h.n_all_max = std::max(h.n_all_max, bp.n_all);
     }
     img.tile_pref[nrun] = h.tile_items;
     h.test_words = gbh::test_words(test_words, ctx->grids.sm);
-    if (!nrun) h.n_mid_min = h.n_hl_min = 0;
+    if (!nrun) h.n_mid_min = 0;
+    h.hl_deal = gbk::kDealBlocks;
+    if (ctx->hl_on && ctx->n_hl < h.n_all_max)
+        h.hl_deal = gbh::hl_deal(&ctx->hl_shares, ctx->primes.data(), ctx->n_hl, h.n_all_max,
+                                 uint32_t(ctx->grids.sm) * uint32_t(ctx->grids.hitlist), gbk::hl_binned(img.runs[0]));
     h.chk_vb = h.ver_vb = h.cnt_vb = h.nlow = 0;
     uint64_t words = 0, sampled_words = 0;  // class words of the segments, and of the exact checker's
     uint64_t smallest = UINT64_MAX;         // of the latter's smallest
@@ -1307,7 +1312,6 @@ static int issue_selfcheck(gbc_ctx *ctx, Slot &s)
         ci.h->n_all_max = std::max(ci.h->n_all_max, bp.n_all);
     }
     ci.h->n_hl_max = ci.h->n_all_max;
-    ci.h->n_hl_min = ci.h->n_all_max;
     ci.h->nseg = 0;  // no checker work
     cudaStream_t st = s.st;
     CK(cudaMemcpyAsync(s.chk_desc_dev, s.chk_desc_host, ctx->layout.bytes, cudaMemcpyHostToDevice, st));

@@ -194,7 +194,8 @@ struct BatchHeader {
     uint32_t tile_items;           // (run, tile, class) items of the tile kernel, tile-major per run
     uint32_t n_mid_max;            // first bits: primes [i0, n_mid_max)
     uint32_t n_mid_min, n_hl_max;  // large primes: [n_mid_min, n_hl_max)
-    uint32_t n_hl_min, n_all_max;  // hit-listed primes: [n_hl_min, n_all_max)
+    uint32_t n_all_max;            // hit-listed primes: [a run's n_hl, n_all_max)
+    uint32_t hl_deal;              // how the harvest deals them out (HlDeal)
     uint32_t chk_vb, ver_vb, cnt_vb; // virtual CTAs of k_check, k_verify, k_count
     uint32_t nlow;                 // segments that need the generic low checker
     // a window of the batch for the per-segment launches of the plain form
@@ -211,6 +212,11 @@ struct BatchHeader {
     // descriptor copy resets them
     uint32_t work[5];
 };
+
+// The hit-listed primes of a CTA of the harvest: consecutive ones, a pass of
+// the grid after the other; by warps, 32 consecutive primes each, in turn over
+// the CTAs; one by one in turn over the CTAs.
+enum HlDeal : uint32_t { kDealBlocks = 0, kDealWarps = 1, kDealLanes = 2 };
 
 constexpr int kWorkTile = 0, kWorkCheck = 1, kWorkVerify = 2, kWorkCount = 3, kWorkBinsort = 4;
 constexpr uint32_t kHlMaxBins = 64;  // region bins of a binned batch (8 classes x up to 8 regions)
@@ -485,6 +491,15 @@ void launch_large(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st);
 // marks of every other batch (after the tiles)
 void launch_hitlist(const gbk::BatchDesc &d, bool direct, const Grids &g, cudaStream_t st);
 void launch_binsort(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st);
+// what hl_deal reads of a context's hit-listed primes, primes[n_lo, n): sum[d][k] =
+// the first CTA's share of the first k rounds of dealing d (blocks, warps), 1 / p summed
+constexpr uint32_t kHlRounds = 512;
+struct HlShares {
+    double sum[2][kHlRounds + 1];
+};
+void hl_shares(const uint32_t *primes, uint32_t n_lo, uint32_t n, uint32_t ctas, HlShares *out);
+// the dealing of a batch whose largest hit-listed prime is primes[n_hi - 1]
+uint32_t hl_deal(const HlShares *sh, const uint32_t *primes, uint32_t n_lo, uint32_t n_hi, uint32_t ctas, bool binned);
 // after the tiles: the overflow marks, the narrow runs' primality tests
 uint32_t test_words(uint64_t words, int sm);
 void launch_map_finish(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st);

@@ -117,6 +117,7 @@ struct gbc_ctx {
     uint32_t tile_bits = 0;   // bits per tile of the persistent tile kernel
     uint32_t tile_stage = 0;  // tile-bin offsets it stages into shared memory
     uint32_t n_hl = 0;                 // index of the first prime >= p_hl
+    gbh::HlShares hl_shares{};         // their shares over the harvest's CTAs
     uint32_t *mtab = nullptr;          // wheel-30 bytes of the primes in [mtab_m0, mtab_m1]
     uint64_t mtab_m0 = 0, mtab_m1 = 0, mtab_bytes = 0;
     uint64_t mtab_builds = 0;

@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "gbc_common.cuh"
@@ -904,13 +905,8 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
     };
     const uint32_t *primes = run0.primes;
     const uint32_t stride = gridDim.x * blockDim.x;
-    // A CTA takes consecutive primes, whose table bytes are neighbours: dealt
-    // out warp by warp across the CTAs 128 segments took 7.55 ms, not 6.93. Few
-    // primes are dealt out so all the same: with less than some passes of the
-    // grid the CTAs' shares of marks differ by more than a bin's quota allows
-    // (the mean and 45%), and the overflow list does not hold the rest.
     // Warp-uniform loops: the warp's first prime bounds them.
-    const bool deal = nhi - i_lo < 8 * stride;
+    const uint32_t deal = d.h->hl_deal;
     // Of several runs only those that the warp's primes reach: 292 segments of
     // uneven windows at 1e15..5e18 39.3 -> 36.9 ms, 16 windows at 1e10..3e18 1.60
     // -> 0.73. One run apart (kMany), since that loop's bound, which the
@@ -918,13 +914,14 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
     // segment 0.70 ms with a loop over all runs, 0.77 with this one, 0.66.
     auto harvest = [&](auto many) {
         constexpr bool kMany = decltype(many)::value;
-        const uint32_t lane = threadIdx.x & 31u;
-        uint32_t i = i_lo + (deal ? ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + lane
-                                  : blockIdx.x * blockDim.x + threadIdx.x);
-        uint32_t p_next = i < nhi ? __ldg(primes + i) : 3u;
+        const uint32_t warp = threadIdx.x >> 5, off = (threadIdx.x & 31u) * (deal == kDealLanes ? gridDim.x : 1u);
+        uint32_t first = i_lo + (deal == kDealBlocks  ? blockIdx.x * blockDim.x + warp * 32
+                                 : deal == kDealWarps ? (warp * gridDim.x + blockIdx.x) * 32
+                                                      : warp * 32 * gridDim.x + blockIdx.x);
+        uint32_t p_next = first + off < nhi ? __ldg(primes + first + off) : 3u;
         uint32_t live = nrun, reach = 0;  // the runs that the warp's primes reach: all of them below reach
-        for (; i - lane < nhi; i += stride) {
-            const uint32_t p = p_next;
+        for (; first < nhi; first += stride) {
+            const uint32_t i = first + off, p = p_next;
             if (i + stride < nhi) p_next = __ldg(primes + i + stride);  // its latency behind this prime's work
             const float rp = __fdividef(1.0f, __uint2float_rn(p));
             uint64_t inv = recip64(p, rp);
@@ -934,8 +931,8 @@ __global__ void __launch_bounds__(kHlThreads, kHlCtas) k_hitlist(BatchDesc d, ui
                 __syncwarp();
                 continue;
             }
-            if (i - lane >= reach) {
-                while (live && s_run[live - 1].n_all <= i - lane) --live;
+            if (first >= reach) {
+                while (live && s_run[live - 1].n_all <= first) --live;
                 reach = live ? s_run[live - 1].n_all : kNone;
             }
             // A run narrower than p / 64: a pair goes on only if one of its
@@ -1438,6 +1435,47 @@ void query_sieve_grids(Grids &g)
     int n = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gbk::k_hitlist, gbk::kHlThreads, 0);
     g.hitlist = n > 0 ? n : 1;
+}
+
+void hl_shares(const uint32_t *primes, uint32_t n_lo, uint32_t n, uint32_t ctas, HlShares *out)
+{
+    for (uint32_t d = 0; d < 2; ++d) {
+        const uint32_t block = d == gbk::kDealBlocks ? gbk::kHlThreads : 32;
+        out->sum[d][0] = 0;
+        for (uint32_t k = 0; k < kHlRounds; ++k) {
+            const uint64_t i = n_lo + uint64_t(k) * block * ctas;
+            out->sum[d][k + 1] = out->sum[d][k] + (i < n ? double(block) / primes[i] : 0.0);
+        }
+    }
+}
+
+// A CTA takes consecutive primes, whose table bytes are neighbours: dealt out
+// warp by warp across the CTAs 128 segments took 7.55 ms, not 6.93. But every
+// CTA has one quota a bin, the mean and 45% (hl_quota), and the first CTA's
+// primes, the smallest of every round, have the most marks: 1.2 of the mean at
+// 4e18 with the tile primes to 1.7e6, 1.42 at 1e15, 3.0 there with those to
+// 2^18, above what the overflow list holds of a wide batch. So the primes are
+// dealt out by warps where blocks would give the first CTA more than 1.40 (1 / p
+// for a prime's marks: 3% above the marks themselves) or there are fewer than 8
+// rounds, whose last is a part of one; and one by one where warps would (a few
+// thousand primes, or primes from 2e4 on: 2.6 of the mean from 1e4 on at 1e12,
+// 1.1 one by one).
+uint32_t hl_deal(const HlShares *sh, const uint32_t *primes, uint32_t n_lo, uint32_t n_hi, uint32_t ctas, bool binned)
+{
+    constexpr double kMost = 1.40;
+    const uint32_t n = n_hi - n_lo;
+    const double lo = std::log(double(primes[n_lo])), hi = std::log(double(primes[n_hi - 1]));
+    const double mean = std::max(std::log(hi / lo), double(n) / primes[n_hi - 1]) / ctas;
+    auto first = [&](uint32_t d, uint32_t block) {  // the first CTA's share; past the summed rounds at most
+        const uint32_t round = block * ctas, rounds = uint32_t((uint64_t(n) + round - 1) / round);
+        if (rounds <= kHlRounds) return sh->sum[d][rounds];
+        const double p = primes[n_lo + kHlRounds * round];
+        return sh->sum[d][kHlRounds] + std::log(hi / std::log(p)) / ctas + block / p;
+    };
+    const bool few = n < 8ull * gbk::kHlThreads * ctas;
+    if (!binned) return few ? gbk::kDealWarps : gbk::kDealBlocks;
+    if (!few && first(gbk::kDealBlocks, gbk::kHlThreads) <= kMost * mean) return gbk::kDealBlocks;
+    return first(gbk::kDealWarps, 32) <= kMost * mean ? gbk::kDealWarps : gbk::kDealLanes;
 }
 
 void launch_binsort(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st)
