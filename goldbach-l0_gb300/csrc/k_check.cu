@@ -83,9 +83,10 @@ constexpr uint32_t kCkWords = kCkThreads - kCkHalo;  // words of a full chunk: o
 constexpr uint32_t kCkHist = 8;                    // windows counted in shared memory
 constexpr uint32_t kCkHalf = 8;                    // classes settled at a time
 constexpr uint32_t kCkQueue = 32 * kCkHalf;        // words of a warp's queue: a block's of that many classes
+constexpr uint32_t kCkMaxChunks = 18;              // chunks of an item at most (check_split)
 constexpr uint32_t kCkLanes = 16;                  // counters of a pair of candidates (lanes l and l + 16 share one)
 static_assert(32 * kCkHalo >= 8 * kCkWindows + 7, "the last window is staged");
-static_assert(17 * kCkWarps * (32 / kCkLanes) * 32 < 65536, "a counter of 16 bits holds an item of 17 chunks");
+static_assert(kCkMaxChunks * kCkWarps * (32 / kCkLanes) * 32 < 65536, "a counter of 16 bits holds an item");
 static_assert(kCkWords <= 512 && kCkFirst % 2 == 0 && kCkFew % 2 == 0, "queue entries and candidate pairs");
 
 struct CkShared {
@@ -670,7 +671,9 @@ void launch_init(const gbk::BatchDesc &d, const Grids &g, cudaStream_t st)
 // warp: 5e5 evens take 0.03 ms, against 0.06 on one CTA a class.
 // A segment of eight CTAs' work or more in a batch of at most 48 chunks per CTA
 // has a fixed number of items per CTA instead, all of the same chunks: one or
-// two or three, the fewest with at most 16 chunks; two at least beside
+// two or three, the fewest with at most 16 chunks on the batch's mean (a
+// segment's own, of 8 items or more, have an eighth more at most: kCkMaxChunks);
+// two at least beside
 // segments of less (smallest), whose items come between. p(n) of every even,
 // one GB300, before the word form's counters: one segment of 467.5M at 4e18
 // 0.30 ms (three items per CTA 0.43), two 0.46 (0.61), eight 1.51 (1.61); 1e9
@@ -686,7 +689,7 @@ void check_split(uint64_t evens, uint64_t words, uint64_t smallest, int sm, uint
     if (items >= 8 * k && k <= 3) {
         const uint64_t m = (mine + gbk::kCkWords * items) / (gbk::kCkWords * items);
         const uint64_t each = (mine + m * items) / (m * items);
-        if (each >= gbk::kCkWarps) {
+        if (each >= gbk::kCkWarps && m <= gbk::kCkMaxChunks) {
             *cw = uint32_t(each);
             *vbx = uint32_t(items);
             return;

@@ -12,6 +12,7 @@ import sys
 import pytest
 
 import gbc
+from conftest import ROOT
 
 CALL = """
 import ctypes as C, sys
@@ -23,6 +24,7 @@ for q in sys.stdin:
     print(cw.value, vbx.value)
 """
 SM, WORDS, WARPS = 152, 501, 16  # multiprocessors; words of a full chunk; warps of a CTA (a word each at least)
+MAX_CHUNKS = 18
 
 
 def splits(queries):
@@ -66,4 +68,10 @@ def test_every_split_covers_its_segment_in_the_kernel_s_bounds():
         queries += [(e, sum(words), min(words), SM) for e in rnd.sample(segs, min(len(segs), 3))]
     for (evens, *_), (cw, vbx) in zip(queries, splits(queries)):
         assert WARPS <= cw <= WORDS and vbx >= 1
-        assert chunks_per_item(evens, cw, vbx) <= 18, (evens, cw, vbx)
+        assert chunks_per_item(evens, cw, vbx) <= MAX_CHUNKS, (evens, cw, vbx)
+
+
+def test_the_counters_are_asserted_for_the_split_s_bound():
+    src = open(os.path.join(ROOT, "goldbach-l0_gb300", "csrc", "k_check.cu")).read()
+    assert f"kCkMaxChunks = {MAX_CHUNKS};" in src
+    assert "static_assert(kCkMaxChunks * " in src and "m <= gbk::kCkMaxChunks" in src
