@@ -27,6 +27,9 @@
 // are taken from there, a word per lane, even by even through the plan's other
 // funnels.
 //
+// Plans without the word form's funnels take their few from a table, word by
+// word (plan_words).
+//
 // Evens no plan funnel settles are pending: (class, word of the segment's
 // evens of the class, bits) for k_tail.
 //
@@ -267,6 +270,62 @@ __device__ __noinline__ void pend_word(const SegParams &sp, const BatchParams &b
     atomicAdd(reinterpret_cast<unsigned long long *>(&res->pending), (unsigned long long)__popc(m));
 }
 
+// The evens T .. T + 31 of a class that its plan settles, T the first even of
+// a word plus s < 32, nf funnels read from the table a member at a time: two
+// loads, a shift and an OR for 32 evens (w: the word of array 0 among the
+// staged windows).
+__device__ __forceinline__ uint32_t plan_word(const uint32_t *w, const uint2 *ev, uint32_t nf, uint32_t s)
+{
+    uint32_t v = 0;
+    for (uint32_t f = 0; f < nf; ++f) {
+        const uint2 e = ev[f];
+        const uint32_t *const a = w + (e.x & 7u) * kVWin;
+        for (uint32_t m = e.y; m; m &= m - 1u) {
+            const int32_t o = int32_t(e.x >> 8) - (__ffs(m) - 1) - int32_t(s);  // below 0: up to s bits ahead
+            const uint32_t *const x = a - (o >> 5);
+            v |= __funnelshift_l(x[-1], x[0], uint32_t(o));
+        }
+    }
+    return v;
+}
+
+// The plan's pending words among the warp's next 32 words of every class, jw ..
+// of the run, by the table (win: the first one's among the staged windows): the
+// words of the segment's evens of a class, a word per lane, are the pending list's.
+__device__ __forceinline__ void plan_words(const SegParams &sp, const uint32_t *win, uint32_t jw,
+                                           const uint2 (*ev)[kVerifyMaxFun], const uint32_t *nf, uint32_t A,
+                                           uint32_t ra, uint32_t B, uint32_t rb)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    gbc_segment_result *const res = sp.res;
+#pragma unroll 1
+    for (uint32_t c = 0; c < GBC_NCLASS; ++c) {
+        const uint32_t T0 = A + (2 * c < ra ? 1u : 0u), T1 = B - (2 * c > rb ? 1u : 0u);
+        const uint32_t t = 32 * (jw + lane) + (T0 & 31u);
+        uint32_t m = 0;
+        if (t >= T0 && t <= T1) m = (T1 - t >= 31 ? ~0u : (2u << (T1 - t)) - 1u) & ~plan_word(win + lane, ev[c], nf[c], T0 & 31u);
+        const uint32_t bal = __ballot_sync(~0u, m != 0);
+        if (!bal) continue;
+        const uint32_t evens = __reduce_add_sync(~0u, __popc(m));
+        uint32_t at = 0;
+        if (lane == 0) {
+            at = atomicAdd(&res->npend, uint32_t(__popc(bal)));
+            atomicAdd(reinterpret_cast<unsigned long long *>(&res->pending), (unsigned long long)evens);
+        }
+        at = __shfl_sync(~0u, at, 0) + __popc(bal & ((1u << lane) - 1u));
+        if (!m) continue;
+        if (at < sp.pend_cap) sp.pend[at] = make_uint2((c << 27) | ((t - T0) >> 5), m);
+        else atomicOr(&res->err, kErrPendOverflow);
+    }
+}
+
+// kWord: the plan holds the word form's three funnels of every class. A plan
+// of fewer than five funnels may not; all its funnels are then taken word by
+// word from the table, and every even that is left is pending. One GB300, 1e7
+// integers a call at 4e18, three and four funnels a class: 0.69 and 0.74 ms (9.31
+// and 4.00 with every even by itself, 1.43 and 1.36 with class words staged
+// class by class); five, in the word form, 0.75.
+template <bool kWord>
 __global__ void __launch_bounds__(kVerifyThreads, kVerifyCtas) k_verify(BatchDesc d, VerifyTables vt)
 {
     __shared__ uint2 s_ev[GBC_NCLASS][kVerifyMaxFun];  // see VerifyTables::ev
@@ -329,6 +388,11 @@ __global__ void __launch_bounds__(kVerifyThreads, kVerifyCtas) k_verify(BatchDes
             phase ^= 1u << buf;
             const uint32_t Jc = J0 + ch * kVChunk;
             const uint32_t *const win = stage + buf * (8 * kVWin);
+            if constexpr (!kWord) {
+                for (uint32_t w = 0; w < kVW && Jc + 32 * w <= jhi; ++w)
+                    plan_words(sp, win + kVBack + 32 * w, Jc + 32 * w, s_ev, s_nf, A, ra, B, rb);
+                continue;
+            }
             // The queue's words, one per lane, even by even; a lane whose word
             // is settled takes the queue's last one. Ends with the queue empty
             // (words may stay with lanes), or with every word settled.
@@ -388,7 +452,7 @@ __global__ void __launch_bounds__(kVerifyThreads, kVerifyCtas) k_verify(BatchDes
                         un[c] = hi > lo ? (0xFFFFFFFFu >> (32 - (hi - lo))) << lo : 0u;
                     }
                 }
-                if (vt.word) vp::word(win + kVBack + 32 * w + lane, un, std::make_index_sequence<8>());
+                vp::word(win + kVBack + 32 * w + lane, un, std::make_index_sequence<8>());
                 // the words still open into the queue
 #pragma unroll
                 for (uint32_t c = 0; c < GBC_NCLASS; ++c) {
@@ -439,14 +503,16 @@ uint32_t verify_vbx(uint64_t evens, int sm)
 
 void launch_verify(const gbk::BatchDesc &d, const gbk::VerifyTables &vt, const Grids &g, cudaStream_t st)
 {
-    gbk::k_verify<<<g.sm * g.verify, gbk::kVerifyThreads, gbk::kVerifySmem, st>>>(d, vt);
+    if (vt.word) gbk::k_verify<true><<<g.sm * g.verify, gbk::kVerifyThreads, gbk::kVerifySmem, st>>>(d, vt);
+    else gbk::k_verify<false><<<g.sm * g.verify, gbk::kVerifyThreads, gbk::kVerifySmem, st>>>(d, vt);
 }
 
 void query_verify_grids(Grids &g)
 {
     int n = 0;
-    cudaFuncSetAttribute(gbk::k_verify, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gbk::kVerifySmem));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gbk::k_verify, gbk::kVerifyThreads, gbk::kVerifySmem);
+    cudaFuncSetAttribute(gbk::k_verify<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gbk::kVerifySmem));
+    cudaFuncSetAttribute(gbk::k_verify<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gbk::kVerifySmem));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gbk::k_verify<true>, gbk::kVerifyThreads, gbk::kVerifySmem);
     g.verify = n > 0 ? n : 1;
 }
 

@@ -88,7 +88,7 @@ typedef struct gbc_config {
     uint32_t plan_funnels;   /* funnels per class of the verify plan (default 8, at most 32; below 6
                                 the evens a production segment leaves to the exact continuation can
                                 overflow its pending list, and the batch fails closed; below 5 the
-                                verify kernel takes every funnel even by even, which is slower) */
+                                verify kernel reads the funnels from a table, which is slower) */
     uint32_t ridge_min;      /* evens with p(n) >= ridge_min are listed (default 3000,
                                 include/config.hpp:104 RIDGE_MIN_DEFAULT) */
     uint32_t launch_mode;    /* 0 or 1: a batch is one replay of the slot's CUDA graph of the whole
