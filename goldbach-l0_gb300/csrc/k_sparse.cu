@@ -793,17 +793,13 @@ void cover(uint32_t mask, uint32_t npat, std::vector<uint32_t> (&sh)[kPatterns +
     for (uint32_t m = mask & ~seen; m; m &= m - 1) sh[0].push_back(uint32_t(__builtin_ctz(m)));
 }
 
-// The plan as the checker reads it. Per even class: the first kWordGroups
-// groups as entries of one row and up to six shifts (x = word of the staged
-// rows | steps of two shifts << 16, y as in a plan entry), every later group
-// as one mask (x = word of the staged rows), and kMaskEnd. False if the entries of a group
-// do not test its candidates, all of them and no other.
-bool check_plan(const gbc_sparse *sp, std::vector<uint2> &entries, std::vector<uint2> &masks, std::vector<uint4> &cls)
+// Even classes [x0, x1) of check_plan, their entries and masks numbered from 0.
+bool check_plan_part(const gbc_sparse *sp, uint32_t x0, uint32_t x1, std::vector<uint2> &entries,
+                     std::vector<uint2> &masks, uint4 *cls)
 {
-    cls.assign(kHalfM, make_uint4(0u, 0u, 0u, 0u));
     const uint32_t cap = sp->cfg.group_cap ? sp->cfg.group_cap : ~0u, npat = sp->rows / kK - 1;
     std::vector<uint32_t> sh[kPatterns + 1];
-    for (uint32_t x = 0; x < kHalfM; ++x) {
+    for (uint32_t x = x0; x < x1; ++x) {
         const uint32_t end = sp->goff[x] + std::min(sp->goff[x + 1] - sp->goff[x], cap);
         uint32_t plan = 0, seen = 0;
         cls[x].x = uint32_t(entries.size());
@@ -841,6 +837,35 @@ bool check_plan(const gbc_sparse *sp, std::vector<uint2> &entries, std::vector<u
         if (n > 32) return false;  // an entry a lane
         cls[x].y = n;
         cls[x].w = plan;
+    }
+    return true;
+}
+
+// The plan as the checker reads it. Per even class: the first kWordGroups
+// groups as entries of one row and up to six shifts (x = word of the staged
+// rows | steps of two shifts << 16, y as in a plan entry), every later group
+// as one mask (x = word of the staged rows), and kMaskEnd. False if the entries of a group
+// do not test its candidates, all of them and no other. A run of classes per
+// thread, put together in class order.
+bool check_plan(const gbc_sparse *sp, std::vector<uint2> &entries, std::vector<uint2> &masks, std::vector<uint4> &cls)
+{
+    cls.assign(kHalfM, make_uint4(0u, 0u, 0u, 0u));
+    const unsigned nt = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    std::vector<std::vector<uint2>> pe(nt), pm(nt);
+    std::vector<char> ok(nt, 0);
+    std::vector<std::thread> th;
+    auto begin = [&](unsigned t) { return kHalfM * t / nt; };
+    for (unsigned t = 0; t < nt; ++t)
+        th.emplace_back([&, t] { ok[t] = check_plan_part(sp, begin(t), begin(t + 1), pe[t], pm[t], cls.data()); });
+    for (auto &x : th) x.join();
+    for (unsigned t = 0; t < nt; ++t) {
+        if (!ok[t]) return false;
+        for (uint32_t x = begin(t); x < begin(t + 1); ++x) {
+            cls[x].x += uint32_t(entries.size());
+            cls[x].z += uint32_t(masks.size());
+        }
+        entries.insert(entries.end(), pe[t].begin(), pe[t].end());
+        masks.insert(masks.end(), pm[t].begin(), pm[t].end());
     }
     return true;
 }
