@@ -1154,8 +1154,8 @@ struct Bpsw {
         return ok;
     }
 
-    // The Jacobi symbol (a | n) is -1; 0 < a < 2^31 without a common factor with n.
-    __device__ __noinline__ static bool jacobi_minus(uint32_t a, uint64_t n)
+    // the Jacobi symbol (a | n), 0 < a < 2^31
+    __device__ __noinline__ static int jacobi(uint32_t a, uint64_t n)
     {
         bool neg = false;
         const int z = __ffs(a) - 1;
@@ -1173,12 +1173,13 @@ struct Bpsw {
             m = a;
             a = t;
         }
-        return neg;
+        return m > 1 ? 0 : neg ? -1 : 1;
     }
 
-    // The first P: the symbols of the primes up to 23 as a sign per k <= 24
-    // give those of (P - 2)(P + 2) up to P = 22; one n in a thousand or so
-    // needs more.
+    // The first P, or 0 where P^2 - 4 has a factor of n before it (n > 2^33 is
+    // then composite; not below P = 127, without a factor below 128): the
+    // symbols of the primes up to 23 as a sign per k <= 24 give those of (P - 2)
+    // (P + 2) up to P = 22; one n in a thousand or so needs more.
     template <uint32_t F>
     __device__ __forceinline__ static uint32_t signs(uint32_t r, uint64_t n)
     {
@@ -1209,13 +1210,19 @@ struct Bpsw {
         if ((n & 7) == 3 || (n & 7) == 5) k ^= 1u << 2 | 1u << 6 | 1u << 8 | 1u << 10 | 1u << 14 | 1u << 18 | 1u << 22 | 1u << 24;
         const uint32_t p = (k ^ k >> 4) & 0x1FFFFEu;  // bit P - 2
         if (p) return uint32_t(__ffs(p)) + 1u;
-        uint32_t x = 23;
-        while (x < 30000 && !jacobi_minus(x * x - 4, n)) ++x;
-        return x;
+        for (uint32_t x = 23; x < 30000; ++x) {
+            const int j = jacobi(x * x - 4, n);
+            if (j <= 0) return j ? x : 0u;
+        }
+        return 0;  // (a square)
     }
 
     // V_d = 2 and U_d = 0 (then V_(d+1) = P), the same with both signs turned,
-    // or V_(d 2^r) = 0 for an r < s - 1 (n + 1 = d 2^s, d odd)
+    // or V_(d 2^r) = 0 for an r < s - 1 (n + 1 = d 2^s, d odd). V_d = 0 is taken
+    // for s = 1 too, where no n has it: with x + 1 / x = P it says x^(n+1) = -1
+    // modulo every prime q of n, so x has an order divisible by 4 there; the
+    // order divides q - (P^2 - 4 | q), so the symbol is q mod 4 for every q, and
+    // -1 for n makes n = 3 mod 4, which is s > 1.
     __device__ __forceinline__ bool lucas() const
     {
         const uint32_t p = lucas_p();
@@ -1240,7 +1247,7 @@ struct Bpsw {
             v = sub(mul(v, v), two);
             ok = v == 0;
         }
-        return ok;
+        return ok && p;  // (a return at the start cost the test 6%)
     }
 };
 
