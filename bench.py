@@ -454,7 +454,7 @@ def sparse_leg(gbc, nseg=2, dlt_log2=26):
             "e2e": {"value": r.evens / r.ms_total / 1e6, "unit": "G evens/s", "h2d_bytes_per_step": 16,
                     "d2h_bytes_per_step": 32 * r.segments + 16 * r.pending},
             "evens": r.evens, "segments": r.segments, "pending": r.pending, "map_primes": r.map_primes,
-            "entries_per_warp_task": r.groups / (r.evens / 4096), "init_s": init_s,
+            "word_entries_per_warp_task": r.groups / (r.evens / 8192), "init_s": init_s,
             "stage_ms": {"sieve": r.ms_sieve, "large": r.ms_large, "check": r.ms_check, "wall": r.ms_total},
             "config": {"workload": f"[{a}, {a + span - 2}]", "M": 30030, "K": 12, "pmax": 40_000_000,
                        "evens_per_class_per_segment": 1 << dlt_log2}}
