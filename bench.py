@@ -265,7 +265,7 @@ def plain_leg(gbc, start, nseg, first_seg, knobs=None):
     segs = [(start + i * SEG, start + i * SEG + SEG - 2) for i in range(first_seg, first_seg + 2 * nseg + 1)]
     limit = segs[-1][1]
     k = {n: v for n, v in (knobs or {}).items()
-         if n in ("p_mid", "mtab_max_gb", "tile_log2", "plan_funnels", "verify_funnels")}
+         if n in ("p_mid", "mtab_max_gb", "tile_log2", "plan_funnels")}
     with gbc.Context(limit=limit, segment_even=SEG, max_batch=1, launch_mode=2, hl_mode=1, **k) as ctx:
         for sl in (0, 1):                                     # warm-up: tables, both slots
             ctx.enqueue_batch(sl, [segs[0]], limit, [gbc.SEG_VERIFY])
@@ -302,7 +302,7 @@ def plain_form_leg(gbc, start, first_seg, knobs=None, k=128):
     segs = [(start + i * SEG, start + i * SEG + SEG - 2) for i in range(first_seg, first_seg + 4 * k)]
     limit = segs[-1][1]
     kn = {n: v for n, v in (knobs or {}).items()
-          if n in ("p_mid", "mtab_max_gb", "tile_log2", "tile_bits", "plan_funnels", "verify_funnels")}
+          if n in ("p_mid", "mtab_max_gb", "tile_log2", "tile_bits", "plan_funnels")}
     flags = [0 if i % 256 == 0 else gbc.SEG_VERIFY for i in range(k)]
     batches = [segs[i * k:(i + 1) * k] for i in range(4)]
     with gbc.Context(limit=limit, segment_even=SEG, max_batch=k, launch_mode=3, hl_mode=1, **kn) as ctx:
@@ -334,7 +334,7 @@ def log_uniform(rnd, lo, hi):
 def sieve_knobs(knobs):
     """The sieve knobs of a knob set (tile size, split, table budget, verify
     plan), without its batch shape."""
-    keep = ("tile_log2", "tile_bits", "p_mid", "mtab_max_gb", "plan_funnels", "verify_funnels")
+    keep = ("tile_log2", "tile_bits", "p_mid", "mtab_max_gb", "plan_funnels")
     return {k: v for k, v in (knobs or {}).items() if k in keep and v}
 
 
@@ -698,7 +698,6 @@ def run_gb300(args, rep):
                          f"of sieving primes per step",
                    "tile_log2": cfg.tile_log2, "tile_bits": cfg.tile_bits, "p_mid": cfg.p_mid, "hl_mode": cfg.hl_mode,
                    "mtab_max_gb": cfg.mtab_max_gb, "plan_funnels": cfg.plan_funnels,
-                   "verify_funnels": cfg.verify_funnels,
                    "launch": "graph replay" if cfg.launch_mode != 2 else "direct launches",
                    "tuning": ("autotuner record " + os.path.relpath(args.tuning or autotune.DEFAULT_RECORD, ROOT))
                    if tuned else "defaults"},

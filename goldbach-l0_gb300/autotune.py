@@ -46,7 +46,7 @@ KNOBS = {
     "plan_funnels": [6, 8, 12, 16],
 }
 DEFAULTS = {"p_mid": 1 << 22, "mtab_max_gb": 48, "tile_log2": 20, "tile_bits": 0, "max_batch": 16,
-            "plan_funnels": 8, "verify_funnels": 3}
+            "plan_funnels": 8}
 DEFAULT_RECORD = os.path.join(HERE, "tuning", "gb300_production_4e18.json")
 
 

@@ -162,7 +162,6 @@ RunStats run_gpu(uint64_t limit, uint64_t segment_even, const std::string &spv_p
     cfg.tile_log2 = 20;
     cfg.tile_bits = kTileBits;
     cfg.plan_funnels = 16;
-    cfg.verify_funnels = 3;
     cfg.sample_every = sample;
     cfg.ridge_min = std::max<uint32_t>(ridge_min, GBC_TAIL_T);  // the plan's phase-A ceiling (ridge.hpp:89)
     gbc_ctx *raw = nullptr;
