@@ -316,7 +316,7 @@ struct VerifyTables {
     uint32_t fun_off[GBC_NCLASS], fun_cnt[GBC_NCLASS];
     uint32_t rest_off[GBC_NCLASS], rest_cnt[GBC_NCLASS];
     uint32_t ridge_min;     // evens with p(n) >= ridge_min are listed with their p(n)
-    uint32_t word;          // 1: the plan holds the word form's three funnels of every class
+    uint32_t word;          // 1: the plan holds the word form's three funnels of every class (0: plan_words)
     uint32_t spin0;         // try_wait rounds of the first wait on a chunk's bulk copies (kStageSpin)
 };
 

@@ -142,7 +142,7 @@ __global__ void k_noalloc_magic(const uint32_t *primes, uint32_t n, uint32_t *ma
 // CTA each: the eight class arrays' tiles in as few, as short waves as can be.
 // A tile costs its visits of every prime, whatever its size (kVisit), and its
 // marks and words (1 per unit): 2^16-bit tiles paid 545 us for 2^29 integers
-// at 1e12, 2184 tiles of one unit each; 114 us in 144 of 16.
+// at 1e12, 2192 tiles of one unit each; 114 us in 144 of 16.
 uint32_t tile_units(uint32_t units, uint32_t sms)
 {
     constexpr uint32_t kVisit = 8;

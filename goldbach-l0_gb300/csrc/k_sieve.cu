@@ -1008,8 +1008,8 @@ constexpr uint32_t kSortChunk = 256 * kSortPer;     // offsets a CTA sorts in sh
 // (consecutive threads, consecutive addresses). Offsets beyond a tile bin's
 // capacity go to the overflow list. The lists start 16-byte aligned (the
 // quota is a multiple of 32 words).
-// Six CTAs per SM (40 registers): the hit-list stage took 8.0 ms per
-// 128-segment batch against 8.2 at four (one wave of persistent CTAs).
+// Six CTAs per SM (40 registers): the hit-list stage takes 6.77 ms per
+// 128-segment batch (four 6.85, five 6.73, eight 7.02; one wave of persistent CTAs).
 __global__ void __launch_bounds__(256, 6) k_binsort(BatchDesc d)
 {
     __shared__ uint32_t s_out[kSortChunk];
@@ -1465,8 +1465,8 @@ void hl_shares(const uint32_t *primes, uint32_t n_lo, uint32_t n, uint32_t ctas,
 // dealt out by warps where blocks would give the first CTA more than 1.40 (1 / p
 // for a prime's marks: 3% above the marks themselves) or there are fewer than 8
 // rounds, whose last is a part of one; and one by one where warps would (a few
-// thousand primes, or primes from 2e4 on: 2.6 of the mean from 1e4 on at 1e12,
-// 1.1 one by one).
+// thousand primes, or primes from 2e4 on: 2.64 of the mean from 1e4 on at 1e12,
+// 1.03 one by one).
 uint32_t hl_deal(const HlShares *sh, const uint32_t *primes, uint32_t n_lo, uint32_t n_hi, uint32_t ctas, bool binned)
 {
     constexpr double kMost = 1.40;
